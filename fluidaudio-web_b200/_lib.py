@@ -77,6 +77,8 @@ SIGNATURES = {
     "fa_conv2d_windows": [P, P, P, P] + [I] * 15 + [PP],
     "fa_bmm_qk": [P, P, P, P, I, I, I, I, PP],
     "fa_bmm_pv": [P, P, P, I, I, I, PP],
+    "fa_attn_step": [P, P, P, P, I, I, I, PP],
+    "fa_attn_step_append": [P, P, P, P, I, I, I, PP],
     "fa_attn_fused": [P, P, P, P, P, P, P, I, I, I, PP],
     "fa_attn_fused_qkv": [P, P, P, P, P, I, I, I, PP],
     "fa_rel_shift_b": [P, P, I, PP],

@@ -397,6 +397,21 @@ class CudaContext:
     def bmmPV(self, p, v, H: int, HD: int, W: int = 1) -> Tensor:
         return self._op(self._lib.fa_bmm_pv, p.h, v.h, H, HD, W)
 
+    def attnStep(self, q, k, v, H: int, HD: int, W: int = 1) -> Optional[Tensor]:
+        """Optional member: bmmPV(softmax(bmmQK(q, k)), v) for one query per window (q [W, H*HD]) in one pass over the
+        keys and values.  None when the shape is outside the kernel's range."""
+        out = C.c_void_p()
+        self._check(self._lib.fa_attn_step(self._h, q.h, k.h, v.h, H, HD, W, C.byref(out)))
+        return self._wrap(out) if out.value else None
+
+    def attnStepAppend(self, qkv, cacheK, cacheV, n: int, NH: int, HD: int) -> Optional[Tensor]:
+        """Optional member: the self-attention step of S streams.  qkv [S, 3*NH*HD] is the new token's q | k | v; its k and
+        v go into row n of the caches [positions, S*NH*HD] and q attends over rows 0..n.  None when the shape is
+        outside the kernel's range (nothing was written then)."""
+        out = C.c_void_p()
+        self._check(self._lib.fa_attn_step_append(self._h, qkv.h, cacheK.h, cacheV.h, n, NH, HD, C.byref(out)))
+        return self._wrap(out) if out.value else None
+
     def attnFused(self, q, k, v, pos, pbu, pbv, H: int, HD: int, W: int) -> Optional[Tensor]:
         """Fused rel-pos self-attention (optional member, compute.d.ts:247-248).  Returns None when the
         shape is outside the fused kernel's range - the caller then runs the separate ops."""

@@ -91,12 +91,22 @@ def load_decoder(ctx, weights: Dict[str, np.ndarray], NH: int, quant: Optional[s
             a = (a * s).astype(f32)
         return ctx.upload(a, 1, a.size)
 
+    def self_qkv(L):
+        """The self-attention projections: one [D, 3D] matrix q | k | v where the backend has the one-pass attention
+        step that reads it (k has no bias: zeros), three matrices otherwise.  Per-column arithmetic is the same."""
+        t = lambda s: f"L{L}_{s}"
+        if not hasattr(ctx, "attnStepAppend"):
+            return dict(sqw=mat(t("sqw"), SCALE), sqb=vec(t("sqb"), SCALE), skw=mat(t("skw")), svw=mat(t("svw")), svb=vec(t("svb")))
+        scaled = lambda k: (weights[t(k)].astype(f32) * SCALE).astype(f32)
+        wide = np.concatenate([scaled("sqw"), weights[t("skw")].astype(f32), weights[t("svw")].astype(f32)], axis=1)
+        bias = np.concatenate([scaled("sqb").reshape(-1), np.zeros(D, f32), weights[t("svb")].astype(f32).reshape(-1)])
+        return dict(sqkvw=_W(ctx, wide, quant), sqkvb=ctx.upload(bias, 1, 3 * D))
+
     layers = []
     for L in range(cfg["layers"]):
         t = lambda s: f"L{L}_{s}"
         layers.append(dict(
-            sqw=mat(t("sqw"), SCALE), sqb=vec(t("sqb"), SCALE), skw=mat(t("skw")), svw=mat(t("svw")), svb=vec(t("svb")),
-            sow=mat(t("sow")), sob=vec(t("sob")), cqw=mat(t("cqw"), SCALE), cqb=vec(t("cqb"), SCALE), ckw=mat(t("ckw")),
+            **self_qkv(L), sow=mat(t("sow")), sob=vec(t("sob")), cqw=mat(t("cqw"), SCALE), cqb=vec(t("cqb"), SCALE), ckw=mat(t("ckw")),
             cvw=mat(t("cvw")), cvb=vec(t("cvb")), cow=mat(t("cow")), cob=vec(t("cob")),
             ln1=(vec(t("ln1w")), vec(t("ln1b"))), ln2=(vec(t("ln2w")), vec(t("ln2b"))), ln3=(vec(t("ln3w")), vec(t("ln3b"))),
             f1w=mat(t("f1w")), f1b=vec(t("f1b")), f2w=mat(t("f2w")), f2b=vec(t("f2b"))))
@@ -110,6 +120,34 @@ def load_decoder(ctx, weights: Dict[str, np.ndarray], NH: int, quant: Optional[s
     cfg["VOCABP"] = VOCABP
     return dict(layers=layers, embed=embed, embedT=_W(ctx, embedTP, quant), pos=np.ascontiguousarray(weights["pos"], dtype=f32),
                 lnf=(vec("lnf_w"), vec("lnf_b")), cfg=cfg)
+
+
+def _self_attention(ctx, h, w, cacheK, cacheV, n, S, D, NH, HD):
+    """The normed token rows h [S, D] -> attention over the S streams' caches [position, S*D], whose row n becomes the
+    token's key and value (raw-whisper-decoder.js:112-124).  Only past+current exist, so there is no mask."""
+    if "sqkvw" in w:
+        qkv = _mm(ctx, h, w["sqkvw"], bias=w["sqkvb"])
+        att = ctx.attnStepAppend(qkv, cacheK, cacheV, n, NH, HD)
+        if att is not None:
+            return att
+        q, k, v = (ctx.sliceCols(qkv, i * D, D) for i in range(3))
+    else:
+        q, k, v = _mm(ctx, h, w["sqw"], bias=w["sqb"]), _mm(ctx, h, w["skw"]), _mm(ctx, h, w["svw"], bias=w["svb"])
+    flat = (lambda t: t) if S == 1 else (lambda t: ctx.reshapeView(t, 1, S * D))
+    ctx.copyRows(cacheK, flat(k), n)
+    ctx.copyRows(cacheV, flat(v), n)
+    probs = ctx.softmax(ctx.bmmQK(flat(q), ctx.rowsView(cacheK, n + 1), None, S * NH, HD))  # [S*NH, n+1]
+    att = ctx.bmmPV(probs, ctx.rowsView(cacheV, n + 1), S * NH, HD)
+    return att if S == 1 else ctx.reshapeView(att, S, D)
+
+
+def _cross_attention(ctx, q, kv, S, NH, HD):
+    """q [S, D] over each stream's own encoder keys and values [S*Tenc, D] (:126-131)."""
+    att = ctx.attnStep(q, kv["k"], kv["v"], NH, HD, S) if hasattr(ctx, "attnStep") else None
+    if att is None:
+        probs = ctx.softmax(ctx.bmmQK(q, kv["k"], None, NH, HD, S))  # one window per stream: [S*NH, Tenc]
+        att = ctx.bmmPV(probs, kv["v"], NH, HD, S)
+    return att
 
 
 # ---------------------------------------------------------------------------- one stream (reference form)
@@ -145,18 +183,10 @@ def decode_next(ctx, dec, kv, st, token: int) -> np.ndarray:
     def body():
         nonlocal x
         for li, w in enumerate(dec["layers"]):
-            h = ln(x, w["ln1"])
-            q = _mm(ctx, h, w["sqw"], bias=w["sqb"])
-            ctx.copyRows(st["selfK"][li], _mm(ctx, h, w["skw"]), n)
-            ctx.copyRows(st["selfV"][li], _mm(ctx, h, w["svw"], bias=w["svb"]), n)
-            K = ctx.rowsView(st["selfK"][li], n + 1)
-            V = ctx.rowsView(st["selfV"][li], n + 1)
-            probs = ctx.softmax(ctx.bmmQK(q, K, None, NH, HD))  # [NH, n+1]; only past+current exist -> no mask
-            x = ctx.add(x, _mm(ctx, ctx.bmmPV(probs, V, NH, HD), w["sow"], bias=w["sob"]))
-            h = ln(x, w["ln2"])
-            cq = _mm(ctx, h, w["cqw"], bias=w["cqb"])
-            cprobs = ctx.softmax(ctx.bmmQK(cq, kv[li]["k"], None, NH, HD))  # [NH, Tenc]
-            x = ctx.add(x, _mm(ctx, ctx.bmmPV(cprobs, kv[li]["v"], NH, HD), w["cow"], bias=w["cob"]))
+            att = _self_attention(ctx, ln(x, w["ln1"]), w, st["selfK"][li], st["selfV"][li], n, 1, D, NH, HD)
+            x = ctx.add(x, _mm(ctx, att, w["sow"], bias=w["sob"]))
+            cq = _mm(ctx, ln(x, w["ln2"]), w["cqw"], bias=w["cqb"])
+            x = ctx.add(x, _mm(ctx, _cross_attention(ctx, cq, kv[li], 1, NH, HD), w["cow"], bias=w["cob"]))
             h = ln(x, w["ln3"])
             x = ctx.add(x, _mm(ctx, _mm(ctx, h, w["f1w"], bias=w["f1b"], act="gelu_erf"), w["f2w"], bias=w["f2b"]))
         st["n"] = n + 1
@@ -220,19 +250,10 @@ def step_streams(ctx, dec, kv, st, x, n: int):
     S = st["S"]
     ln = lambda x, lp: ctx.layernorm(x, lp[0], lp[1])
     for li, w in enumerate(dec["layers"]):
-        h = ln(x, w["ln1"])
-        q = _mm(ctx, h, w["sqw"], bias=w["sqb"])
-        ctx.copyRows(st["selfK"][li], ctx.reshapeView(_mm(ctx, h, w["skw"]), 1, S * D), n)
-        ctx.copyRows(st["selfV"][li], ctx.reshapeView(_mm(ctx, h, w["svw"], bias=w["svb"]), 1, S * D), n)
-        K = ctx.rowsView(st["selfK"][li], n + 1)
-        V = ctx.rowsView(st["selfV"][li], n + 1)
-        probs = ctx.softmax(ctx.bmmQK(ctx.reshapeView(q, 1, S * D), K, None, S * NH, HD))  # [S*NH, n+1]
-        att = ctx.reshapeView(ctx.bmmPV(probs, V, S * NH, HD), S, D)
+        att = _self_attention(ctx, ln(x, w["ln1"]), w, st["selfK"][li], st["selfV"][li], n, S, D, NH, HD)
         x = _mm_add(ctx, x, att, w["sow"], bias=w["sob"])
-        h = ln(x, w["ln2"])
-        cq = _mm(ctx, h, w["cqw"], bias=w["cqb"])
-        cprobs = ctx.softmax(ctx.bmmQK(cq, kv[li]["k"], None, NH, HD, S))  # one window per stream: [S*NH, Tenc]
-        x = _mm_add(ctx, x, ctx.bmmPV(cprobs, kv[li]["v"], NH, HD, S), w["cow"], bias=w["cob"])
+        cq = _mm(ctx, ln(x, w["ln2"]), w["cqw"], bias=w["cqb"])
+        x = _mm_add(ctx, x, _cross_attention(ctx, cq, kv[li], S, NH, HD), w["cow"], bias=w["cob"])
         h = ln(x, w["ln3"])
         x = _mm_add(ctx, x, _mm(ctx, h, w["f1w"], bias=w["f1b"], act="gelu_erf"), w["f2w"], bias=w["f2b"])
     return _mm(ctx, ln(x, dec["lnf"]), dec["embedT"])

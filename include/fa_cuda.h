@@ -255,6 +255,14 @@ int fa_conv2d(fa_ctx *ctx, const fa_tensor *x, const fa_tensor *w, const fa_tens
 int fa_bmm_qk(fa_ctx *ctx, const fa_tensor *q, const fa_tensor *b, const fa_tensor *qb, int H, int HD, int W,
               int b_shared, fa_tensor **out);                                             /* bmmQK :191 */
 int fa_bmm_pv(fa_ctx *ctx, const fa_tensor *p, const fa_tensor *v, int H, int HD, int W, fa_tensor **out); /* bmmPV :193 */
+/* Attention of one query per window in one pass (optional members of token-by-token decoding).
+ * fa_attn_step: bmmPV(softmax(bmmQK(q, k)), v) for q [W, H*HD], k and v [W*Tk, H*HD].
+ * fa_attn_step_append: the self-attention form.  qkv [S, 3*NH*HD] holds q | k | v of S streams' new token, the caches are
+ * [positions, S*NH*HD]; writes the token's k and v into row n, attends over rows 0..n, gives [S, NH*HD].
+ * *out == NULL with status 0 means "not this shape" (nothing was written; the caller takes the separate ops). */
+int fa_attn_step(fa_ctx *ctx, const fa_tensor *q, const fa_tensor *k, const fa_tensor *v, int H, int HD, int W, fa_tensor **out);
+int fa_attn_step_append(fa_ctx *ctx, const fa_tensor *qkv, fa_tensor *cache_k, fa_tensor *cache_v, int n, int NH, int HD,
+                        fa_tensor **out);
 /* attnFused :247-248 (optional member; may yield no tensor, the caller then uses the separate ops):
  * rel-pos self-attention for W windows of T = q.rows/W frames; pos [2T-1, H*HD] is the projected
  * positional table, pbu/pbv [1, H*HD].  *out == NULL with status 0 means "not this shape". */
