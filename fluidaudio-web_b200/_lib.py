@@ -77,6 +77,7 @@ SIGNATURES = {
     "fa_conv2d_windows": [P, P, P, P] + [I] * 15 + [PP],
     "fa_bmm_qk": [P, P, P, P, I, I, I, I, PP],
     "fa_bmm_pv": [P, P, P, I, I, I, PP],
+    "fa_linear_step": [P, P, P, P, C.c_float, P, P, P, I, I, P, I, P, PP],
     "fa_attn_step": [P, P, P, P, I, I, I, PP],
     "fa_attn_step_append": [P, P, P, P, I, I, I, PP],
     "fa_attn_fused": [P, P, P, P, P, P, P, I, I, I, PP],

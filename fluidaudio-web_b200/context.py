@@ -397,6 +397,16 @@ class CudaContext:
     def bmmPV(self, p, v, H: int, HD: int, W: int = 1) -> Tensor:
         return self._op(self._lib.fa_bmm_pv, p.h, v.h, H, HD, W)
 
+    def linearStep(self, x, w, scale=None, N: int = 0, K: int = 0, *, norm=None, bias=None, act="none", add=None,
+                   eps: float = 1e-5) -> Tensor:
+        """Optional member: add + act(layernorm(x) @ W + bias), one linear layer of a decoding step.  W is a tensor, or
+        PackedBytes with scale, N and K as for matmulInt8; norm = (gamma, beta).  One launch for a single row, the
+        separate members for more."""
+        q8 = isinstance(w, PackedBytes)
+        g, b = norm if norm is not None else (None, None)
+        return self._op(self._lib.fa_linear_step, x.h, self._h_of(g), self._h_of(b), eps, None if q8 else w.h, w.h if q8 else None,
+                        self._h_of(scale), N, K, self._h_of(bias), ACT[act], self._h_of(add))
+
     def attnStep(self, q, k, v, H: int, HD: int, W: int = 1) -> Optional[Tensor]:
         """Optional member: bmmPV(softmax(bmmQK(q, k)), v) for one query per window (q [W, H*HD]) in one pass over the
         keys and values.  None when the shape is outside the kernel's range."""

@@ -10,10 +10,9 @@
 //                 y = s_m * sum_blk scale[n,blk] * ((S1 - zp*A1) + (S2 - zp*A2) / 128).
 //                 Arithmetic budget: ~1 lane-op per weight at M = 1 (an f32 unpack-and-FMA needs 4).
 //   k_gemv_kn     matmul with f16-storage B [K][N] (lib.rs:59-94) and matmulInt8 with wq [K][N]
-//                 (lib.rs:143-162): N-contiguous rows.  A warp owns 32*VEC consecutive columns, the 8 warps of
-//                 a CTA take rows k round-robin, K is split over gridDim.y; activations stay f32 (exact).
-//                 Partial sums meet in a scratch buffer and the last CTA to arrive (an atomic ticket, no
-//                 waiting) adds them in slice order, so the result does not depend on scheduling.
+//                 (lib.rs:143-162) at M = 1: N-contiguous rows.  A block owns 128 consecutive columns, its 8 warps
+//                 take rows k round-robin, K is split over the ranks of a cluster; activations stay f32 (exact), and
+//                 a layernorm of the row can run in front of the product.  Sums meet in a fixed order.
 #include <cuda_fp16.h>
 
 #include <type_traits>
@@ -266,148 +265,173 @@ __device__ __forceinline__ float gemv_finish(float acc, int m, int n, int N, con
   return v;
 }
 
-// VEC weights per lane and row: 8 (f16, 16-byte loads) or 4 (f16, 8-byte loads, for N % 8 != 0) or 16 (int8).
-template <int VEC, bool I8>
-__device__ __forceinline__ void load_row(const void *w, size_t off, float (&f)[VEC]) {
-  if constexpr (I8) {
-    static_assert(VEC == 16, "int8 rows are read 16 bytes at a time");
-    const uint4 v = __ldcs((const uint4 *)((const int8_t *)w + off));
-    const unsigned wd[4] = {v.x ^ 0x80808080u, v.y ^ 0x80808080u, v.z ^ 0x80808080u, v.w ^ 0x80808080u};
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      // byte b of (q + 128) into the mantissa of 2^23: the float 8388608 + q + 128, then back to q
-      f[i * 4 + 0] = __uint_as_float(__byte_perm(wd[i], 0x4B000000u, 0x7650)) - 8388736.0f;
-      f[i * 4 + 1] = __uint_as_float(__byte_perm(wd[i], 0x4B000000u, 0x7651)) - 8388736.0f;
-      f[i * 4 + 2] = __uint_as_float(__byte_perm(wd[i], 0x4B000000u, 0x7652)) - 8388736.0f;
-      f[i * 4 + 3] = __uint_as_float(__byte_perm(wd[i], 0x4B000000u, 0x7653)) - 8388736.0f;
-    }
-  } else if constexpr (VEC == 8) {
-    const uint4 v = __ldcs((const uint4 *)((const __half *)w + off));
-    const __half2 *h = (const __half2 *)&v;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const float2 t = __half22float2(h[i]);
-      f[2 * i] = t.x, f[2 * i + 1] = t.y;
-    }
-  } else {
-    static_assert(VEC == 4, "f16 rows are read 16 or 8 bytes at a time");
-    const uint2 v = __ldcs((const uint2 *)((const __half *)w + off));
-    const __half2 *h = (const __half2 *)&v;
-    const float2 t0 = __half22float2(h[0]), t1 = __half22float2(h[1]);
-    f[0] = t0.x, f[1] = t0.y, f[2] = t1.x, f[3] = t1.y;
-  }
+// Four consecutive weights of a row as loaded (4 bytes of int8, 8 of f16), and as floats.
+template <bool I8>
+struct RawRow {
+  using type = typename std::conditional<I8, unsigned, uint2>::type;
+};
+template <bool I8>
+__device__ __forceinline__ typename RawRow<I8>::type load_raw(const void *w, size_t off) {
+  if constexpr (I8)
+    return __ldcs((const unsigned *)((const int8_t *)w + off));
+  else
+    return __ldcs((const uint2 *)((const __half *)w + off));
+}
+__device__ __forceinline__ float4 widen(unsigned v) {
+  // byte b of (q + 128) into the mantissa of 2^23: the float 8388608 + q + 128, then back to q
+  const unsigned x = v ^ 0x80808080u;
+  return make_float4(__uint_as_float(__byte_perm(x, 0x4B000000u, 0x7650)) - 8388736.0f,
+                     __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7651)) - 8388736.0f,
+                     __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7652)) - 8388736.0f,
+                     __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7653)) - 8388736.0f);
+}
+__device__ __forceinline__ float4 widen(uint2 v) {
+  const __half2 *h = (const __half2 *)&v;
+  const float2 a = __half22float2(h[0]), b = __half22float2(h[1]);
+  return make_float4(a.x, a.y, b.x, b.y);
 }
 
-template <int M, int VEC, bool I8>
-__global__ void __launch_bounds__(kThreads) k_gemv_kn(const float *__restrict__ a, const void *__restrict__ w,
-                                                      float *__restrict__ y, float *__restrict__ partials,
-                                                      int *__restrict__ tickets, int K, int N, int kslice, GemvEp ep) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  float *as = (float *)smem;                 // [M][kslice] activations of this K slice
-  float *red = as + (size_t)M * kslice;      // [8][32*VEC]
-  __shared__ int last_flag;
-  constexpr int U = I8 ? 2 : 4;              // rows in flight per warp
-  constexpr int CW = 32 * VEC;               // columns per CTA
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int k0 = blockIdx.y * kslice, k1 = min(K, k0 + kslice), ks = gridDim.y;
-  const int c0 = blockIdx.x * CW + lane * VEC;
-  const bool live = c0 < N;  // N % VEC == 0, so a live lane owns VEC whole columns
-  fa_grid_dep_sync();
-  for (int i = tid; i < M * kslice; i += kThreads) {
-    const int m = i / kslice, kk = i - m * kslice;
-    as[i] = k0 + kk < k1 ? a[(size_t)m * K + k0 + kk] : 0.f;
-  }
+__device__ __forceinline__ float block_sum(float v, float *red, int lane, int warp) {
+  v = warp_sum_f(v);
+  if (lane == 0) red[warp] = v;
   __syncthreads();
-  float acc[M][VEC];
+  float t = red[0];
 #pragma unroll
-  for (int m = 0; m < M; m++)
+  for (int i = 1; i < kThreads / 32; i++) t += red[i];
+  __syncthreads();
+  return t;
+}
+
+// y[n] = act(sum_k x[k] * w[k][n] * colscale[n] + bias[n]) + add[n] for ONE row x [K]; with NORM, x is first replaced by
+// its layernorm (gamma, beta: two-pass mean and variance as in k_layernorm_reg).
+//
+// What bounds it: the weight stream of the large matrices (66 MB of int8 for the vocabulary projection), latency for the
+// others: 1.6 MB are 0.3 us of HBM time, so the launch is a chain of load -> row sum -> exchange between K slices.
+// Hence the layout: a block owns 128 columns (one 4-byte int8 or 8-byte f16 load per lane and row) and a K slice, its
+// 8 warps take rows round-robin with kKnU loads per lane in flight, the first of them requested before the launch waits
+// for its predecessor where the weights can only have been written by an upload (int8 payloads).  K slices are the
+// ranks of a cluster: their sums meet in rank 0's shared memory, in rank order, after one cluster barrier.  (The form
+// before this one let the slices meet in global memory behind a ticket, up to 40 partial rows read by the last block.)
+// Measured, K = N = 1280 int8 in a decoder step: 7.3 us from launch to end, wait for the predecessor included, where the
+// layernorm, product and residual add were three launches; 1280 x 51868 int8 with the layernorm 25 us (2.7 TB/s) against
+// a layernorm, a digit pass and a tensor-core product of 3.8 + 2.6 + 12.5 us that read the row as two int8 digits
+// instead of f32.  A 16-token decoder pass of one stream: 8.24 -> 5.1 ms, what is left is the host's 9 us per launch.
+constexpr int kKnU = 16, kKnCols = 128, kKnSlice = 2048;  // loads in flight per lane, columns per block, rows of x held at a time
+constexpr int kKnNormMax = 4096;                           // longest row that the layernorm prologue holds in registers
+
+struct KnParams {
+  const float *x, *gamma, *beta;
+  const void *w;
+  float *y;
+  int K, N, kslice;
+  float eps;
+  GemvEp ep;
+};
+
+template <bool I8, bool NORM>
+__global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
+  __shared__ __align__(16) float xs[kKnSlice];
+  __shared__ __align__(16) float4 red[kThreads / 32][32];
+  __shared__ float cred[8][kKnCols];  // rank 0: the K slices' sums
+  __shared__ float stat[kThreads / 32];
+  using Raw = typename RawRow<I8>::type;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.y, ks = gridDim.y, N = p.N, K = p.K;
+  const int k0 = rank * p.kslice, k1 = min(K, k0 + p.kslice);
+  const int c0 = blockIdx.x * kKnCols + lane * 4;
+  const bool live = c0 < N;  // N % 4 == 0: a live lane owns four whole columns
+  const int cc = live ? c0 : 0;
+  Raw raw[kKnU];
+  auto fetch = [&](int kk) {
 #pragma unroll
-    for (int v = 0; v < VEC; v++) acc[m][v] = 0.f;
-  if (live) {
-    for (int kk = k0 + warp * U; kk < k1; kk += 8 * U) {
-      float f[U][VEC];
+    for (int u = 0; u < kKnU; u++) {
+      const int k = kk + u * 8;
+      raw[u] = Raw{};
+      if (k < k1) raw[u] = load_raw<I8>(p.w, (size_t)k * N + cc);
+    }
+  };
+  int kk = k0 + warp;  // rows kk, kk + 8, ...
+  if (I8) fetch(kk);
+  if (ks > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // every rank runs before a remote store
+  fa_grid_dep_sync();
+  if (!I8) fetch(kk);
+  if (NORM) {
+    float4 v[kKnNormMax / 4 / kThreads];
+    const int k4 = K >> 2;
+    float s = 0.f;
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int k = kk + u < k1 ? kk + u : k1 - 1;
-        load_row<VEC, I8>(w, (size_t)k * N + c0, f[u]);
+    for (int u = 0; u < kKnNormMax / 4 / kThreads; u++) {
+      const int q = tid + u * kThreads;
+      v[u] = q < k4 ? ((const float4 *)p.x)[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+      s += (v[u].x + v[u].y) + (v[u].z + v[u].w);
+    }
+    const float mean = block_sum(s, stat, lane, warp) / (float)K;
+    float vs = 0.f;
+#pragma unroll
+    for (int u = 0; u < kKnNormMax / 4 / kThreads; u++)
+      if (tid + u * kThreads < k4) {
+        const float a = v[u].x - mean, b = v[u].y - mean, c = v[u].z - mean, d = v[u].w - mean;
+        vs += (a * a + b * b) + (c * c + d * d);
       }
+    const float inv = 1.0f / sqrtf(block_sum(vs, stat, lane, warp) / (float)K + p.eps);
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        if (kk + u < k1) {
+    for (int u = 0; u < kKnNormMax / 4 / kThreads; u++) {
+      const int q = tid + u * kThreads, k = q * 4;
+      if (q < k4 && k >= k0 && k < k1) {  // kslice % 8 == 0: a quad lies in one slice; the slice fits xs (host check)
+        const float4 g = ((const float4 *)p.gamma)[q], b = ((const float4 *)p.beta)[q];
+        *(float4 *)(xs + (k - k0)) = make_float4((v[u].x - mean) * inv * g.x + b.x, (v[u].y - mean) * inv * g.y + b.y,
+                                                 (v[u].z - mean) * inv * g.z + b.z, (v[u].w - mean) * inv * g.w + b.w);
+      }
+    }
+    __syncthreads();
+  }
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int base = k0; base < k1; base += kKnSlice) {
+    const int end = min(k1, base + kKnSlice);
+    if (!NORM) {
+      if (base > k0) __syncthreads();
+      for (int i = tid; i < end - base; i += kThreads) xs[i] = p.x[base + i];
+      __syncthreads();
+    }
+    while (kk < end) {  // a batch never straddles `end` on its way: kKnSlice % (8 * kKnU) == 0
 #pragma unroll
-          for (int m = 0; m < M; m++) {
-            const float av = as[m * kslice + (kk + u - k0)];
-#pragma unroll
-            for (int v = 0; v < VEC; v++) acc[m][v] = fmaf(av, f[u][v], acc[m][v]);
-          }
+      for (int u = 0; u < kKnU; u++) {
+        const int k = kk + u * 8;
+        if (k < end) {
+          const float a = xs[k - base];
+          const float4 f = widen(raw[u]);
+          acc.x = fmaf(a, f.x, acc.x), acc.y = fmaf(a, f.y, acc.y), acc.z = fmaf(a, f.z, acc.z), acc.w = fmaf(a, f.w, acc.w);
         }
       }
+      kk += 8 * kKnU;
+      if (kk < k1) fetch(kk);
     }
   }
-  // the 8 warps' partial sums, one activation row at a time, added in warp order
-  for (int m = 0; m < M; m++) {
-#pragma unroll
-    for (int v = 0; v < VEC; v++) red[warp * CW + lane * VEC + v] = acc[m][v];
-    __syncthreads();
-    for (int c = tid; c < CW; c += kThreads) {
-      const int n = blockIdx.x * CW + c;
-      if (n < N) {
-        float s = red[c];
-#pragma unroll
-        for (int wv = 1; wv < 8; wv++) s += red[wv * CW + c];
-        if (ks == 1)
-          y[(size_t)m * N + n] = gemv_finish(s, m, n, N, ep);
-        else
-          partials[((size_t)blockIdx.y * M + m) * N + n] = s;
-      }
-    }
-    __syncthreads();
-  }
-  if (ks == 1) return;
-  __threadfence();
-  if (tid == 0) {
-    const int old = atomicAdd(&tickets[blockIdx.x], 1);
-    last_flag = old == ks - 1;
-    if (last_flag) tickets[blockIdx.x] = 0;  // ready for the next launch on this stream
-  }
+  red[warp][lane] = acc;
   __syncthreads();
-  if (!last_flag) return;
-  __threadfence();
-  for (int i = tid; i < M * CW; i += kThreads) {
-    const int m = i / CW, n = blockIdx.x * CW + (i - m * CW);
-    if (n < N) {
-      float s = 0.f;
-#pragma unroll 8
-      for (int q = 0; q < ks; q++) s += __ldcg(&partials[((size_t)q * M + m) * N + n]);
-      y[(size_t)m * N + n] = gemv_finish(s, m, n, N, ep);
+  float sum = 0.f;
+  if (tid < kKnCols) {
+    const float *r = (const float *)red;
+    sum = r[tid];
+#pragma unroll
+    for (int i = 1; i < kThreads / 32; i++) sum += r[i * kKnCols + tid];
+  }
+  if (ks > 1) {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (tid < kKnCols) {
+      uint32_t remote;
+      const uint32_t local = (uint32_t)__cvta_generic_to_shared(&cred[rank][tid]);
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(0));
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(sum) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (rank != 0) return;
+    if (tid < kKnCols) {
+      sum = cred[0][tid];
+      for (int i = 1; i < ks; i++) sum += cred[i][tid];
     }
   }
-}
-
-template <int M, int VEC, bool I8>
-int launch_kn(fa_ctx *ctx, const float *a, const void *w, float *y, float *partials, int K, int N, int kslice, int ksplit,
-              const GemvEp &ep) {
-  const size_t smem = ((size_t)M * kslice + 8 * 32 * VEC) * sizeof(float);
-  auto kern = k_gemv_kn<M, VEC, I8>;
-  if (smem > 48 * 1024) FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  {
-    LaunchScope ls(ctx, I8 ? "gemv_i8" : "gemv_f16");
-    fa_launch_dep(ctx, kern, dim3(ceil_div(N, 32 * VEC), ksplit), dim3(kThreads), smem, a, w, y, partials, ctx->gemv_tickets, K,
-                  N, kslice, ep);
-  }
-  FA_LAUNCH_CHECK(ctx, "gemv_kn");
-  return FA_OK;
-}
-
-template <int VEC, bool I8>
-int dispatch_kn(fa_ctx *ctx, int M, const float *a, const void *w, float *y, float *partials, int K, int N, int kslice,
-                int ksplit, const GemvEp &ep) {
-  switch (M) {
-    case 1: return launch_kn<1, VEC, I8>(ctx, a, w, y, partials, K, N, kslice, ksplit, ep);
-    case 2: return launch_kn<2, VEC, I8>(ctx, a, w, y, partials, K, N, kslice, ksplit, ep);
-    case 3: return launch_kn<3, VEC, I8>(ctx, a, w, y, partials, K, N, kslice, ksplit, ep);
-    default: return launch_kn<4, VEC, I8>(ctx, a, w, y, partials, K, N, kslice, ksplit, ep);
-  }
+  const int n = blockIdx.x * kKnCols + tid;
+  if (tid < kKnCols && n < N) p.y[n] = gemv_finish(sum, 0, n, N, p.ep);
 }
 
 template <int M>
@@ -663,36 +687,43 @@ int fa_nbits_mma(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *sc
 // N-contiguous weights: one activation row only.  From two rows on, the tensor-core kernel (which shares each
 // weight tile between all rows for free) is at least as fast as this one; measured on 1280 x 1280 f16 at
 // M = 4: 10.6 us here against 7.3 us there.
-bool fa_gemv_kn_ok(int M, int N, int K, bool i8) { return M == 1 && K >= 1 && N >= 1 && (N % (i8 ? 16 : 4)) == 0; }
+bool fa_gemv_kn_ok(int M, int N, int K) { return M == 1 && K >= 1 && N >= 4 && (N & 3) == 0; }
 
-// w: f16 [K][N] (i8 = false) or int8 [K][N]; y = act(acc * colscale[n] + bias[n]) + add[m][n].
-int fa_gemv_kn(fa_ctx *ctx, const float *a, const void *w, bool i8, const float *colscale, const float *bias, int act,
-               const float *add, float *y, int M, int N, int K) {
-  const int vec = i8 ? 16 : ((N & 7) == 0 ? 8 : 4);
-  const int strips = ceil_div(N, 32 * vec);
-  // enough CTAs to put ~4 on every SM; a K slice of at most 2048 rows so its activations fit shared memory
-  const int target = 2, cap = 40;
-  int ksplit = ceil_div(ctx->sm_count * target, strips);
-  int max_split = ceil_div(K, 32);
-  if (max_split > cap) max_split = cap;
-  if (ksplit > max_split) ksplit = max_split;
-  if (ksplit < ceil_div(K, 2048)) ksplit = ceil_div(K, 2048);
-  if (ksplit < 1) ksplit = 1;
-  int kslice = ceil_div(K, ksplit);
-  kslice = (kslice + 7) / 8 * 8;
-  ksplit = ceil_div(K, kslice);
-  FA_REQUIRE(ctx, strips <= ctx->gemv_ticket_count, "gemv: %d column strips exceed the ticket array", strips);
-  void *partials = nullptr;
-  size_t pbytes = 0;
-  if (ksplit > 1) FA_TRY(fa_block_acquire(ctx, (size_t)ksplit * M * N * sizeof(float), &partials, &pbytes));
-  GemvEp ep{colscale, bias, add, act};
-  int rc;
-  if (i8)
-    rc = dispatch_kn<16, true>(ctx, M, a, w, y, (float *)partials, K, N, kslice, ksplit, ep);
-  else if (vec == 8)
-    rc = dispatch_kn<8, false>(ctx, M, a, w, y, (float *)partials, K, N, kslice, ksplit, ep);
-  else
-    rc = dispatch_kn<4, false>(ctx, M, a, w, y, (float *)partials, K, N, kslice, ksplit, ep);
-  if (partials) fa_block_release(ctx, partials);
-  return rc;
+// The layernorm prologue holds the row in registers and a K slice of it in shared memory, in whole quads.
+bool fa_gemv_kn_norm_ok(int K) { return K >= 4 && (K & 3) == 0 && K <= kKnNormMax; }
+
+// w: f16 [K][N] (i8 = false) or int8 [K][N]; y = act(acc * colscale[n] + bias[n]) + add[n]; gamma != NULL: layernorm first.
+int fa_gemv_kn(fa_ctx *ctx, const float *x, const float *gamma, const float *beta, float eps, const void *w, bool i8,
+               const float *colscale, const float *bias, int act, const float *add, float *y, int N, int K) {
+  KnParams p{x, gamma, beta, w, y, K, N, 0, eps, GemvEp{colscale, bias, add, act}};
+  // K slices = ranks of a cluster, as many (1, 2, 4, 8) as give about two blocks per SM and leave 64 rows to each; the
+  // layernorm form needs its slice in shared memory whole.
+  const int strips = ceil_div(N, kKnCols);
+  int ks = 1;
+  while (ks < 8 && strips * ks * 2 <= 2 * ctx->sm_count + ctx->sm_count / 4 && K >= 64 * ks * 2) ks *= 2;
+  while (gamma && ks < 8 && ceil_div(K, ks) > kKnSlice) ks *= 2;
+  p.kslice = (ceil_div(K, ks) + 7) / 8 * 8;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  cfg.gridDim = dim3(strips, ks);
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = ctx->stream;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see fa_launch_dep
+  attr[0].val.programmaticStreamSerializationAllowed = ctx->pdl ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = ks;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ks > 1 ? 2 : 1;
+  cudaError_t e;
+  {
+    LaunchScope ls(ctx, i8 ? "gemv_i8" : "gemv_f16");
+    if (gamma)
+      e = i8 ? cudaLaunchKernelEx(&cfg, k_gemv_kn<true, true>, p) : cudaLaunchKernelEx(&cfg, k_gemv_kn<false, true>, p);
+    else
+      e = i8 ? cudaLaunchKernelEx(&cfg, k_gemv_kn<true, false>, p) : cudaLaunchKernelEx(&cfg, k_gemv_kn<false, false>, p);
+  }
+  if (e != cudaSuccess) return fa_fail(ctx, FA_ERR_CUDA, "launch gemv_kn: %s", cudaGetErrorString(e));
+  return FA_OK;
 }

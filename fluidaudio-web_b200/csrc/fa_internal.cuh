@@ -311,8 +311,6 @@ int fa_simt_nbits(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *s
 // fa_gemv.cu: decode-size (M <= 16) bandwidth kernels.
 int fa_gemv_nbits(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y,
                   int M, int N, int K, int nblk, int zpb);
-int fa_gemv_kn(fa_ctx *ctx, const float *a, const void *b, int b_kind, const float *colscale, const float *bias,
-               int act, const float *add, float *c, int M, int N, int K);
 // fa_gemm_tc.cu: tcgen05 kernels and their prepasses.
 struct TcEpilogue {
   const float *rowscale = nullptr;  // [M] multiplies the accumulator (int8 activation scales)
@@ -358,9 +356,10 @@ int fa_nbits_mma(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *sc
                  int K, int nblk, int zpb, bool hilo);
 int fa_gemv_nbits(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y, int M,
                   int N, int K, int nblk, int zpb);
-bool fa_gemv_kn_ok(int M, int N, int K, bool i8);
-int fa_gemv_kn(fa_ctx *ctx, const float *a, const void *w, bool i8, const float *colscale, const float *bias, int act,
-               const float *add, float *y, int M, int N, int K);
+bool fa_gemv_kn_ok(int M, int N, int K);
+bool fa_gemv_kn_norm_ok(int K);
+int fa_gemv_kn(fa_ctx *ctx, const float *x, const float *gamma, const float *beta, float eps, const void *w, bool i8,
+               const float *colscale, const float *bias, int act, const float *add, float *y, int N, int K);
 int fa_prep_a_f16(fa_ctx *ctx, const float *a, int M, int K, __half *out);
 int fa_prep_a_f16_hilo(fa_ctx *ctx, const float *a, int M, int K, __half *out);
 int fa_prep_a_f16_perm8(fa_ctx *ctx, const float *a, int M, int K, __half *out);

@@ -226,7 +226,7 @@ static int matmul_impl(fa_ctx *ctx, const fa_tensor *a, fa_tensor *b, const fa_t
   // A row operand that already carries a valid packed shadow and is headed for the tensor cores is not read as
   // f32 at all (and, if it is a lazy hidden-layer result, must not be: that would fill its f32 storage for nothing).
   const bool tc_route = b->storage == FA_F16 && !b->view && tc_shape_ok(ctx, M, N, K) &&
-                        !(gemv_shape_ok(ctx, M, N, K) && fa_gemv_kn_ok(M, N, K, false));
+                        !(gemv_shape_ok(ctx, M, N, K) && fa_gemv_kn_ok(M, N, K));
   const bool shadow_only = tc_route && a->storage == FA_F32 && !a->view && a->a16_valid && !a->a16_hilo &&
                            a->rows > ctx->f16_hilo_rows;
   if (!shadow_only) FA_TRY(fa_as_f32(ctx, a, &ap, &atmp));
@@ -235,8 +235,8 @@ static int matmul_impl(fa_ctx *ctx, const fa_tensor *a, fa_tensor *b, const fa_t
   int rc;
   const float *biasp = bias ? (const float *)bias->dptr : nullptr;
   const float *addp = add ? (const float *)add->dptr : nullptr;
-  if (b->storage == FA_F16 && gemv_shape_ok(ctx, M, N, K) && fa_gemv_kn_ok(M, N, K, false)) {
-    rc = fa_gemv_kn(ctx, ap, b->dptr, false, nullptr, biasp, act, addp, (float *)c->dptr, M, N, K);
+  if (b->storage == FA_F16 && gemv_shape_ok(ctx, M, N, K) && fa_gemv_kn_ok(M, N, K)) {
+    rc = fa_gemv_kn(ctx, ap, nullptr, nullptr, 0.0f, b->dptr, false, nullptr, biasp, act, addp, (float *)c->dptr, N, K);
   } else if (b->storage == FA_F16 && !b->view && tc_shape_ok(ctx, M, N, K)) {
     Scratch sa(ctx);
     const __half *a16 = nullptr;
@@ -337,8 +337,8 @@ extern "C" int fa_matmul_scatter(fa_ctx *ctx, const fa_tensor *a, fa_tensor *b, 
   return rc;
 }
 
-extern "C" int fa_matmul_int8(fa_ctx *ctx, const fa_tensor *a, fa_bytes *wq, const fa_tensor *scale, int N, int K,
-                              const fa_tensor *bias, int act, fa_tensor **out) {
+static int matmul_int8_impl(fa_ctx *ctx, const fa_tensor *a, fa_bytes *wq, const fa_tensor *scale, int N, int K,
+                            const fa_tensor *bias, int act, const fa_tensor *add, fa_tensor **out) {
   if (!ctx || !out) return fa_fail(ctx, FA_ERR_INVALID, "matmulInt8: NULL argument");
   FA_REQUIRE(ctx, fa_valid(ctx, a) && fa_valid_bytes(ctx, wq), "matmulInt8: unknown handle");
   FA_REQUIRE(ctx, N > 0 && K > 0, "matmulInt8: N=%d K=%d", N, K);
@@ -349,6 +349,10 @@ extern "C" int fa_matmul_int8(fa_ctx *ctx, const fa_tensor *a, fa_bytes *wq, con
   FA_REQUIRE(ctx, act >= 0 && act <= 5, "matmulInt8: unknown activation code %d", act);
   FA_TRY(check_vec(ctx, scale, N, "matmulInt8: scale"));
   if (bias) FA_TRY(check_vec(ctx, bias, N, "matmulInt8: bias"));
+  if (add) {
+    FA_TRY(check_vec(ctx, add, M * N, "matmulInt8: add"));
+    FA_REQUIRE(ctx, add->rows == M && add->cols == N, "matmulInt8: add is [%d,%d], expected [%d,%d]", add->rows, add->cols, M, N);
+  }
   FA_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
   const float *ap = nullptr;
   fa_tensor *atmp = nullptr;
@@ -357,8 +361,9 @@ extern "C" int fa_matmul_int8(fa_ctx *ctx, const fa_tensor *a, fa_bytes *wq, con
   FA_TRY(fa_tensor_new(ctx, M, N, FA_F32, true, &c));
   int rc = FA_OK;
   const float *biasp = bias ? (const float *)bias->dptr : nullptr;
-  if (gemv_shape_ok(ctx, M, N, K) && fa_gemv_kn_ok(M, N, K, true)) {
-    rc = fa_gemv_kn(ctx, ap, wq->dptr, true, (const float *)scale->dptr, biasp, act, nullptr, (float *)c->dptr, M, N, K);
+  const float *addp = add ? (const float *)add->dptr : nullptr;
+  if (gemv_shape_ok(ctx, M, N, K) && fa_gemv_kn_ok(M, N, K)) {
+    rc = fa_gemv_kn(ctx, ap, nullptr, nullptr, 0.0f, wq->dptr, true, (const float *)scale->dptr, biasp, act, addp, (float *)c->dptr, N, K);
   } else if (tc_shape_ok(ctx, M, N, K)) {
     const int limbs = ctx->int8_limbs;
     Scratch sa(ctx), ss(ctx);
@@ -371,11 +376,12 @@ extern "C" int fa_matmul_int8(fa_ctx *ctx, const fa_tensor *a, fa_bytes *wq, con
       ep.rowscale = (const float *)ss.p;
       ep.colscale = (const float *)scale->dptr;
       ep.bias = biasp;
+      ep.add = addp;
       ep.act = act;
       rc = fa_tc_gemm_i8(ctx, (const int8_t *)sa.p, limbs, (const int8_t *)wq->nk_i8, c->dptr, false, M, N, K, ep);
     }
   } else {
-    rc = fa_simt_gemm(ctx, ap, wq->dptr, 2, (const float *)scale->dptr, biasp, act, nullptr, (float *)c->dptr, M, N, K);
+    rc = fa_simt_gemm(ctx, ap, wq->dptr, 2, (const float *)scale->dptr, biasp, act, addp, (float *)c->dptr, M, N, K);
   }
   if (atmp) fa_free_tensor(ctx, atmp);
   if (rc != FA_OK) {
@@ -386,10 +392,54 @@ extern "C" int fa_matmul_int8(fa_ctx *ctx, const fa_tensor *a, fa_bytes *wq, con
   return FA_OK;
 }
 
+extern "C" int fa_matmul_int8(fa_ctx *ctx, const fa_tensor *a, fa_bytes *wq, const fa_tensor *scale, int N, int K,
+                              const fa_tensor *bias, int act, fa_tensor **out) {
+  return matmul_int8_impl(ctx, a, wq, scale, N, K, bias, act, nullptr, out);
+}
+
+// One linear layer of a decoding step: add + act(layernorm(x) @ W + bias).  A single row runs as one launch of the
+// GEMV kernel, everything else as the separate members (the residual then rides the product's epilogue).
+extern "C" int fa_linear_step(fa_ctx *ctx, const fa_tensor *x, const fa_tensor *gamma, const fa_tensor *beta, float eps,
+                              fa_tensor *w, fa_bytes *wq, const fa_tensor *scale, int N, int K, const fa_tensor *bias, int act,
+                              const fa_tensor *add, fa_tensor **out) {
+  if (!ctx || !out) return fa_fail(ctx, FA_ERR_INVALID, "linearStep: NULL argument");
+  FA_REQUIRE(ctx, fa_valid(ctx, x) && (w ? fa_valid(ctx, w) : fa_valid_bytes(ctx, wq)), "linearStep: unknown handle");
+  FA_REQUIRE(ctx, (gamma == nullptr) == (beta == nullptr), "linearStep: gamma and beta go together");
+  if (w) K = w->rows, N = w->cols;
+  auto al = [](const fa_tensor *t) { return ((uintptr_t)t->dptr & 15) == 0; };
+  const bool one = x->rows == 1 && x->cols == K && x->storage == FA_F32 && (!w || w->storage == FA_F16) && N > 0 && K > 0 &&
+                   gemv_shape_ok(ctx, 1, N, K) && fa_gemv_kn_ok(1, N, K) && act >= 0 && act <= 5 &&
+                   (w || wq->nbytes >= (size_t)N * K) && (!add || (add->rows == 1 && add->cols == N)) &&
+                   (!gamma || (fa_gemv_kn_norm_ok(K) && fa_valid(ctx, gamma) && fa_valid(ctx, beta) && al(x) && al(gamma) && al(beta)));
+  if (one) {
+    FA_TRY(check_vec(ctx, x, K, "linearStep: x"));
+    if (gamma) FA_TRY(check_vec(ctx, gamma, K, "linearStep: gamma"));
+    if (beta) FA_TRY(check_vec(ctx, beta, K, "linearStep: beta"));
+    if (!w) FA_TRY(check_vec(ctx, scale, N, "linearStep: scale"));
+    if (bias) FA_TRY(check_vec(ctx, bias, N, "linearStep: bias"));
+    if (add) FA_TRY(check_vec(ctx, add, N, "linearStep: add"));
+    FA_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
+    auto f = [](const fa_tensor *t) { return t ? (const float *)t->dptr : nullptr; };
+    fa_tensor *c = nullptr;
+    FA_TRY(fa_tensor_new(ctx, 1, N, FA_F32, true, &c));
+    const int rc = fa_gemv_kn(ctx, f(x), f(gamma), f(beta), eps, w ? w->dptr : wq->dptr, !w, w ? nullptr : f(scale), f(bias), act,
+                              f(add), (float *)c->dptr, N, K);
+    if (rc != FA_OK) fa_free_tensor(ctx, c);
+    else *out = c;
+    return rc;
+  }
+  fa_tensor *n = nullptr;
+  if (gamma) FA_TRY(fa_layernorm(ctx, x, gamma, beta, eps, &n));
+  const fa_tensor *a = n ? n : x;
+  const int rc = w ? fa_matmul(ctx, a, w, bias, act, add, out) : matmul_int8_impl(ctx, a, wq, scale, N, K, bias, act, add, out);
+  if (n) fa_free_tensor(ctx, n);
+  return rc;
+}
+
 // fa_matmul_int8's tensor-core route for a caller that has written the activation digit planes and the row scales
 // itself (the batched TDT joint): same product, same epilogue, no pass over the activations.
 bool fa_matmul_int8_planes_ok(fa_ctx *ctx, int M, int N, int K) {
-  return !(gemv_shape_ok(ctx, M, N, K) && fa_gemv_kn_ok(M, N, K, true)) && tc_shape_ok(ctx, M, N, K);
+  return !(gemv_shape_ok(ctx, M, N, K) && fa_gemv_kn_ok(M, N, K)) && tc_shape_ok(ctx, M, N, K);
 }
 int fa_matmul_int8_planes(fa_ctx *ctx, const int8_t *a_planes, const float *rowscale, int limbs, int M, fa_bytes *wq,
                           const float *colscale, int N, int K, const float *bias, float *c) {

@@ -62,12 +62,20 @@ def _mm(ctx, x, w: _W, bias=None, act="none"):
     return ctx.matmul(x, w.t, dict(bias=bias, act=act))
 
 
-def _mm_add(ctx, res, x, w: _W, bias=None):
-    """res + (x @ w + bias): the residual rides the product's epilogue where the member takes `add`
-    (matmul, compute.d.ts:155); same f32 sum as a separate add()."""
-    if w.quant == "int8":
-        return ctx.add(res, ctx.matmulInt8(x, w.q, w.s, w.N, w.K, bias=bias))
-    return ctx.matmul(x, w.t, dict(bias=bias, add=res))
+def _linear(ctx, x, w: _W, norm=None, bias=None, act="none", add=None):
+    """add + act(layernorm(x) @ w + bias), norm and add optional: one call (for a single row one launch) where the
+    backend has the member, the separate ops with the same sums otherwise."""
+    if hasattr(ctx, "linearStep"):
+        if w.quant == "int8":
+            return ctx.linearStep(x, w.q, w.s, w.N, w.K, norm=norm, bias=bias, act=act, add=add)
+        return ctx.linearStep(x, w.t, norm=norm, bias=bias, act=act, add=add)
+    if norm is not None:
+        x = ctx.layernorm(x, norm[0], norm[1])
+    if add is None:
+        return _mm(ctx, x, w, bias=bias, act=act)
+    if w.quant == "int8" or x.rows == 1:
+        return ctx.add(add, _mm(ctx, x, w, bias=bias, act=act))
+    return ctx.matmul(x, w.t, dict(bias=bias, act=act, add=add))  # the residual rides the epilogue (compute.d.ts:155)
 
 
 def load_decoder(ctx, weights: Dict[str, np.ndarray], NH: int, quant: Optional[str] = None) -> dict:
@@ -122,16 +130,17 @@ def load_decoder(ctx, weights: Dict[str, np.ndarray], NH: int, quant: Optional[s
                 lnf=(vec("lnf_w"), vec("lnf_b")), cfg=cfg)
 
 
-def _self_attention(ctx, h, w, cacheK, cacheV, n, S, D, NH, HD):
-    """The normed token rows h [S, D] -> attention over the S streams' caches [position, S*D], whose row n becomes the
+def _self_attention(ctx, x, w, cacheK, cacheV, n, S, D, NH, HD):
+    """The token rows x [S, D], normed -> attention over the S streams' caches [position, S*D], whose row n becomes the
     token's key and value (raw-whisper-decoder.js:112-124).  Only past+current exist, so there is no mask."""
     if "sqkvw" in w:
-        qkv = _mm(ctx, h, w["sqkvw"], bias=w["sqkvb"])
+        qkv = _linear(ctx, x, w["sqkvw"], norm=w["ln1"], bias=w["sqkvb"])
         att = ctx.attnStepAppend(qkv, cacheK, cacheV, n, NH, HD)
         if att is not None:
             return att
         q, k, v = (ctx.sliceCols(qkv, i * D, D) for i in range(3))
     else:
+        h = ctx.layernorm(x, *w["ln1"])
         q, k, v = _mm(ctx, h, w["sqw"], bias=w["sqb"]), _mm(ctx, h, w["skw"]), _mm(ctx, h, w["svw"], bias=w["svb"])
     flat = (lambda t: t) if S == 1 else (lambda t: ctx.reshapeView(t, 1, S * D))
     ctx.copyRows(cacheK, flat(k), n)
@@ -148,6 +157,15 @@ def _cross_attention(ctx, q, kv, S, NH, HD):
         probs = ctx.softmax(ctx.bmmQK(q, kv["k"], None, NH, HD, S))  # one window per stream: [S*NH, Tenc]
         att = ctx.bmmPV(probs, kv["v"], NH, HD, S)
     return att
+
+
+def _layer(ctx, x, w, kv, cacheK, cacheV, n, S, D, NH, HD):
+    """One decoder layer for the new token's rows x [S, D] (:110-137)."""
+    x = _linear(ctx, _self_attention(ctx, x, w, cacheK, cacheV, n, S, D, NH, HD), w["sow"], bias=w["sob"], add=x)
+    cq = _linear(ctx, x, w["cqw"], norm=w["ln2"], bias=w["cqb"])
+    x = _linear(ctx, _cross_attention(ctx, cq, kv, S, NH, HD), w["cow"], bias=w["cob"], add=x)
+    h = _linear(ctx, x, w["f1w"], norm=w["ln3"], bias=w["f1b"], act="gelu_erf")
+    return _linear(ctx, h, w["f2w"], bias=w["f2b"], add=x)
 
 
 # ---------------------------------------------------------------------------- one stream (reference form)
@@ -174,7 +192,6 @@ def decode_next(ctx, dec, kv, st, token: int) -> np.ndarray:
     """Feed one token through the cached decoder; logits [VOCAB] for it (:103-142)."""
     cfg = dec["cfg"]
     D, NH, HD, VOCAB = cfg["D"], cfg["NH"], cfg["HD"], cfg["VOCAB"]
-    ln = lambda x, lp: ctx.layernorm(x, lp[0], lp[1])
     n = st["n"]
     emb = dec["embed"][token] + dec["pos"][n]
     x = ctx.upload(emb, 1, D)
@@ -183,14 +200,9 @@ def decode_next(ctx, dec, kv, st, token: int) -> np.ndarray:
     def body():
         nonlocal x
         for li, w in enumerate(dec["layers"]):
-            att = _self_attention(ctx, ln(x, w["ln1"]), w, st["selfK"][li], st["selfV"][li], n, 1, D, NH, HD)
-            x = ctx.add(x, _mm(ctx, att, w["sow"], bias=w["sob"]))
-            cq = _mm(ctx, ln(x, w["ln2"]), w["cqw"], bias=w["cqb"])
-            x = ctx.add(x, _mm(ctx, _cross_attention(ctx, cq, kv[li], 1, NH, HD), w["cow"], bias=w["cob"]))
-            h = ln(x, w["ln3"])
-            x = ctx.add(x, _mm(ctx, _mm(ctx, h, w["f1w"], bias=w["f1b"], act="gelu_erf"), w["f2w"], bias=w["f2b"]))
+            x = _layer(ctx, x, w, kv[li], st["selfK"][li], st["selfV"][li], n, 1, D, NH, HD)
         st["n"] = n + 1
-        logits = _mm(ctx, ln(x, dec["lnf"]), dec["embedT"])  # [1, VOCABP]
+        logits = _linear(ctx, x, dec["embedT"], norm=dec["lnf"])  # [1, VOCABP]
         return ctx.stageDownload(logits)
 
     try:
@@ -248,15 +260,9 @@ def step_streams(ctx, dec, kv, st, x, n: int):
     cfg = dec["cfg"]
     D, NH, HD = cfg["D"], cfg["NH"], cfg["HD"]
     S = st["S"]
-    ln = lambda x, lp: ctx.layernorm(x, lp[0], lp[1])
     for li, w in enumerate(dec["layers"]):
-        att = _self_attention(ctx, ln(x, w["ln1"]), w, st["selfK"][li], st["selfV"][li], n, S, D, NH, HD)
-        x = _mm_add(ctx, x, att, w["sow"], bias=w["sob"])
-        cq = _mm(ctx, ln(x, w["ln2"]), w["cqw"], bias=w["cqb"])
-        x = _mm_add(ctx, x, _cross_attention(ctx, cq, kv[li], S, NH, HD), w["cow"], bias=w["cob"])
-        h = ln(x, w["ln3"])
-        x = _mm_add(ctx, x, _mm(ctx, h, w["f1w"], bias=w["f1b"], act="gelu_erf"), w["f2w"], bias=w["f2b"])
-    return _mm(ctx, ln(x, dec["lnf"]), dec["embedT"])
+        x = _layer(ctx, x, w, kv[li], st["selfK"][li], st["selfV"][li], n, S, D, NH, HD)
+    return _linear(ctx, x, dec["embedT"], norm=dec["lnf"])
 
 
 def decode_next_streams(ctx, dec, kv, st, tokens: Sequence[int], want_logits: bool = False):

@@ -255,6 +255,12 @@ int fa_conv2d(fa_ctx *ctx, const fa_tensor *x, const fa_tensor *w, const fa_tens
 int fa_bmm_qk(fa_ctx *ctx, const fa_tensor *q, const fa_tensor *b, const fa_tensor *qb, int H, int HD, int W,
               int b_shared, fa_tensor **out);                                             /* bmmQK :191 */
 int fa_bmm_pv(fa_ctx *ctx, const fa_tensor *p, const fa_tensor *v, int H, int HD, int W, fa_tensor **out); /* bmmPV :193 */
+/* One linear layer of a decoding step (optional member): add + act(layernorm(x) @ W + bias), gamma / beta, bias and add
+ * optional.  W is `w` (f16 or f32 storage, [K][N]) or, with w == NULL, the int8 payload wq + scale as in fa_matmul_int8.
+ * A single row is one launch; more rows run as the separate members. */
+int fa_linear_step(fa_ctx *ctx, const fa_tensor *x, const fa_tensor *gamma, const fa_tensor *beta, float eps, fa_tensor *w,
+                   fa_bytes *wq, const fa_tensor *scale, int N, int K, const fa_tensor *bias, int act, const fa_tensor *add,
+                   fa_tensor **out);
 /* Attention of one query per window in one pass (optional members of token-by-token decoding).
  * fa_attn_step: bmmPV(softmax(bmmQK(q, k)), v) for q [W, H*HD], k and v [W*Tk, H*HD].
  * fa_attn_step_append: the self-attention form.  qkv [S, 3*NH*HD] holds q | k | v of S streams' new token, the caches are
