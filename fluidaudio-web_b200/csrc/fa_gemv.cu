@@ -78,15 +78,14 @@ __device__ __forceinline__ void nbits_block(const uint4 (&wv)[R], const float (&
 // early is safe, while scales, zero-points and activations (tensors a kernel may have produced) are read after the
 // wait.  The stream over the weights - the whole cost of the product - thus runs under the predecessor's tail and
 // the prologue instead of after them (measured before the change: ~4 us of a 5.5 us launch had no weight byte in
-// flight, against 1.6 us of streaming).  PRE blocks per lane are requested early (64 blocks per row at K = 2048 =
-// 2 per lane); longer rows load the rest in the loop.
+// flight, against 1.6 us of streaming).  PRE blocks per lane and column are requested early, PRE * R the same for every
+// R: few columns on long rows (N = 2048, K = 8192) keep as many bytes in flight as many on short ones, see launch_nbits.
 // Prologue: a thread owns 8 consecutive k of one row, which is exactly one 32-bit word of the even-k digit plane and
 // one of the odd-k plane, so digits go to shared memory as whole words and the per-block digit sums are two shuffles.
-template <int M, int R>
+template <int M, int R, int PRE>
 __global__ void __launch_bounds__(kThreads, 2) k_gemv_nbits(const float *__restrict__ a, const uint8_t *__restrict__ bq,
                                                             const float *__restrict__ scales, const uint8_t *__restrict__ zp,
                                                             float *__restrict__ y, int N, int K, int nblk, int zpb) {
-  constexpr int PRE = 2;
   extern __shared__ __align__(16) unsigned char smem[];
   int8_t *dig = (int8_t *)smem;                     // [M][2] planes of K bytes: even-k words of every block (16 B
                                                     // each, so 8 lanes read 128 consecutive bytes), then odd-k words
@@ -434,15 +433,11 @@ __global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
   if (tid < kKnCols && n < N) p.y[n] = gemv_finish(sum, 0, n, N, p.ep);
 }
 
-template <int M>
-int launch_nbits(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y, int N,
-                 int K, int nblk, int zpb) {
+template <int M, int R, int PRE>
+int launch_nbits_r(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y, int N,
+                   int K, int nblk, int zpb) {
   const size_t smem = (size_t)M * 2 * K + (size_t)M * 2 * nblk * 4 + 8 * M * 4;
-  // output columns per warp pass (each digit load is shared between R rows of weights): 4 for one activation row -
-  // with two resident CTAs per SM (register cap 128) one wave then covers 148 * 2 * 8 * 4 = 9472 columns - and 2 for
-  // more rows, where 4 would not fit the registers next to the early-requested weights
-  constexpr int R = M == 1 ? 4 : 2;
-  auto kern = k_gemv_nbits<M, R>;
+  auto kern = k_gemv_nbits<M, R, PRE>;
   if (smem > 48 * 1024) FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // one resident wave: every CTA pays the digit prologue once and a second wave would pay it twice
   int per_sm = 0;
@@ -457,6 +452,24 @@ int launch_nbits(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *sc
   }
   FA_LAUNCH_CHECK(ctx, "gemv_nbits");
   return FA_OK;
+}
+
+// Output columns per warp pass (each digit load is shared between R rows of weights): 4 for one activation row - with two
+// resident CTAs per SM (register cap 128) one wave then covers 148 * 2 * 8 * 4 = 9472 columns - and 2 for more rows,
+// where 4 would not fit the registers next to the early-requested weights; fewer while the CTAs would not cover the SMs.
+// Measured at one row, K = 8192, N = 2048 in a recorded chain: 64 CTAs of 4 columns per warp 11.5 us, 256 of 1 column
+// 6.7 us (11 MB: 1.6 us of HBM time); N = 8192, K = 2048 keeps its 4 columns (4.2 us).
+template <int M>
+int launch_nbits(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y, int N,
+                 int K, int nblk, int zpb) {
+  if constexpr (M == 1) {
+    if (ceil_div(N, 8 * 4) >= ctx->sm_count) return launch_nbits_r<1, 4, 2>(ctx, a, bq, scales, zp, y, N, K, nblk, zpb);
+    if (ceil_div(N, 8 * 2) >= ctx->sm_count) return launch_nbits_r<1, 2, 4>(ctx, a, bq, scales, zp, y, N, K, nblk, zpb);
+    return launch_nbits_r<1, 1, 8>(ctx, a, bq, scales, zp, y, N, K, nblk, zpb);
+  } else {
+    if (ceil_div(N, 8 * 2) >= ctx->sm_count) return launch_nbits_r<M, 2, 2>(ctx, a, bq, scales, zp, y, N, K, nblk, zpb);
+    return launch_nbits_r<M, 1, 4>(ctx, a, bq, scales, zp, y, N, K, nblk, zpb);
+  }
 }
 
 }  // namespace
