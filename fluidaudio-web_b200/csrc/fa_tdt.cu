@@ -20,7 +20,11 @@
 // Six launches per round, each scheduled under its predecessor's tail (programmatic dependent launch).
 // The prediction network is evaluated for every window in every round: for a window that did not emit, its inputs
 // (committed state, last token) are unchanged, so the result is the same as the cached one the reference keeps.
-// A round is recorded once and replayed; the host looks at a device counter of finished windows every few rounds.
+// The host enqueues the launches directly, ahead of the device: a round's six take it less time than they take the device
+// (31 us for up to 32 windows), and recording a round to replay it cost 0.2-0.3 ms per decode plus ~6 us of idle device
+// between two replays.  How many rounds are still certain follows from the windows' positions (a round advances a window
+// by four frames at most); the positions are read back half-way through that many, under the other half, so that the
+// device neither waits for the host nor runs more than a few rounds past the end.
 // Gate nonlinearities are the crate's own exp / tanh approximations (lib.rs:49-68), evaluated with separate
 // multiplies and adds, so that the only difference from the reference is the summation order inside the products.
 #include "fa_internal.cuh"
@@ -142,8 +146,7 @@ __global__ void __launch_bounds__(kPickThreads) k_tdt_pick(const float *__restri
                                                            int *__restrict__ ids, int *__restrict__ frames,
                                                            float *__restrict__ h0t, const float *__restrict__ nh0t,
                                                            float *__restrict__ h1t, const float *__restrict__ nh1t, float *__restrict__ c0,
-                                                           float *__restrict__ c1, const float *__restrict__ nc0, const float *__restrict__ nc1,
-                                                           int *__restrict__ done_count) {
+                                                           float *__restrict__ c1, const float *__restrict__ nc0, const float *__restrict__ nc1) {
   static_assert(VOCAB == 8 * kPickThreads + 1 && HID <= kPickThreads, "eight logits per thread and one more for thread 0");
   __shared__ float sv[32];
   __shared__ int si[32];
@@ -211,7 +214,6 @@ __global__ void __launch_bounds__(kPickThreads) k_tdt_pick(const float *__restri
     else if (tok == BLANK || em >= MAX_SYMBOLS) { tn += 1; em = 0; }
     t[w] = tn;
     emitted[w] = em;
-    if (tn >= T) atomicAdd(done_count, 1);
     s_tok = tok;
   }
   __syncthreads();
@@ -474,6 +476,10 @@ struct fa_tdt {
   fa_tensor *gate_tab = nullptr, *wr[2] = {nullptr, nullptr}, *bsum1 = nullptr, *pred_w = nullptr, *pred_b = nullptr;
   fa_tensor *out_b = nullptr, *out_scale = nullptr, *ones = nullptr, *out_w = nullptr;
   fa_bytes *out_q = nullptr;
+  // the decode loop's read-back: page-locked copy of the windows' positions (grown to the largest W seen) and its event
+  int *t_host = nullptr;
+  int t_cap = 0;
+  cudaEvent_t t_read = nullptr;
 };
 
 static void tdt_release(fa_ctx *ctx, fa_tdt *d) {
@@ -481,6 +487,8 @@ static void tdt_release(fa_ctx *ctx, fa_tdt *d) {
   for (fa_tensor *t : ts)
     if (t) fa_free_tensor(ctx, t);
   if (d->out_q) fa_free_bytes(ctx, d->out_q);
+  if (d->t_host) cudaFreeHost(d->t_host);
+  if (d->t_read) cudaEventDestroy(d->t_read);
   delete d;
 }
 
@@ -570,13 +578,14 @@ extern "C" int fa_tdt_free(fa_ctx *ctx, fa_tdt *d) {
 namespace {
 
 struct TdtState {
-  // chunk-transposed [ceil(W/32)][HID][32]: committed and candidate hidden states
-  fa_tensor *h0t = nullptr, *nh0t = nullptr, *h1t = nullptr, *nh1t = nullptr;
-  fa_tensor *c0 = nullptr, *c1 = nullptr, *nc0 = nullptr, *nc1 = nullptr, *predproj = nullptr, *J = nullptr;  // [W][HID]
+  fa_tensor *state = nullptr;  // every recurrent vector below, one block, cleared by one memset
+  // chunk-transposed [ceil(W/32)][HID][32]: committed and candidate hidden states; [W][HID]: cell states
+  float *h0t = nullptr, *nh0t = nullptr, *h1t = nullptr, *nh1t = nullptr, *c0 = nullptr, *c1 = nullptr, *nc0 = nullptr, *nc1 = nullptr;
+  fa_tensor *predproj = nullptr, *J = nullptr;   // [W][HID]
   fa_tensor *logits = nullptr;                   // [W][LOGITS] when the joint's digit planes are written here
   void *planes = nullptr, *rowscale = nullptr;   // the int8 product's row operand (see k_tdt_joint_digits)
   size_t planes_bytes = 0, rowscale_bytes = 0;
-  void *ints = nullptr;  // t, emitted, last_tok, counts [W each], done_count, then ids and frames [W*cap each]
+  void *ints = nullptr;  // t, emitted, last_tok, counts [W each], then ids and frames [W*cap each]
   size_t ints_bytes = 0;
 };
 
@@ -602,15 +611,15 @@ int tdt_predict(fa_ctx *ctx, fa_tdt *d, TdtState &s, int W, const int *last_tok)
   const int withhold = ctx->tc_withhold_chunk;
   ctx->tc_withhold_chunk = -1;  // one launch only
   RowsParams p{};
-  p.xa = (const float *)s.h0t->dptr, p.xb = p.xa, p.wt = (const float *)d->wr[0]->dptr;
+  p.xa = s.h0t, p.xb = p.xa, p.wt = (const float *)d->wr[0]->dptr;
   p.tab = (const float *)d->gate_tab->dptr, p.last_tok = last_tok;
-  p.c = (const float *)s.c0->dptr, p.nc = (float *)s.nc0->dptr, p.nht = (float *)s.nh0t->dptr;
+  p.c = s.c0, p.nc = s.nc0, p.nht = s.nh0t;
   FA_TRY(tdt_rows<2>(ctx, p, HID / 5, W, withhold));
-  p.xa = (const float *)s.nh0t->dptr, p.xb = (const float *)s.h1t->dptr, p.wt = (const float *)d->wr[1]->dptr;
-  p.bias = (const float *)d->bsum1->dptr, p.c = (const float *)s.c1->dptr, p.nc = (float *)s.nc1->dptr, p.nht = (float *)s.nh1t->dptr;
+  p.xa = s.nh0t, p.xb = s.h1t, p.wt = (const float *)d->wr[1]->dptr;
+  p.bias = (const float *)d->bsum1->dptr, p.c = s.c1, p.nc = s.nc1, p.nht = s.nh1t;
   FA_TRY(tdt_rows<1>(ctx, p, HID / 5, W, -1));
   RowsParams q{};
-  q.xa = (const float *)s.nh1t->dptr, q.xb = q.xa, q.wt = (const float *)d->pred_w->dptr, q.bias = (const float *)d->pred_b->dptr;
+  q.xa = s.nh1t, q.xb = q.xa, q.wt = (const float *)d->pred_w->dptr, q.bias = (const float *)d->pred_b->dptr;
   q.out = (float *)s.predproj->dptr;
   FA_TRY(tdt_rows<0>(ctx, q, HID / kRowsCols, W, -1));
   FA_LAUNCH_CHECK(ctx, "tdt_predict");
@@ -618,8 +627,8 @@ int tdt_predict(fa_ctx *ctx, fa_tdt *d, TdtState &s, int W, const int *last_tok)
 }
 
 int tdt_round(fa_ctx *ctx, fa_tdt *d, TdtState &s, const fa_tensor *proj, int W, int T, int cap) {
-  int *t = (int *)s.ints, *emitted = t + W, *last_tok = t + 2 * W, *counts = t + 3 * W, *done = t + 4 * W;
-  int *ids = done + 4, *frames = ids + (size_t)W * cap;
+  int *t = (int *)s.ints, *emitted = t + W, *last_tok = t + 2 * W, *counts = t + 3 * W;
+  int *ids = t + 4 * W, *frames = ids + (size_t)W * cap;
   fa_tensor *logits = nullptr;
   if (s.planes) {
     {
@@ -645,10 +654,10 @@ int tdt_round(fa_ctx *ctx, fa_tdt *d, TdtState &s, const fa_tensor *proj, int W,
   {
     LaunchScope ls(ctx, "tdt_pick");
     FA_CHECK_CUDA(ctx, fa_launch_dep(ctx, k_tdt_pick, dim3(W), dim3(kPickThreads), 0, lg, LOGITS, T, cap, t, emitted, last_tok, counts,
-                                     ids, frames, (float *)s.h0t->dptr,
-                                     (const float *)s.nh0t->dptr, (float *)s.h1t->dptr, (const float *)s.nh1t->dptr,
-                                     (float *)s.c0->dptr, (float *)s.c1->dptr, (const float *)s.nc0->dptr,
-                                     (const float *)s.nc1->dptr, done));
+                                     ids, frames, s.h0t,
+                                     s.nh0t, s.h1t, s.nh1t,
+                                     s.c0, s.c1, s.nc0,
+                                     s.nc1));
   }
   if (logits) FA_TRY(fa_free_tensor(ctx, logits));
   FA_LAUNCH_CHECK(ctx, "tdt_round");
@@ -672,53 +681,71 @@ extern "C" int fa_tdt_decode_proj(fa_ctx *ctx, fa_tdt *d, const fa_tensor *proj,
   TdtState s;
   const int saved_limbs = ctx->int8_limbs;
   ctx->int8_limbs = 3;  // f32-grade activations for the joint's int8 product: token picks follow the f32 reference
-  fa_graph *graph = nullptr;
   int rc = FA_OK, rounds = 0;
   auto alloc = [&](int r, int c, fa_tensor **t) { return rc == FA_OK ? (rc = fa_alloc(ctx, r, c, t)) : rc; };
   const int wpad = ceil_div(W, 32) * 32;
-  alloc(wpad, HID, &s.h0t), alloc(wpad, HID, &s.nh0t), alloc(wpad, HID, &s.h1t), alloc(wpad, HID, &s.nh1t),
-      alloc(W, HID, &s.c0), alloc(W, HID, &s.c1), alloc(W, HID, &s.nc0), alloc(W, HID, &s.nc1), alloc(W, HID, &s.predproj),
-      alloc(W, HID, &s.J);
-  const size_t n_int = (size_t)4 * W + 4 + (size_t)2 * W * cap;
+  alloc(4 * wpad + 4 * W, HID, &s.state), alloc(W, HID, &s.predproj), alloc(W, HID, &s.J);
+  const size_t n_int = (size_t)4 * W + (size_t)2 * W * cap;
   if (rc == FA_OK) rc = fa_block_acquire(ctx, n_int * 4, &s.ints, &s.ints_bytes);
   if (rc == FA_OK && d->out_q && fa_matmul_int8_planes_ok(ctx, W, LOGITS, HID)) {
     alloc(W, LOGITS, &s.logits);
     if (rc == FA_OK) rc = fa_block_acquire(ctx, fa_tc_act_bytes(W, HID, 1, ctx->int8_limbs), &s.planes, &s.planes_bytes);
     if (rc == FA_OK) rc = fa_block_acquire(ctx, (size_t)W * 4, &s.rowscale, &s.rowscale_bytes);
   }
-  int *t = (int *)s.ints, *last_tok = t + 2 * W, *done = t + 4 * W;
+  if (rc == FA_OK && d->t_cap < W) {
+    if (d->t_host) cudaFreeHost(d->t_host);
+    d->t_host = nullptr, d->t_cap = 0;
+    cudaError_t e = cudaHostAlloc(&d->t_host, (size_t)W * 4, cudaHostAllocDefault);
+    if (e == cudaSuccess && !d->t_read) e = cudaEventCreateWithFlags(&d->t_read, cudaEventDisableTiming);
+    if (e != cudaSuccess) rc = fa_fail(ctx, FA_ERR_CUDA, "tdtDecodeProj: %s", cudaGetErrorString(e));
+    else d->t_cap = W;
+  }
+  int *t = (int *)s.ints, *last_tok = t + 2 * W;
   if (rc == FA_OK) {
+    float *base = (float *)s.state->dptr;
+    const size_t hs = (size_t)wpad * HID, cs = (size_t)W * HID;
+    s.h0t = base, s.nh0t = base + hs, s.h1t = base + 2 * hs, s.nh1t = base + 3 * hs;
+    s.c0 = base + 4 * hs, s.c1 = s.c0 + cs, s.nc0 = s.c0 + 2 * cs, s.nc1 = s.c0 + 3 * cs;
     // decode_proj :290-294: zero state, last token = blank, predict + predproj once
-    fa_tensor *z[] = {s.h0t, s.nh0t, s.h1t, s.nh1t, s.c0, s.c1, s.nc0, s.nc1};
-    for (fa_tensor *x : z) cudaMemsetAsync(x->dptr, 0, (size_t)x->rows * x->cols * 4, ctx->stream);
-    cudaMemsetAsync(s.ints, 0, n_int * 4, ctx->stream);
+    cudaError_t e = cudaMemsetAsync(base, 0, (4 * hs + 4 * cs) * 4, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s.ints, 0, n_int * 4, ctx->stream);
+    if (e != cudaSuccess) rc = fa_fail(ctx, FA_ERR_CUDA, "tdtDecodeProj: %s", cudaGetErrorString(e));
+  }
+  if (rc == FA_OK) {
     k_fill_int<<<ceil_div(W, 256), 256, 0, ctx->stream>>>(last_tok, W, BLANK);
     rc = tdt_predict(ctx, d, s, W, last_tok);
   }
-  // one round eagerly (first-use caches of the weights), then the round as a recorded batch, replayed
-  if (rc == FA_OK) rc = tdt_round(ctx, d, s, proj, W, T, cap);
-  rounds = 1;
-  if (rc == FA_OK) rc = fa_graph_begin(ctx);
-  if (rc == FA_OK) {
-    rc = tdt_round(ctx, d, s, proj, W, T, cap);
-    fa_graph *g = nullptr;
-    const int rc2 = fa_graph_end(ctx, &g);
-    if (rc == FA_OK) rc = rc2;
-    graph = g;
-  }
-  int done_host = 0;
-  const int max_rounds = T * (MAX_SYMBOLS + 1) + 2, check_every = 16;
+  const int max_rounds = T * (MAX_SYMBOLS + 1) + 2, max_step = LOGITS - VOCAB - 1, min_rounds = 4;
+  int done_host = 0, sure = ceil_div(T, max_step);  // rounds that the window furthest behind still needs at least
+  auto run = [&](int n) {
+    for (; n > 0 && rc == FA_OK; n--, rounds++) rc = tdt_round(ctx, d, s, proj, W, T, cap);
+  };
   while (rc == FA_OK && done_host < W && rounds < max_rounds) {
-    for (int i = 0; i < check_every && rc == FA_OK; i++, rounds++) rc = fa_graph_launch(ctx, graph);
+    const int n = sure > min_rounds ? sure : min_rounds, first = (n + 1) / 2;
+    run(first);
     if (rc == FA_OK) {
-      cudaError_t e = cudaMemcpyAsync(&done_host, done, 4, cudaMemcpyDeviceToHost, ctx->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+      cudaError_t e = cudaMemcpyAsync(d->t_host, t, (size_t)W * 4, cudaMemcpyDeviceToHost, ctx->stream);
+      if (e == cudaSuccess) e = cudaEventRecord(d->t_read, ctx->stream);
       if (e != cudaSuccess) rc = fa_fail(ctx, FA_ERR_CUDA, "tdtDecodeProj: %s", cudaGetErrorString(e));
     }
+    const int second = sure > first ? sure - first : 0;  // certain to be needed as well: they run under the read-back
+    run(second);
+    if (rc == FA_OK) {
+      const cudaError_t e = cudaEventSynchronize(d->t_read);
+      if (e != cudaSuccess) rc = fa_fail(ctx, FA_ERR_CUDA, "tdtDecodeProj: %s", cudaGetErrorString(e));
+    }
+    if (rc != FA_OK) break;
+    int behind = T;
+    done_host = 0;
+    for (int w = 0; w < W; w++) {
+      if (d->t_host[w] >= T) done_host++;
+      else if (d->t_host[w] < behind) behind = d->t_host[w];
+    }
+    sure = ceil_div(T - behind, max_step) - second;
   }
   if (rc == FA_OK && done_host < W) rc = fa_fail(ctx, FA_ERR_INVALID, "tdtDecodeProj: %d of %d windows unfinished after %d rounds", W - done_host, W, rounds);
   if (rc == FA_OK) {
-    int *counts = t + 3 * W, *ids = done + 4, *frames = ids + (size_t)W * cap;
+    int *counts = t + 3 * W, *ids = t + 4 * W, *frames = ids + (size_t)W * cap;
     cudaError_t e = cudaMemcpyAsync(counts_host, counts, (size_t)W * 4, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ids_host, ids, (size_t)W * cap * 4, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(frames_host, frames, (size_t)W * cap * 4, cudaMemcpyDeviceToHost, ctx->stream);
@@ -726,7 +753,6 @@ extern "C" int fa_tdt_decode_proj(fa_ctx *ctx, fa_tdt *d, const fa_tensor *proj,
     if (rc == FA_OK) rc = fa_sync(ctx);
   }
   const std::string msg = ctx->err;
-  if (graph) fa_graph_free(ctx, graph);
   if (s.ints) fa_block_release(ctx, s.ints);
   if (s.planes) fa_block_release(ctx, s.planes);
   if (s.rowscale) fa_block_release(ctx, s.rowscale);
