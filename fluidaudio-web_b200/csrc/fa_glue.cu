@@ -1136,33 +1136,51 @@ __global__ void __launch_bounds__(256, 4) k_conv2d_c1_3x3(const float *__restric
 }
 
 // Per-row argmax: out[r] = {index, value}; ties resolve to the lowest index like the host loop
-// of src/engines/asr-whisper/index.ts:80-97.
-__global__ void __launch_bounds__(256) k_argmax_rows(const float *__restrict__ x, float *__restrict__ out, int R, int ld,
-                                                     int C) {
+// of src/engines/asr-whisper/index.ts:80-97.  One block of 32 warps per row, eight loads of a thread in flight: a row is
+// too short to split (207 KB at 51866 columns) and what bounds it is the latency of its loads, one batch after another.
+// Measured, 64 rows of 51866 columns: 33 us with 256 threads and one load in flight each, under 10 us so.
+constexpr int kArgThreads = 1024, kArgBatch = 8;
+__global__ void __launch_bounds__(kArgThreads) k_argmax_rows(const float *__restrict__ x, float *__restrict__ out, int R, int ld,
+                                                             int C) {
   fa_grid_dep_sync();
-  __shared__ float bv[8];
-  __shared__ int bi[8];
+  __shared__ float bv[kArgThreads / 32];
+  __shared__ int bi[kArgThreads / 32];
+  auto better = [](float v, int j, float best, int idx) { return v > best || (v == best && j < idx); };
   for (int r = blockIdx.x; r < R; r += gridDim.x) {
     const float *row = x + (size_t)r * ld;
     float best = -INFINITY;
     int idx = 0x7fffffff;
-    for (int j = threadIdx.x; j < C; j += 256) {
-      float v = row[j];
-      if (v > best || (v == best && j < idx)) { best = v; idx = j; }
-    }
+    for (int j0 = threadIdx.x; j0 < C; j0 += kArgThreads * kArgBatch) {
+      float v[kArgBatch];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-      if (ov > best || (ov == best && oi < idx)) { best = ov; idx = oi; }
+      for (int u = 0; u < kArgBatch; u++) {
+        const int j = j0 + u * kArgThreads;
+        v[u] = j < C ? row[j] : -INFINITY;
+      }
+#pragma unroll
+      for (int u = 0; u < kArgBatch; u++) {
+        const int j = j0 + u * kArgThreads;
+        if (j < C && better(v[u], j, best, idx)) { best = v[u]; idx = j; }
+      }
     }
+    auto warp_best = [&]() {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+        if (better(ov, oi, best, idx)) { best = ov; idx = oi; }
+      }
+    };
+    warp_best();
     if ((threadIdx.x & 31) == 0) { bv[threadIdx.x >> 5] = best; bi[threadIdx.x >> 5] = idx; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 1; w < 8; w++)
-        if (bv[w] > bv[0] || (bv[w] == bv[0] && bi[w] < bi[0])) { bv[0] = bv[w]; bi[0] = bi[w]; }
-      out[(size_t)r * 2] = (float)bi[0];
-      out[(size_t)r * 2 + 1] = bv[0];
+    if (threadIdx.x < 32) {
+      best = bv[threadIdx.x], idx = bi[threadIdx.x];
+      warp_best();
+      if (threadIdx.x == 0) {
+        out[(size_t)r * 2] = (float)idx;
+        out[(size_t)r * 2 + 1] = best;
+      }
     }
     __syncthreads();
   }
@@ -2221,7 +2239,7 @@ extern "C" int fa_argmax_rows(fa_ctx *ctx, const fa_tensor *x, int ncols, fa_ten
     int grid = x->rows < ctx->sm_count * 8 ? x->rows : ctx->sm_count * 8;
     {
       LaunchScope ls(ctx, "argmax_rows");
-      fa_launch_dep(ctx, k_argmax_rows, dim3(grid), dim3(256), 0, (const float *)x->dptr, (float *)y->dptr, x->rows, x->cols, ncols);
+      fa_launch_dep(ctx, k_argmax_rows, dim3(grid), dim3(kArgThreads), 0, (const float *)x->dptr, (float *)y->dptr, x->rows, x->cols, ncols);
     }
     FA_LAUNCH_CHECK(ctx, "argmax_rows");
   }
