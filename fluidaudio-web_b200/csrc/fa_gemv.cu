@@ -307,7 +307,7 @@ __device__ __forceinline__ float block_sum(float v, float *red, int lane, int wa
 // What bounds it: the weight stream of the large matrices (66 MB of int8 for the vocabulary projection), latency for the
 // others: 1.6 MB are 0.3 us of HBM time, so the launch is a chain of load -> row sum -> exchange between K slices.
 // Hence the layout: a block owns 128 columns (one 4-byte int8 or 8-byte f16 load per lane and row) and a K slice, its
-// 8 warps take rows round-robin with kKnU loads per lane in flight, the first of them requested before the launch waits
+// 8 warps take rows round-robin with two batches of kKnU loads per lane in flight, the first ones requested before the launch waits
 // for its predecessor where the weights can only have been written by an upload (int8 payloads).  K slices are the
 // ranks of a cluster: their sums meet in rank 0's shared memory, in rank order, after one cluster barrier.  (The form
 // before this one let the slices meet in global memory behind a ticket, up to 40 partial rows read by the last block.)
@@ -315,7 +315,7 @@ __device__ __forceinline__ float block_sum(float v, float *red, int lane, int wa
 // layernorm, product and residual add were three launches; 1280 x 51868 int8 with the layernorm 25 us (2.7 TB/s) against
 // a layernorm, a digit pass and a tensor-core product of 3.8 + 2.6 + 12.5 us that read the row as two int8 digits
 // instead of f32.  A 16-token decoder pass of one stream: 8.24 -> 5.1 ms, what is left is the host's 9 us per launch.
-constexpr int kKnU = 16, kKnCols = 128, kKnSlice = 2048;  // loads in flight per lane, columns per block, rows of x held at a time
+constexpr int kKnU = 16, kKnCols = 128, kKnSlice = 2048;  // loads in a lane's batch, columns per block, rows of x held at a time
 constexpr int kKnNormMax = 4096;                           // longest row that the layernorm prologue holds in registers
 
 struct KnParams {
@@ -339,8 +339,8 @@ __global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
   const int c0 = blockIdx.x * kKnCols + lane * 4;
   const bool live = c0 < N;  // N % 4 == 0: a live lane owns four whole columns
   const int cc = live ? c0 : 0;
-  Raw raw[kKnU];
-  auto fetch = [&](int kk) {
+  Raw ra[kKnU], rb[kKnU];
+  auto fetch = [&](Raw(&raw)[kKnU], int kk) {
 #pragma unroll
     for (int u = 0; u < kKnU; u++) {
       const int k = kk + u * 8;
@@ -349,10 +349,10 @@ __global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
     }
   };
   int kk = k0 + warp;  // rows kk, kk + 8, ...
-  if (I8) fetch(kk);
+  if (I8) fetch(ra, kk), fetch(rb, kk + 8 * kKnU);
   if (ks > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // every rank runs before a remote store
   fa_grid_dep_sync();
-  if (!I8) fetch(kk);
+  if (!I8) fetch(ra, kk), fetch(rb, kk + 8 * kKnU);
   if (NORM) {
     float4 v[kKnNormMax / 4 / kThreads];
     const int k4 = K >> 2;
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
       for (int i = tid; i < end - base; i += kThreads) xs[i] = p.x[base + i];
       __syncthreads();
     }
-    while (kk < end) {  // a batch never straddles `end` on its way: kKnSlice % (8 * kKnU) == 0
+    auto consume = [&](const Raw(&raw)[kKnU], int kk) {
 #pragma unroll
       for (int u = 0; u < kKnU; u++) {
         const int k = kk + u * 8;
@@ -401,8 +401,12 @@ __global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
           acc.x = fmaf(a, f.x, acc.x), acc.y = fmaf(a, f.y, acc.y), acc.z = fmaf(a, f.z, acc.z), acc.w = fmaf(a, f.w, acc.w);
         }
       }
-      kk += 8 * kKnU;
-      if (kk < k1) fetch(kk);
+    };
+    for (; kk < end; kk += 16 * kKnU) {  // no pair of batches straddles `end` on its way: kKnSlice % (16 * kKnU) == 0
+      consume(ra, kk);
+      if (kk + 16 * kKnU < k1) fetch(ra, kk + 16 * kKnU);
+      consume(rb, kk + 8 * kKnU);
+      if (kk + 24 * kKnU < k1) fetch(rb, kk + 24 * kKnU);
     }
   }
   red[warp][lane] = acc;
