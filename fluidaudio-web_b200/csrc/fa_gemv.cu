@@ -493,22 +493,33 @@ int fa_gemv_nbits(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *s
   }
 }
 
-// ---- int4, 5..16 activation rows: weights streamed once as uploaded, dequantised in registers, mma.sync -------------
-// The tensor-core GEMM serves these shapes from a dequantised f16 copy of the weights (4x the bytes of the 4-bit
-// matrix) and pays cluster set-up, a packing prepass and a split-K hand-off for ~0.5 GFLOP of work.  Here a CTA owns
-// groups of 8 output columns; its 16 warps split the K blocks of a group between them (a warp takes 4 consecutive
-// 32-weight blocks, one per lane of a column's 4-lane group, as ONE 16-byte load per lane, so the 4 lanes of a column
-// read 64 consecutive bytes), widens its nibbles to f16 with (q - zp) * scale, and multiplies them as the B fragment
-// of mma.sync.m16n8k16 against all (up to 16) activation rows at once; partial sums of the 16 warps meet in shared
-// memory.  Which K index sits in which of the instruction's 16 k-slots does not matter for a sum, so a lane uses the
-// nibbles in the order one mask extracts them (k, k+4 of every group of 8), and the activation rows are stored in
-// shared memory in that same order (f16 value plane and, optionally, the rounding-residue plane that keeps f32-grade
-// activations) with a row pitch and block pitch that make the A-fragment loads conflict-free.
-constexpr int kMmaWarps = 16;
-constexpr int kMmaBatch = 4;   // column groups whose partial tiles are reduced together (one pair of block barriers)
-constexpr int kMmaSeg = 80;    // bytes per 32-k block of an activation row in shared memory (64 + 16: the 4 lanes of a
-                               // column group read blocks b..b+3 of a row at 16-byte bank groups 0, 5, 2, 7)
-__host__ __device__ constexpr int mma_row_pitch(int nblk) { return nblk * kMmaSeg + (((nblk * kMmaSeg / 16) % 8) == 4 ? 0 : ((4 - (nblk * kMmaSeg / 16) % 8 + 8) % 8) * 16); }
+namespace {
+
+// ---- int4, 5..16 activation rows: weights streamed once as uploaded, widened in registers, mma.sync -------------------
+// The tensor-core GEMM serves these shapes from a dequantised f16 copy of the weights: four times the bytes, a packing
+// prepass and a split-K hand-off for ~0.5 GFLOP of work, and weights (q - zp) * scale rounded to f16.  Here the 4-bit
+// weights are read once, in the layout they were uploaded in, and the block scale multiplies the block's f32 sum, so that
+// the weights stay exact.
+//
+// What bounds it: instruction issue.  A warp owns ONE quad of 32-weight blocks (16 warps x 4 blocks = the 2048 k that the
+// activation planes of 16 rows leave room for in shared memory) and walks up to G groups of 8 output columns with it:
+//   - a lane loads one whole block per group (16 bytes; the 4 lanes of a column read 64 consecutive bytes), all groups up
+//     front, before the launch waits for its predecessor (the payload is only ever written by an upload);
+//   - a 4 x 4 transpose between the 4 lanes of a column (4 shuffles) gives each lane word j of all four blocks, so that
+//     one mma.sync.m16n8k16 works inside ONE block and the scale can wait for its result;
+//   - a nibble pair (k, k + 4) becomes two f16 `1024 + q` with one mask, minus 1024 + zp: exact.  Which k sits in which of
+//     the instruction's slots does not matter for a sum; the activation rows lie in shared memory in the same order, a
+//     lane's 8 values of a block as one 16-byte load (row pitch = 64 mod 128 bytes: conflict-free), and are read once per
+//     block for all groups;
+//   - per block and group: 4 mma (value and residue plane of the activations), then 4 multiply-adds with the scale.
+// The 16 warps' sums meet in shared memory in warp order; K beyond 2048 is split over the ranks of a cluster, whose sums
+// meet in rank 0's shared memory in rank order.
+// Measured, 16 rows, recorded blocks: N = 8192, K = 2048 12.4 us and N = 2048, K = 8192 14.7 us, against 14.1 and 20.0 us (digit
+// pass included) for the f16 copy on the tensor cores, which read 33.5 MB where this reads 10.5.
+constexpr int kMmaWarps = 16, kMmaThreads = kMmaWarps * 32;
+constexpr int kMmaSliceBlk = kMmaWarps * 4;  // 32-weight blocks per K slice
+constexpr int kMmaMaxSlices = 4;
+__host__ __device__ constexpr int mma_row_pitch(int blks) { return blks * 64 + ((blks & 1) ? 0 : 64); }
 
 __device__ __forceinline__ void mma16816_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -516,188 +527,247 @@ __device__ __forceinline__ void mma16816_f16(float (&c)[4], uint32_t a0, uint32_
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <bool HILO>
-__global__ void __launch_bounds__(kMmaWarps * 32, 1) k_nbits_mma(const float *__restrict__ a, const uint8_t *__restrict__ bq,
-                                                                  const float *__restrict__ scales, const uint8_t *__restrict__ zp,
-                                                                  float *__restrict__ y, int M, int N, int K, int nblk, int zpb) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int pitch = mma_row_pitch(nblk);
-  unsigned char *planes = smem;                                         // [HILO ? 2 : 1][16][pitch]
-  float *red = (float *)(smem + (size_t)(HILO ? 2 : 1) * 16 * pitch);   // [kMmaBatch][kMmaWarps][32][4]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int groups = N >> 3, quads = (nblk + 3) >> 2;
-  const uint4 *bq4 = (const uint4 *)bq;
-  constexpr int D = kMmaBatch;  // column groups whose weights are requested ahead: slot gi of the registers below always
-                                // serves the gi-th group of a batch, so a value still in flight is never moved
+struct MmaParams {
+  const float *a;
+  const uint8_t *bq;
+  const float *scales;
+  const uint8_t *zp;
+  float *y;
+  int M, N, K, nblk, zpb;
+  int slice;  // blocks per K slice (a multiple of 4, at most kMmaSliceBlk)
+  int gper;   // column groups per thread block
+};
 
-  // requests of this warp's first quad of the first D column groups (weights do not depend on earlier kernels)
+// Lane j of 4 holds words 0..3 of block j; afterwards word j of blocks 0..3.
+__device__ __forceinline__ void transpose4(uint4 &w, int lane) {
+  const bool o1 = lane & 1, o2 = lane & 2;
+  unsigned t = __shfl_xor_sync(0xffffffffu, o1 ? w.x : w.y, 1);
+  if (o1) w.x = t; else w.y = t;
+  t = __shfl_xor_sync(0xffffffffu, o1 ? w.z : w.w, 1);
+  if (o1) w.z = t; else w.w = t;
+  t = __shfl_xor_sync(0xffffffffu, o2 ? w.x : w.z, 2);
+  if (o2) w.x = t; else w.z = t;
+  t = __shfl_xor_sync(0xffffffffu, o2 ? w.y : w.w, 2);
+  if (o2) w.y = t; else w.w = t;
+}
+
+template <bool HILO, int G>
+__global__ void __launch_bounds__(kMmaThreads, 1) k_nbits_mma(const MmaParams p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g4 = lane >> 2, j4 = lane & 3;
+  const int rank = blockIdx.y, slices = gridDim.y, b0 = rank * p.slice, nb = min(p.slice, p.nblk - b0);  // blocks of this slice
+  const int pitch = mma_row_pitch(p.slice);
+  unsigned char *ap = smem;                                                     // [planes][16 rows][pitch]
+  float4 *red = (float4 *)(smem + (size_t)(HILO ? 2 : 1) * 16 * pitch);         // [16 warps][G][32]
+  float4 *cred = red + kMmaWarps * G * 32;                                      // rank 0: [2][slices][G][32]
+  const int qb = b0 + warp * 4;         // first block of the warp's quad
+  const int qn = min(4, b0 + nb - qb);  // its blocks (<= 0: none)
+  const int groups = p.N >> 3, gfirst = blockIdx.x * p.gper, gend = min(groups, gfirst + p.gper);
+  const uint4 *bq4 = (const uint4 *)p.bq;
+
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  uint4 pw[D];
-  float psc[D];
-  unsigned pzb[D];
+  uint4 w[G];
+  auto fetch = [&](int g0) {
 #pragma unroll
-  for (int d = 0; d < D; d++) {
-    const int cg = blockIdx.x + d * gridDim.x, b = 4 * warp + t;
-    const bool ok = cg < groups && b < nblk;
-    const size_t n = (size_t)(cg * 8 + g);
-    pw[d] = ok ? __ldcs(bq4 + n * nblk + b) : make_uint4(0u, 0u, 0u, 0u);
-    psc[d] = ok ? __ldg(scales + n * nblk + b) : 0.f;
-    pzb[d] = ok ? (unsigned)__ldg(zp + n * zpb + (b >> 1)) : 0u;
-  }
+    for (int g = 0; g < G; g++) {
+      w[g] = make_uint4(0u, 0u, 0u, 0u);
+      if (g0 + g < gend && j4 < qn) w[g] = __ldcs(bq4 + (size_t)((g0 + g) * 8 + g4) * p.nblk + qb + j4);
+    }
+  };
+  fetch(gfirst);
+  if (slices > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // every rank runs before a remote store
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  // ---- activation rows -> f16 planes, 8 consecutive k per thread, stored k0,k4,k1,k5,k2,k6,k3,k7 ----
-  const int words = nblk * 4;
-  unsigned any_residue = 0u;
-  const bool avec = (K & 7) == 0 && ((uintptr_t)a & 15) == 0;  // rows start 16-byte aligned: two float4 per word
-  for (int e = tid; e < 16 * words; e += kMmaWarps * 32) {
-    const int m = e / words, w = e - m * words, k0 = w * 8;
-    float x[8];
-    if (avec && m < M && k0 + 8 <= K) {
-      const float4 x0 = __ldg((const float4 *)(a + (size_t)m * K + k0)), x1 = __ldg((const float4 *)(a + (size_t)m * K + k0 + 4));
-      x[0] = x0.x, x[1] = x0.y, x[2] = x0.z, x[3] = x0.w, x[4] = x1.x, x[5] = x1.y, x[6] = x1.z, x[7] = x1.w;
-    } else {
+  // activation rows of this K slice: 8 consecutive k of one row per step, as halves k0,k4,k1,k5,k2,k6,k3,k7; a thread
+  // requests four steps before it converts the first (every block reads all the rows: 131 KB at 16 x 2048)
+  const bool quads = (p.K & 3) == 0;
+  for (int i0 = tid; i0 < 16 * p.slice * 4; i0 += 4 * kMmaThreads) {
+    float x[4][8];
 #pragma unroll
-      for (int i = 0; i < 8; i++) x[i] = (m < M && k0 + i < K) ? __ldg(a + (size_t)m * K + k0 + i) : 0.f;
+    for (int s = 0; s < 4; s++) {
+      const int i = i0 + s * kMmaThreads, m = i / (p.slice * 4), k = b0 * 32 + (i - m * p.slice * 4) * 8;
+#pragma unroll
+      for (int u = 0; u < 8; u++) x[s][u] = 0.f;
+      if (m < p.M) {  // (i past the end: m >= 16)
+        const float *row = p.a + (size_t)m * p.K;
+        if (quads && k + 8 <= p.K) {
+          const float4 x0 = *(const float4 *)(row + k), x1 = *(const float4 *)(row + k + 4);
+          x[s][0] = x0.x, x[s][1] = x0.y, x[s][2] = x0.z, x[s][3] = x0.w, x[s][4] = x1.x, x[s][5] = x1.y, x[s][6] = x1.z, x[s][7] = x1.w;
+        } else {
+#pragma unroll
+          for (int u = 0; u < 8; u++)
+            if (k + u < p.K) x[s][u] = row[k + u];
+        }
+      }
     }
-    __half2 h[4], l[4];
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+      const int i = i0 + s * kMmaThreads, m = i / (p.slice * 4), oct = i - m * p.slice * 4;
+      if (m >= 16) break;
+      __half2 h[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) h[u] = __floats2half2_rn(x[s][u], x[s][u + 4]);
+      *(uint4 *)(ap + (size_t)m * pitch + oct * 16) = *(const uint4 *)h;
+      if (HILO) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const float2 f = __half22float2(h[u]);
+          h[u] = __floats2half2_rn(x[s][u] - f.x, x[s][u + 4] - f.y);
+        }
+        *(uint4 *)(ap + (size_t)(16 + m) * pitch + oct * 16) = *(const uint4 *)h;
+      }
+    }
+  }
+  __syncthreads();
+  if (slices > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+
+  int pass = 0;
+  for (int g0 = gfirst; g0 < gend; g0 += G, pass++) {
+    if (g0 > gfirst) fetch(g0);
+    float sc[G];     // lane: block j4 of column g4
+    unsigned z4[G];  // column g4: zero-points of the quad's blocks, a nibble each
+#pragma unroll
+    for (int g = 0; g < G; g++) {
+      sc[g] = 0.f, z4[g] = 0u;
+      if (g0 + g < gend && qn > 0) {
+        const int n = (g0 + g) * 8 + g4;
+        if (j4 < qn) sc[g] = __ldg(p.scales + (size_t)n * p.nblk + qb + j4);
+        const uint8_t *z = p.zp + (size_t)n * p.zpb + (qb >> 1);  // qb is a multiple of 4
+        z4[g] = __ldg(z);
+        if (qn > 2) z4[g] |= (unsigned)__ldg(z + 1) << 8;
+      }
+    }
+    float acc[G][4];
+#pragma unroll
+    for (int g = 0; g < G; g++) {
+      transpose4(w[g], lane);
+#pragma unroll
+      for (int c = 0; c < 4; c++) acc[g][c] = 0.f;
+    }
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-      h[i] = __floats2half2_rn(x[i], x[i + 4]);
-      const float2 f = __half22float2(h[i]);
-      l[i] = __floats2half2_rn(x[i] - f.x, x[i + 4] - f.y);
-    }
-    unsigned char *dst = planes + (size_t)m * pitch + (w >> 2) * kMmaSeg + (w & 3) * 16;
-    *(uint4 *)dst = make_uint4(*(uint32_t *)&h[0], *(uint32_t *)&h[1], *(uint32_t *)&h[2], *(uint32_t *)&h[3]);
-    if (HILO) {
-      const uint4 lv = make_uint4(*(uint32_t *)&l[0], *(uint32_t *)&l[1], *(uint32_t *)&l[2], *(uint32_t *)&l[3]);
-      *(uint4 *)(dst + (size_t)16 * pitch) = lv;
-      any_residue |= (lv.x | lv.y | lv.z | lv.w) & 0x7FFF7FFFu;
-    }
-  }
-  // rows that are exactly representable in f16 (activations that arrive as f16 values) have an all-zero residue
-  // plane: its products are skipped for the whole launch
-  const bool use_residue = HILO && __syncthreads_or(any_residue != 0u);
-  if (!HILO) __syncthreads();
-
-  // (the walk over the column groups exists twice, with and without the residue products: as a test inside the loop
-  // the compiler predicates the instructions instead of branching around them, and they keep their issue slots)
-  auto walk = [&](auto res_tag) {
-  constexpr bool kRes = decltype(res_tag)::value;
-  for (int cg0 = blockIdx.x; cg0 < groups; cg0 += kMmaBatch * gridDim.x) {
-    float c[kMmaBatch][4];
+      if (i >= qn) break;  // warp-uniform
+      const unsigned char *src = ap + (size_t)g4 * pitch + (warp * 4 + i) * 64 + j4 * 16;
+      const uint4 h0 = *(const uint4 *)src, h1 = *(const uint4 *)(src + (size_t)8 * pitch);
+      uint4 l0, l1;
+      if (HILO) l0 = *(const uint4 *)(src + (size_t)16 * pitch), l1 = *(const uint4 *)(src + (size_t)24 * pitch);
 #pragma unroll
-    for (int gi = 0; gi < kMmaBatch; gi++) {
-      c[gi][0] = c[gi][1] = c[gi][2] = c[gi][3] = 0.f;
-      const int cg = cg0 + gi * gridDim.x;
-      if (cg >= groups) continue;  // (block-uniform)
-      const int n = cg * 8 + g;
-      for (int q = warp; q < quads; q += kMmaWarps) {
-        const int b = 4 * q + t;
-        const bool in = b < nblk;
-        uint4 wv;
-        float sc;
-        unsigned zb;
-        if (q == warp) {
-          wv = pw[gi], sc = psc[gi], zb = pzb[gi];
-        } else {
-          wv = in ? __ldcs(bq4 + (size_t)n * nblk + b) : make_uint4(0u, 0u, 0u, 0u);
-          sc = in ? __ldg(scales + (size_t)n * nblk + b) : 0.f;
-          zb = in ? (unsigned)__ldg(zp + (size_t)n * zpb + (b >> 1)) : 0u;
+      for (int g = 0; g < G; g++) {
+        if (g0 + g >= gend) break;
+        const unsigned x = i == 0 ? w[g].x : (i == 1 ? w[g].y : (i == 2 ? w[g].z : w[g].w));
+        const unsigned zz = 0x6400u + ((z4[g] >> (4 * i)) & 15u), z2 = zz | (zz << 16);  // 1024 + zp, twice
+        uint32_t b[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const unsigned q = ((x >> (4 * u)) & 0x000F000Fu) | 0x64006400u;
+          const __half2 d = __hsub2(*(const __half2 *)&q, *(const __half2 *)&z2);
+          b[u] = *(const uint32_t *)&d;
         }
-        const int z = (b & 1) ? (int)(zb >> 4) : (int)(zb & 15u);
-        const __half2 s2 = __float2half2_rn(sc);
-        const uint32_t s2_u = *(const uint32_t *)&s2, zsub_u = 0x64006400u + (uint32_t)z * 0x00010001u;  // 1024 + zp, both halves
-        const unsigned char *arow = planes + (size_t)g * pitch + (size_t)(in ? b : 0) * kMmaSeg;
-        const uint32_t wd[4] = {wv.x, wv.y, wv.z, wv.w};
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
+        mma16816_f16(c, h0.x, h1.x, h0.y, h1.y, b[0], b[1]);
+        mma16816_f16(c, h0.z, h1.z, h0.w, h1.w, b[2], b[3]);
+        if (HILO) {
+          mma16816_f16(c, l0.x, l1.x, l0.y, l1.y, b[0], b[1]);
+          mma16816_f16(c, l0.z, l1.z, l0.w, l1.w, b[2], b[3]);
+        }
+        const float s0 = __shfl_sync(0xffffffffu, sc[g], j4 * 8 + i), s1 = __shfl_sync(0xffffffffu, sc[g], j4 * 8 + 4 + i);
+        acc[g][0] = fmaf(s0, c[0], acc[g][0]), acc[g][1] = fmaf(s1, c[1], acc[g][1]);
+        acc[g][2] = fmaf(s0, c[2], acc[g][2]), acc[g][3] = fmaf(s1, c[3], acc[g][3]);
+      }
+    }
+    if (pass > 0) __syncthreads();  // the sums of the pass before have been read
 #pragma unroll
-        for (int wi = 0; wi < 4; wi++) {
-          // word wi = k 8wi..8wi+7 of the block: pairs (k0,k4) (k1,k5) (k2,k6) (k3,k7)
-          uint32_t bp[4];
+    for (int g = 0; g < G; g++) red[(warp * G + g) * 32 + lane] = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+    __syncthreads();
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (tid < G * 32) {
+      t = red[tid];
 #pragma unroll
-          for (int pi = 0; pi < 4; pi++) {
-            const uint32_t hx = ((wd[wi] >> (4 * pi)) & 0x000F000Fu) | 0x64006400u;  // 1024 + q in both halves
-            uint32_t d;
-            asm("{\n\t.reg .b32 t;\n\tsub.f16x2 t, %1, %2;\n\tmul.f16x2 %0, t, %3;\n\t}" : "=r"(d) : "r"(hx), "r"(zsub_u), "r"(s2_u));
-            bp[pi] = d;
-          }
-          const uint4 a_lo8 = *(const uint4 *)(arow + wi * 16);                        // row g:     (k0,k4)(k1,k5)(k2,k6)(k3,k7)
-          const uint4 a_hi8 = *(const uint4 *)(arow + (size_t)8 * pitch + wi * 16);    // row g + 8
-          mma16816_f16(c[gi], a_lo8.x, a_hi8.x, a_lo8.y, a_hi8.y, bp[0], bp[1]);
-          mma16816_f16(c[gi], a_lo8.z, a_hi8.z, a_lo8.w, a_hi8.w, bp[2], bp[3]);
-          if (kRes) {
-            const uint4 r_lo8 = *(const uint4 *)(arow + (size_t)16 * pitch + wi * 16);
-            const uint4 r_hi8 = *(const uint4 *)(arow + (size_t)24 * pitch + wi * 16);
-            mma16816_f16(c[gi], r_lo8.x, r_hi8.x, r_lo8.y, r_hi8.y, bp[0], bp[1]);
-            mma16816_f16(c[gi], r_lo8.z, r_hi8.z, r_lo8.w, r_hi8.w, bp[2], bp[3]);
-          }
+      for (int v = 1; v < kMmaWarps; v++) {
+        const float4 o = red[v * G * 32 + tid];
+        t.x += o.x, t.y += o.y, t.z += o.z, t.w += o.w;
+      }
+    }
+    if (slices > 1) {
+      // two buffers: a rank stores pass n + 2 only after the barrier of pass n + 1, which rank 0 reaches when it has read n
+      float4 *buf = cred + (size_t)(pass & 1) * slices * G * 32;
+      if (tid < G * 32) {
+        uint32_t remote;
+        const uint32_t local = (uint32_t)__cvta_generic_to_shared(buf + rank * G * 32 + tid);
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(0));
+        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(remote), "f"(t.x), "f"(t.y), "f"(t.z), "f"(t.w) : "memory");
+      }
+      asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+      if (rank == 0 && tid < G * 32) {
+        t = buf[tid];
+        for (int v = 1; v < slices; v++) {
+          const float4 o = buf[v * G * 32 + tid];
+          t.x += o.x, t.y += o.y, t.z += o.z, t.w += o.w;
         }
       }
-      // request this warp's first quad of the same slot's group in the next batch
-      {
-        const int cgn = cg + D * gridDim.x, b = 4 * warp + t;
-        const bool ok = cgn < groups && b < nblk;
-        const size_t nn = (size_t)(cgn * 8 + g);
-        pw[gi] = ok ? __ldcs(bq4 + nn * nblk + b) : make_uint4(0u, 0u, 0u, 0u);
-        psc[gi] = ok ? __ldg(scales + nn * nblk + b) : 0.f;
-        pzb[gi] = ok ? (unsigned)__ldg(zp + nn * zpb + (b >> 1)) : 0u;
-      }
     }
-    // the 16 warps' partial tiles of the batch meet in shared memory; every thread adds one (group, element) in warp
-    // order and stores it
-#pragma unroll
-    for (int gi = 0; gi < kMmaBatch; gi++)
-      *(float4 *)(red + (((size_t)gi * kMmaWarps + warp) * 32 + lane) * 4) = make_float4(c[gi][0], c[gi][1], c[gi][2], c[gi][3]);
-    __syncthreads();
-    {
-      const int gi = tid >> 7, ln = (tid >> 2) & 31, ci = tid & 3;  // 512 threads = 4 groups x 32 lanes x 4 elements
-      const int cg = cg0 + gi * gridDim.x;
-      if (cg < groups) {
-        float sum = 0.f;
-#pragma unroll
-        for (int w = 0; w < kMmaWarps; w++) sum += red[(((size_t)gi * kMmaWarps + w) * 32 + ln) * 4 + ci];
-        const int gg = ln >> 2, tt = ln & 3;
-        const int m = gg + ((ci & 2) ? 8 : 0), col = cg * 8 + 2 * tt + (ci & 1);
-        if (m < M) y[(size_t)m * N + col] = sum;
-      }
+    const int g = g0 + (tid >> 5);
+    if (rank == 0 && tid < G * 32 && g < gend) {
+      const int n = g * 8 + j4 * 2;
+      if (g4 < p.M) *(float2 *)(p.y + (size_t)g4 * p.N + n) = make_float2(t.x, t.y);
+      if (g4 + 8 < p.M) *(float2 *)(p.y + (size_t)(g4 + 8) * p.N + n) = make_float2(t.z, t.w);
     }
-    __syncthreads();
   }
-  };
-  if (use_residue) walk(std::true_type{}); else walk(std::false_type{});
 }
+
+size_t mma_smem(bool hilo, int G, int slice, int slices) {
+  return (size_t)(hilo ? 2 : 1) * 16 * mma_row_pitch(slice) + (size_t)G * 32 * 16 * (kMmaWarps + (slices > 1 ? 2 * slices : 0));
+}
+// K slices (a power of two: clusters of 3 place badly) and blocks per slice, a multiple of 4
+void mma_slices(int nblk, int &slices, int &slice) {
+  for (slices = 1; slices * kMmaSliceBlk < nblk; slices *= 2) {}
+  slice = ceil_div(ceil_div(nblk, slices), 4) * 4;
+}
+
+template <bool HILO, int G>
+cudaError_t launch_mma(fa_ctx *ctx, cudaLaunchConfig_t &cfg, const MmaParams &p) {
+  cfg.dynamicSmemBytes = mma_smem(HILO, G, p.slice, (int)cfg.gridDim.y);
+  const cudaError_t e = cudaFuncSetAttribute(k_nbits_mma<HILO, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+  return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, k_nbits_mma<HILO, G>, p);
+}
+
+}  // namespace
 
 // int4 products with up to 16 activation rows on k_nbits_mma.  hilo: the rows enter as value + residue f16 planes.
-bool fa_nbits_mma_ok(int M, int N, int K, int block_size, bool hilo) {
-  if (!(M >= 1 && M <= 16 && block_size == 32 && K >= 32 && N >= 8 && (N & 7) == 0)) return false;
-  const int nblk = (K + 31) / 32;
-  const size_t smem = (size_t)(hilo ? 2 : 1) * 16 * mma_row_pitch(nblk) + (size_t)kMmaBatch * kMmaWarps * 32 * 16;
-  return smem <= 224 * 1024;
+bool fa_nbits_mma_ok(int M, int N, int K, int block_size) {
+  return M >= 1 && M <= 16 && block_size == 32 && K >= 32 && K <= kMmaMaxSlices * kMmaSliceBlk * 32 && N >= 8 && (N & 7) == 0;
 }
-
-// Measured at K = 2048 (recorded replays): 3.8 us + 1.15 us (1.37 with the residue plane) per column group a thread block
-// walks, against 10.5-13 us for the tensor-core GEMM on the dequantised copy whatever N is - this kernel is the faster
-// one while a block has at most five groups.
-bool fa_nbits_mma_worth(fa_ctx *ctx, int N) { return (long long)(N / 8) <= 5ll * ctx->sm_count; }
 
 int fa_nbits_mma(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y, int M, int N,
                  int K, int nblk, int zpb, bool hilo) {
-  const size_t smem = (size_t)(hilo ? 2 : 1) * 16 * mma_row_pitch(nblk) + (size_t)kMmaBatch * kMmaWarps * 32 * 16;
-  const int groups = N / 8;
-  const dim3 grid((unsigned)(groups < ctx->sm_count ? groups : ctx->sm_count)), block(kMmaWarps * 32);
+  MmaParams p{a, bq, scales, zp, y, M, N, K, nblk, zpb, 0, 0};
+  int slices;
+  mma_slices(nblk, slices, p.slice);
+  // column groups per thread block: as many as leave one wave of blocks (clusters of K slices do not tile every GPC, so
+  // an eighth of the SMs is left out of the count there); walked 8, 4 or 2 at a time
+  const int groups = N / 8, room = slices == 1 ? ctx->sm_count : ctx->sm_count * 7 / 8 / slices;
+  p.gper = ceil_div(groups, room < 1 ? 1 : room);
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  cfg.gridDim = dim3(ceil_div(groups, p.gper), slices);
+  cfg.blockDim = dim3(kMmaThreads);
+  cfg.stream = ctx->stream;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see fa_launch_dep
+  attr[0].val.programmaticStreamSerializationAllowed = ctx->pdl ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = slices;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = slices > 1 ? 2 : 1;
   cudaError_t e;
   {
     LaunchScope ls(ctx, "nbits_mma");
-    if (hilo) {
-      FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_nbits_mma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      e = fa_launch_dep(ctx, k_nbits_mma<true>, grid, block, smem, a, bq, scales, zp, y, M, N, K, nblk, zpb);
-    } else {
-      FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_nbits_mma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      e = fa_launch_dep(ctx, k_nbits_mma<false>, grid, block, smem, a, bq, scales, zp, y, M, N, K, nblk, zpb);
-    }
+    if (p.gper <= 2) e = hilo ? launch_mma<true, 2>(ctx, cfg, p) : launch_mma<false, 2>(ctx, cfg, p);
+    else if (p.gper <= 4) e = hilo ? launch_mma<true, 4>(ctx, cfg, p) : launch_mma<false, 4>(ctx, cfg, p);
+    else e = hilo ? launch_mma<true, 8>(ctx, cfg, p) : launch_mma<false, 8>(ctx, cfg, p);
   }
   if (e != cudaSuccess) return fa_fail(ctx, FA_ERR_CUDA, "launch nbits_mma: %s", cudaGetErrorString(e));
-  FA_LAUNCH_CHECK(ctx, "nbits_mma");
   return FA_OK;
 }
 

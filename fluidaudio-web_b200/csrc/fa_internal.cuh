@@ -350,8 +350,7 @@ int fa_tc_gemm_i8(fa_ctx *ctx, const int8_t *a_packed, int limbs, const int8_t *
 // CUDA-core products for M <= kGemvMaxRows activation rows, on the weights as uploaded (fa_gemv.cu)
 constexpr int kGemvMaxRows = 4;
 bool fa_gemv_nbits_ok(int M, int N, int K, int block_size);
-bool fa_nbits_mma_ok(int M, int N, int K, int block_size, bool hilo);
-bool fa_nbits_mma_worth(fa_ctx *ctx, int N);
+bool fa_nbits_mma_ok(int M, int N, int K, int block_size);
 int fa_nbits_mma(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y, int M, int N,
                  int K, int nblk, int zpb, bool hilo);
 int fa_gemv_nbits(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y, int M,
