@@ -1691,35 +1691,60 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
   p.o16_col_lo = ep.o16_col_lo;
   int num_tiles = p.tiles_n * p.tiles_m * p.batches;
   // Products whose tiles fit one wave of the SMs (decode sizes, thin encoder shapes) are bound by what ONE thread
-  // block can pull from L2 / HBM (measured ~120 GB/s per SM) on top of a fixed launch-and-ramp cost, so the aim is
-  // as many busy SMs as possible without a second wave: first shorter row tiles (no reduction needed), then K split
-  // over a cluster of 2, 4 or 8 CTAs whose partial tiles meet in shared memory.  Measured on 24 thin shapes: a
-  // second wave costs more than any split saves; clusters of 3, 5, 6, 7 place badly on the GPCs (2x slower);
-  // fewer than 4 K chunks per CTA no longer pays for the reduction.
+  // block can pull from L2 / HBM on top of a fixed launch-and-ramp cost, so the tile height and a split of K over a
+  // cluster of 2, 4 or 8 CTAs (whose partial tiles meet in shared memory) are chosen together by their estimated time.
+  // The estimate, in ns beside the fixed cost, fitted to sweeps of both over 30 shapes of the f16, int8 and tf32 forms:
+  //   chunk     1 per 128-byte operand row a CTA loads per K chunk, at least 160 (one chunk's latency chain)
+  //   height    6 per row of the tile (its epilogue)
+  //   split     3700 for the hand-over of a split tile (f16 and tf32: 1500 + 35 per row) up to 64 rows, 5500 above, 2500
+  //             more for halves of tiles above 96 rows, 600 more for eighths
+  //   spread    14 per CTA: of two equal choices the one with fewer, which leaves the next launch room to start
+  // One wave only (a second one costs more than any split saves): clusters do not tile every GPC, so quarters may use
+  // 7/8 of the SMs and eighths 2/3; clusters of 3, 5, 6, 7 place badly (2x slower).  Against the rule before it (shortest
+  // tile of at least 64 rows, then the widest split), recorded products, us: f32 300 x 4096 x 1024 35.6 -> 28.8, 800 x 4096
+  // x 1024 62.2 -> 51.6; int8 100 x 1024 x 4096 11.7 -> 7.9, 300 x 2048 x 1024 14.0 -> 11.0; f16 300 x 1024 x 1024 8.4 ->
+  // 5.8, 200 x 1024 x 1024 7.2 -> 5.7.
   // (the split-K finish stores rows at pitch N: a caller-chosen pitch keeps the one-CTA-per-tile form)
   p.splitk = 1;
   p.kb_per_split = p.num_kb;
   const bool split_ok = !raw_i32 && !ep.out16 && ep.n_peers == 0 && (ep.ldc == 0 || ep.ldc == N) && p.batches == 1;
   if (split_ok && num_tiles <= ctx->sm_count) {
-    const int mt_hi = p.MT;
+    const int mt_hi = mt < mt_max ? mt : mt_max, w_rows = (KIND == 4 ? 2 : 1) * 128;
     int best_mt = p.MT, best_s = 1;
-    // shortest row tile of at least 64 rows (or the whole of a shorter M) whose tiles still fit one wave
-    for (int cand = mt_hi; cand >= (mt_hi < 64 ? mt_hi : 64); cand -= 16) {
-      if ((long long)p.tiles_n * ceil_div(M, cand) > ctx->sm_count) break;
-      best_mt = cand;
-    }
-    while (best_mt > 16 && ceil_div(M, best_mt - 16) == ceil_div(M, best_mt)) best_mt -= 16;  // same tiling, less padding
-    // K split (tiles of at most 64 rows: the reduction of taller tiles costs more than the split saves): the widest
-    // power-of-two cluster that keeps one wave and at least 4 K chunks per CTA
-    if (best_mt <= 64) {
-      const long long tiles = (long long)p.tiles_n * ceil_div(M, best_mt);
-      for (int sp = 2; sp <= 8; sp *= 2) {
-        if (tiles * sp > ctx->sm_count || p.num_kb / sp < 4) break;
+    // f32-grade products (residue planes): a sum that stays in one accumulator longer loses more to its truncation, so K is
+    // split at least as wide as by the plain rule: the shortest tile of at least 64 rows that keeps one wave, then the
+    // widest split that does (with the K = 1280 products of a decoder token unsplit, its logits were 5.1e-5 off the CPU
+    // reference, over the 5e-5 that they keep to split four ways)
+    if (KIND == 4 || (KIND == 0 && limbs == 2)) {
+      for (int cand = p.MT; cand >= (p.MT < 64 ? p.MT : 64); cand -= 16) {
+        if ((long long)p.tiles_n * ceil_div(M, cand) > ctx->sm_count) break;
+        best_mt = cand;
+      }
+      while (best_mt > 16 && ceil_div(M, best_mt - 16) == ceil_div(M, best_mt)) best_mt -= 16;  // same tiling, less padding
+      for (int sp = 2; sp <= 8 && best_mt <= 64; sp *= 2) {
+        if ((long long)p.tiles_n * ceil_div(M, best_mt) * sp > ctx->sm_count || p.num_kb / sp < 4) break;
         best_s = sp;
       }
     }
+    const int min_s = best_s;
+    long long best = -1;
+    for (int cand = mt_hi; cand >= (mt_hi < 32 ? mt_hi : 32); cand -= 16) {
+      const int tiles_m = ceil_div(M, cand);
+      if (cand > 32 && ceil_div(M, cand - 16) == tiles_m) continue;  // same tiling with less padding further down
+      for (int sp = min_s; sp <= 8; sp *= 2) {
+        const long long ctas = (long long)p.tiles_n * tiles_m * sp;
+        const int room = sp == 8 ? ctx->sm_count * 2 / 3 : (sp == 4 ? ctx->sm_count * 7 / 8 : ctx->sm_count);
+        if (ctas > room || (sp > 1 && (cand > kSplitMaxMT || p.num_kb / sp < 4))) continue;
+        const long long rows = w_rows + cand * limbs, chunks = ceil_div(p.num_kb, sp);
+        if ((sp - 1) * chunks >= p.num_kb) continue;  // the last CTA of the cluster would have nothing
+        long long cost = chunks * (rows > 160 ? rows : 160) + 6 * cand + 14 * ctas;
+        if (sp > 1)
+          cost += (cand > 64 ? 5500 : (KIND == 1 ? 3700 : 1500 + 35 * cand)) + (sp == 2 && cand > 96 ? 2500 : 0) + (sp == 8 ? 600 : 0);
+        if (best < 0 || cost < best) best = cost, best_mt = cand, best_s = sp;
+      }
+    }
     if (ctx->tc_tile_rows > 0 || ctx->tc_split_k > 0) {  // tuning overrides (options "tc_tile_rows", "tc_split_k")
-      if (ctx->tc_tile_rows > 0) best_mt = ((ctx->tc_tile_rows + 15) / 16) * 16 < mt_hi ? ((ctx->tc_tile_rows + 15) / 16) * 16 : mt_hi;
+      if (ctx->tc_tile_rows > 0) best_mt = ((ctx->tc_tile_rows + 15) / 16) * 16 < mt_max ? ((ctx->tc_tile_rows + 15) / 16) * 16 : mt_max;
       best_s = ctx->tc_split_k > 0 ? ctx->tc_split_k : 1;
       if (best_mt > kSplitMaxMT) best_s = 1;
       while (best_s > 1 && p.num_kb / best_s < 2) best_s--;
