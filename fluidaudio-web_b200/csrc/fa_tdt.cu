@@ -476,10 +476,12 @@ struct fa_tdt {
   fa_tensor *gate_tab = nullptr, *wr[2] = {nullptr, nullptr}, *bsum1 = nullptr, *pred_w = nullptr, *pred_b = nullptr;
   fa_tensor *out_b = nullptr, *out_scale = nullptr, *ones = nullptr, *out_w = nullptr;
   fa_bytes *out_q = nullptr;
-  // the decode loop's read-back: page-locked copy of the windows' positions (grown to the largest W seen) and its event
+  // the decode loop's read-back: page-locked copy of the windows' positions (grown to the largest W seen), made on a stream
+  // of its own (a copy in the rounds' stream held the next round up for 12 us), and the events around it
   int *t_host = nullptr;
   int t_cap = 0;
-  cudaEvent_t t_read = nullptr;
+  cudaStream_t side = nullptr;
+  cudaEvent_t t_at = nullptr, t_read = nullptr;
 };
 
 static void tdt_release(fa_ctx *ctx, fa_tdt *d) {
@@ -488,6 +490,8 @@ static void tdt_release(fa_ctx *ctx, fa_tdt *d) {
     if (t) fa_free_tensor(ctx, t);
   if (d->out_q) fa_free_bytes(ctx, d->out_q);
   if (d->t_host) cudaFreeHost(d->t_host);
+  if (d->side) cudaStreamDestroy(d->side);
+  if (d->t_at) cudaEventDestroy(d->t_at);
   if (d->t_read) cudaEventDestroy(d->t_read);
   delete d;
 }
@@ -696,6 +700,8 @@ extern "C" int fa_tdt_decode_proj(fa_ctx *ctx, fa_tdt *d, const fa_tensor *proj,
     if (d->t_host) cudaFreeHost(d->t_host);
     d->t_host = nullptr, d->t_cap = 0;
     cudaError_t e = cudaHostAlloc(&d->t_host, (size_t)W * 4, cudaHostAllocDefault);
+    if (e == cudaSuccess && !d->side) e = cudaStreamCreateWithFlags(&d->side, cudaStreamNonBlocking);
+    if (e == cudaSuccess && !d->t_at) e = cudaEventCreateWithFlags(&d->t_at, cudaEventDisableTiming);
     if (e == cudaSuccess && !d->t_read) e = cudaEventCreateWithFlags(&d->t_read, cudaEventDisableTiming);
     if (e != cudaSuccess) rc = fa_fail(ctx, FA_ERR_CUDA, "tdtDecodeProj: %s", cudaGetErrorString(e));
     else d->t_cap = W;
@@ -724,8 +730,12 @@ extern "C" int fa_tdt_decode_proj(fa_ctx *ctx, fa_tdt *d, const fa_tensor *proj,
     const int n = sure > min_rounds ? sure : min_rounds, first = (n + 1) / 2;
     run(first);
     if (rc == FA_OK) {
-      cudaError_t e = cudaMemcpyAsync(d->t_host, t, (size_t)W * 4, cudaMemcpyDeviceToHost, ctx->stream);
-      if (e == cudaSuccess) e = cudaEventRecord(d->t_read, ctx->stream);
+      // (rounds enqueued below may move a position before it is copied: positions only grow and every such round is
+      // counted in `second`, so the bound made from them stays one)
+      cudaError_t e = cudaEventRecord(d->t_at, ctx->stream);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(d->side, d->t_at, 0);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(d->t_host, t, (size_t)W * 4, cudaMemcpyDeviceToHost, d->side);
+      if (e == cudaSuccess) e = cudaEventRecord(d->t_read, d->side);
       if (e != cudaSuccess) rc = fa_fail(ctx, FA_ERR_CUDA, "tdtDecodeProj: %s", cudaGetErrorString(e));
     }
     const int second = sure > first ? sure - first : 0;  // certain to be needed as well: they run under the read-back
@@ -753,6 +763,7 @@ extern "C" int fa_tdt_decode_proj(fa_ctx *ctx, fa_tdt *d, const fa_tensor *proj,
     if (rc == FA_OK) rc = fa_sync(ctx);
   }
   const std::string msg = ctx->err;
+  if (rc != FA_OK && d->side) cudaStreamSynchronize(d->side);  // no copy of the positions outlives its source
   if (s.ints) fa_block_release(ctx, s.ints);
   if (s.planes) fa_block_release(ctx, s.planes);
   if (s.rowscale) fa_block_release(ctx, s.rowscale);
