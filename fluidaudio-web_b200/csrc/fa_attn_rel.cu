@@ -13,6 +13,13 @@
 // packed operand of the separate-op form is - multiply V from the same shared memory.  Operands f16,
 // accumulation f32 (mma.sync m16n8k16: the problem is 0.04 GFLOP per CTA and latency bound, a tcgen05 pipeline
 // with TMEM accumulators cannot shift rows by a per-row amount without the same round trip through shared memory).
+//
+// What bounds it is shared-memory reads: every warp reads all keys, its positional window and all values as B fragments
+// (344 ldmatrix.x4 a warp at T = 192).  So key tiles past T are left out (KT is the
+// next multiple of three tiles of 16 keys), and when the (window, head) pairs do not fill
+// the GPU their query tiles are dealt to two or three CTAs, each with its own copy of the operands: the reads of a CTA
+// shrink with its share while the fills stay.  Measured per
+// launch: 6 windows of 134 frames 20.0 -> 11.9 us, one window of 47 frames 13.9 -> 7.5 us, 32 windows of 188 as before (43.8 us).
 #include "fa_internal.cuh"
 
 namespace {
@@ -134,7 +141,8 @@ __device__ __forceinline__ void q_tile_packed(__half *dst, const __half *__restr
 
 // PACKED: q, k, v are column ranges [0,S), [S,2S), [2S,3S) of ONE projection stored as its packed f16 operand
 // (q points at it, k and v are unused, ldq is ignored); otherwise f32 rows ldq floats apart.
-template <bool PACKED>
+// KT: 16-key tiles computed, T <= 16 * KT.
+template <bool PACKED, int KT>
 __global__ void __launch_bounds__(kAWarps * 32, 1)
     k_attn_rel(const float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v,
                const __half *__restrict__ pos16, const float *__restrict__ pbu, const float *__restrict__ pbv,
@@ -148,7 +156,7 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int NP = 2 * T - 1;
 
-  const int i0 = warp * 16, r0 = i0 + g, r1 = r0 + 8;
+  const int i0 = (warp * gridDim.y + blockIdx.y) * 16, r0 = i0 + g, r1 = r0 + 8;  // gridDim.y CTAs share the query tiles
   const bool ok0 = r0 < T, ok1 = r1 < T;
   const bool active = i0 < T;  // warps whose 16 rows all lie past T only help with the fills and the barriers
   const float *qrows = q + ((size_t)w * T + (active ? i0 : 0)) * ldq + h * kAHD;  // q, k, v rows are ldq floats apart
@@ -160,7 +168,7 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
   const __half *qkv16 = (const __half *)q;
   const size_t mw = (size_t)w * T;
   if (PACKED) {  // the keys first: their copy group is the one the content scores wait for
-    fill_rows_packed(Ks, qkv16, S + h * kAHD, mw, Mrows, T, kAT);
+    fill_rows_packed(Ks, qkv16, S + h * kAHD, mw, Mrows, T, KT * 16);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   // the head's positional rows (already f16) go to shared memory as asynchronous 16-byte copies that nobody waits
@@ -179,7 +187,7 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
     if (active) q_tile_packed(qu_tile, qkv16, h * kAHD, mw + i0, Mrows, pbu + h * kAHD, qvalid, lane);
     asm volatile("cp.async.wait_group 1;" ::: "memory");  // the keys have landed, the positional rows may still fly
   } else {
-    fill_rows_f16(Ks, k + (size_t)w * T * ldq + h * kAHD, ldq, T, kAT);
+    fill_rows_f16(Ks, k + (size_t)w * T * ldq + h * kAHD, ldq, T, KT * 16);
     if (active) q_tile_f16(qu_tile, qrows, pbu + h * kAHD, ldq, qvalid, lane);
   }
   __syncthreads();
@@ -189,9 +197,9 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
   const int lm_row = (lane & 7) + ((lane >> 4) << 3), lm_col = ((lane >> 3) & 1) << 3;
   const int la_off = ((lane & 7) + (((lane >> 3) & 1) << 3)) * kALd + ((lane >> 4) << 3);
 
-  float s[24][4];
+  float s[2 * KT][4];
 #pragma unroll
-  for (int n = 0; n < 24; n++) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+  for (int n = 0; n < 2 * KT; n++) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
 
   // content scores: S = (q + u) K^T, 16 x 192 per warp
   if (active) {
@@ -201,7 +209,7 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
       ldsm4(a, qu_tile + la_off + ks * 16);
       const __half *kb = Ks + (size_t)lm_row * kALd + ks * 16 + lm_col;
 #pragma unroll
-      for (int np = 0; np < 12; np++) {
+      for (int np = 0; np < KT; np++) {
         uint32_t b[4];
         ldsm4(b, kb + (size_t)np * 16 * kALd);
         mma16816(s[2 * np], a, b[0], b[1]);
@@ -224,7 +232,9 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
   // p_lo = T - 16 - i0 + j0 cover bd[i][T-1-i+j] for the warp's 16 rows and the block's 64 keys
   if (active) {
 #pragma unroll  // (unrolled so that s[] is indexed statically and stays in registers)
-    for (int jb = 0; jb < 3; jb++) {
+    for (int jb = 0; jb < (KT + 3) / 4; jb++) {
+      constexpr int kTiles[3] = {KT < 4 ? KT : 4, KT < 8 ? KT - 4 : 4, KT - 8};  // 16-key tiles of each 64-key block
+      const int nt = kTiles[jb];
       float c[10][4];
 #pragma unroll
       for (int n = 0; n < 10; n++) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
@@ -235,6 +245,7 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
         ldsm4(a, qv_tile + la_off + ks * 16);
 #pragma unroll
         for (int np = 0; np < 5; np++) {
+          if (np > nt) continue;
           uint32_t b[4];
           ldsm4(b, pb + (size_t)np * 16 * kALd + ks * 16);
           mma16816(c[2 * np], a, b[0], b[1]);
@@ -243,6 +254,7 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
       }
 #pragma unroll
       for (int n = 0; n < 10; n++) {
+        if (n >= 2 * nt + 2) continue;
         *(float2 *)(st + g * kAStLd + 8 * n + 2 * t) = make_float2(c[n][0], c[n][1]);
         *(float2 *)(st + (g + 8) * kAStLd + 8 * n + 2 * t) = make_float2(c[n][2], c[n][3]);
       }
@@ -250,7 +262,8 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
       const float *s0 = st + g * kAStLd + 15 - g + 2 * t, *s1 = st + (g + 8) * kAStLd + 7 - g + 2 * t;
 #pragma unroll
       for (int n = 0; n < 8; n++) {
-        float(&d)[4] = s[jb * 8 + n];
+        if (n >= 2 * nt) continue;
+        float(&d)[4] = s[jb * 8 + n < 2 * KT ? jb * 8 + n : 0];
         d[0] += s0[8 * n];
         d[1] += s0[8 * n + 1];
         d[2] += s1[8 * n];
@@ -261,11 +274,11 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
   }
 
   // softmax over the keys (columns j >= T masked), rows r0 and r1 of this thread's quad
-  uint32_t pf[12][4];
+  uint32_t pf[KT][4];
   if (active) {
     float m0 = -INFINITY, m1 = -INFINITY;
 #pragma unroll
-    for (int n = 0; n < 24; n++) {
+    for (int n = 0; n < 2 * KT; n++) {
       const int j = 8 * n + 2 * t;
       if (j >= T) s[n][0] = s[n][2] = -INFINITY;
       if (j + 1 >= T) s[n][1] = s[n][3] = -INFINITY;
@@ -278,7 +291,7 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
     m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, 2));
     float z0 = 0.f, z1 = 0.f;
 #pragma unroll
-    for (int n = 0; n < 24; n++) {
+    for (int n = 0; n < 2 * KT; n++) {
       s[n][0] = __expf(s[n][0] - m0);
       s[n][1] = __expf(s[n][1] - m0);
       s[n][2] = __expf(s[n][2] - m1);
@@ -292,7 +305,7 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
     z1 += __shfl_xor_sync(0xffffffffu, z1, 2);
     const float inv0 = 1.0f / z0, inv1 = 1.0f / z1;
 #pragma unroll
-    for (int kk = 0; kk < 12; kk++) {
+    for (int kk = 0; kk < KT; kk++) {
       pf[kk][0] = pack_h2(s[2 * kk][0] * inv0, s[2 * kk][1] * inv0);
       pf[kk][1] = pack_h2(s[2 * kk][2] * inv1, s[2 * kk][3] * inv1);
       pf[kk][2] = pack_h2(s[2 * kk + 1][0] * inv0, s[2 * kk + 1][1] * inv0);
@@ -301,11 +314,11 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
   }
   __syncthreads();  // every warp is done with its q + v tile
   if (PACKED) {
-    fill_rows_packed(Ks, qkv16, 2 * S + h * kAHD, mw, Mrows, T, kAT);
+    fill_rows_packed(Ks, qkv16, 2 * S + h * kAHD, mw, Mrows, T, KT * 16);
     asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
-    fill_rows_f16(Ks, v + (size_t)w * T * ldq + h * kAHD, ldq, T, kAT);
+    fill_rows_f16(Ks, v + (size_t)w * T * ldq + h * kAHD, ldq, T, KT * 16);
   }
   __syncthreads();  // V is in place
   if (!active) return;
@@ -318,7 +331,7 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
     // transposed loads: matrices = (key half 0|1) x (n tile 0|1)
     const __half *vb = Ks + (size_t)((lane & 7) + (((lane >> 3) & 1) << 3)) * kALd + ((lane >> 4) << 3);
 #pragma unroll
-    for (int kk = 0; kk < 12; kk++) {
+    for (int kk = 0; kk < KT; kk++) {
 #pragma unroll
       for (int np = 0; np < 8; np++) {
         uint32_t b[4];
@@ -342,6 +355,11 @@ __global__ void __launch_bounds__(kAWarps * 32, 1)
       if (ok1) *(__half2 *)(d + m1 * 64) = __floats2half2_rn(o[n][2], o[n][3]);
     }
   }
+}
+
+template <bool PACKED>
+auto attn_rel_kernel(int kt) {
+  return kt <= 3 ? k_attn_rel<PACKED, 3> : (kt <= 6 ? k_attn_rel<PACKED, 6> : (kt <= 9 ? k_attn_rel<PACKED, 9> : k_attn_rel<PACKED, 12>));
 }
 
 struct Block {  // pool block released at scope exit
@@ -384,8 +402,10 @@ int fa_attn_rel(fa_ctx *ctx, const float *q, const float *k, const float *v, con
              "attnFused: q/k/v rows must be 16-byte aligned");
   static bool attr_set[64] = {false};
   if (!attr_set[ctx->device & 63]) {
-    FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_attn_rel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kASmem));
-    FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_attn_rel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kASmem));
+    for (int kt = 3; kt <= 12; kt += 3) {
+      FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(attn_rel_kernel<false>(kt), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kASmem));
+      FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(attn_rel_kernel<true>(kt), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kASmem));
+    }
     attr_set[ctx->device & 63] = true;
   }
   const int NP = 2 * T - 1, S = H * HD;
@@ -422,11 +442,15 @@ int fa_attn_rel(fa_ctx *ctx, const float *q, const float *k, const float *v, con
   }
   {
     LaunchScope ls(ctx, "attn_rel");
+    const int pairs = W * H, tiles = ceil_div(T, 16);
+    int split = pairs * 3 <= ctx->sm_count ? 3 : (pairs * 2 <= ctx->sm_count ? 2 : 1);  // one wave: a CTA has an SM to itself
+    if (split > tiles) split = tiles;
+    const int kt = ceil_div(tiles, 3) * 3;
     if (ldq == 0)  // q is the packed f16 operand of the fused q|k|v projection
-      fa_launch_dep(ctx, k_attn_rel<true>, dim3((unsigned)(W * H)), dim3(kAWarps * 32), kASmem, q, k, v, pos16, pbu, pbv, out,
+      fa_launch_dep(ctx, attn_rel_kernel<true>(kt), dim3((unsigned)pairs, split), dim3(kAWarps * 32), kASmem, q, k, v, pos16, pbu, pbv, out,
                     out16, T, H, W * T, ldq);
     else
-      fa_launch_dep(ctx, k_attn_rel<false>, dim3((unsigned)(W * H)), dim3(kAWarps * 32), kASmem, q, k, v, pos16, pbu, pbv, out,
+      fa_launch_dep(ctx, attn_rel_kernel<false>(kt), dim3((unsigned)pairs, split), dim3(kAWarps * 32), kASmem, q, k, v, pos16, pbu, pbv, out,
                     out16, T, H, W * T, ldq);
   }
   FA_LAUNCH_CHECK(ctx, "attn_rel");
