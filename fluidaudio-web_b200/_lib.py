@@ -21,6 +21,25 @@ class ProfileEntry(C.Structure):
 
 
 # name -> argtypes (every function returns int except fa_last_error)
+class Linear(C.Structure):
+    _fields_ = [("w", P), ("scale", P), ("bias", P), ("N", I), ("K", I)]
+
+
+class DecoderLayer(C.Structure):
+    _fields_ = [(n, Linear) for n in ("sqkv", "so", "cq", "co", "f1", "f2")] + [
+        (n, P) for n in ("ln1_w", "ln1_b", "ln2_w", "ln2_b", "ln3_w", "ln3_b")]
+
+
+class FeedForward(C.Structure):
+    _fields_ = [(n, P) for n in ("ln_w", "ln_b", "w1", "w2", "b1", "b2")]
+
+
+class ConformerLayer(C.Structure):
+    _fields_ = [("ff1", FeedForward), ("ff2", FeedForward)] + [
+        (n, P) for n in ("lnatt_w", "lnatt_b", "lnconv_w", "lnconv_b", "lnout_w", "lnout_b", "q", "k", "v", "qkv", "pos", "out",
+                         "pw1", "pw2", "qb", "kb", "vb", "qkvb", "outb", "pw1b", "pw2b", "pbu", "pbv", "dw", "dwb")]
+
+
 SIGNATURES = {
     "fa_ctx_create": [I, PP],
     "fa_ctx_destroy": [P],
@@ -80,6 +99,8 @@ SIGNATURES = {
     "fa_linear_step": [P, P, P, P, C.c_float, P, P, P, I, I, P, I, P, PP],
     "fa_attn_step": [P, P, P, P, I, I, I, PP],
     "fa_attn_step_append": [P, P, P, P, I, I, I, PP],
+    "fa_decoder_step": [P, P, I, P, PP, PP, PP, PP, I, I, I, P, P, P, PP],
+    "fa_conformer_block": [P, P, P, P, P, I, I, I, I, I, P, P, PP, PP],
     "fa_attn_fused": [P, P, P, P, P, P, P, I, I, I, PP],
     "fa_attn_fused_qkv": [P, P, P, P, P, I, I, I, PP],
     "fa_rel_shift_b": [P, P, I, PP],

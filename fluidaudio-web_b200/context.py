@@ -422,6 +422,52 @@ class CudaContext:
         self._check(self._lib.fa_attn_step_append(self._h, qkv.h, cacheK.h, cacheV.h, n, NH, HD, C.byref(out)))
         return self._wrap(out) if out.value else None
 
+    # -- layer loops in native code (optional members) -----------------------------------------------
+    def _linear_of(self, w, bias) -> "_lib.Linear":
+        """(weights, bias) as the C struct; weights are a tensor [K, N] or (PackedBytes, scale, N, K)."""
+        if isinstance(w, tuple):
+            q, scale, N, K = w
+            return _lib.Linear(q.h, scale.h, self._h_of(bias), N, K)
+        return _lib.Linear(w.h, None, self._h_of(bias), w.cols, w.rows)
+
+    def decoderWeights(self, layers: Sequence[dict], lnf, logits):
+        """The weights of decoderStep.  A layer maps sqkv, so, cq, co, f1, f2 to (weights, bias) and ln1..ln3 to
+        (gamma, beta); lnf is (gamma, beta), logits the vocabulary matrix."""
+        arr = (_lib.DecoderLayer * len(layers))()
+        for d, w in zip(arr, layers):
+            for n in ("sqkv", "so", "cq", "co", "f1", "f2"):
+                setattr(d, n, self._linear_of(*w[n]))
+            for n in ("ln1", "ln2", "ln3"):
+                setattr(d, n + "_w", w[n][0].h), setattr(d, n + "_b", w[n][1].h)
+        return arr, lnf[0].h, lnf[1].h, self._linear_of(logits, None)
+
+    def decoderStep(self, weights, x, crossK, crossV, selfK, selfV, n: int, NH: int, HD: int) -> Tensor:
+        """Optional member: one token of S streams through all layers, x [S, D] -> logits (see fa_decoder_step)."""
+        arr, g, b, logits = weights
+        handles = lambda ts: (C.c_void_p * len(arr))(*[t.h for t in ts])  # noqa: E731
+        return self._op(self._lib.fa_decoder_step, arr, len(arr), x.h, handles(crossK), handles(crossV), handles(selfK), handles(selfV),
+                        n, NH, HD, g, b, C.byref(logits))
+
+    def conformerWeights(self, w: dict):
+        """The weights of conformerBlock from an encoder layer's dict of tensors (absent ones: None)."""
+        h = lambda n, i=None: self._h_of(w.get(n) if i is None else w[n][i])  # noqa: E731
+        ff = lambda n: _lib.FeedForward(h("ln" + n, 0), h("ln" + n, 1), h(n + "w1"), h(n + "w2"), h(n + "b1"), h(n + "b2"))  # noqa: E731
+        d = _lib.ConformerLayer(ff("ff1"), ff("ff2"))
+        for n in ("lnatt", "lnconv", "lnout"):
+            setattr(d, n + "_w", h(n, 0)), setattr(d, n + "_b", h(n, 1))
+        for n in ("q", "k", "v", "qkv", "pos", "out", "qb", "kb", "vb", "qkvb", "outb", "pw1b", "pw2b", "dw", "dwb"):
+            setattr(d, n, h(n))
+        d.pw1, d.pw2, d.pbu, d.pbv = h("pw1T"), h("pw2T"), h("pbuAll"), h("pbvAll")
+        return d
+
+    def conformerBlock(self, weights, x, xff, pos, posProjected: bool, H: int, HD: int, W: int, dwK: int, nextLn=None):
+        """Optional member: one conformer block (see fa_conformer_block) -> (x, layernorm(x, nextLn) or None)."""
+        y, z = C.c_void_p(), C.c_void_p()
+        g, b = nextLn if nextLn is not None else (None, None)
+        self._check(self._lib.fa_conformer_block(self._h, C.byref(weights), x.h, self._h_of(xff), pos.h, 1 if posProjected else 0, H, HD,
+                                                 W, dwK, self._h_of(g), self._h_of(b), C.byref(y), C.byref(z)))
+        return self._wrap(y), (self._wrap(z) if z.value else None)
+
     def attnFused(self, q, k, v, pos, pbu, pbv, H: int, HD: int, W: int) -> Optional[Tensor]:
         """Fused rel-pos self-attention (optional member, compute.d.ts:247-248).  Returns None when the
         shape is outside the fused kernel's range - the caller then runs the separate ops."""

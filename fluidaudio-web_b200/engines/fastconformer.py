@@ -132,7 +132,10 @@ def load_encoder(ctx, weights: Dict[str, np.ndarray], cfg_override: Optional[dic
                 lw["qkvb"] = ctx.upload(b, 1, b.size)
             else:
                 lw["qkvb"] = None
-    return dict(sub=sub, layers=layers, cfg=cfg, _pe={}, _posProj={})
+    enc = dict(sub=sub, layers=layers, cfg=cfg, _pe={}, _posProj={})
+    if hasattr(ctx, "conformerBlock") and not any(isinstance(t, Int8Weight) for lw in layers for t in lw.values()):
+        enc["native"] = [ctx.conformerWeights(lw) for lw in layers]  # optional member: a block in one call
+    return enc
 
 
 def pos_encoding(Tsub: int, D: int) -> np.ndarray:
@@ -253,6 +256,14 @@ def encode_batch(ctx, enc, mels: List[np.ndarray], layer_hook=None, use_fast: bo
         xn = ln_op(x, lp) if xn is None else xn
         return mm(ctx, mm(ctx, xn, w1, dict(bias=b1, act="silu")), w2, dict(bias=b2, add=x))
 
+    def pos_proj(L, w):
+        """The projected positional table: constant per (layer, Tsub), cached across groups of windows (:307-317)."""
+        p = enc["_posProj"].get((L, Tsub))
+        if p is None:
+            p = ctx.pin(mm(ctx, peT, w["pos"]))
+            enc["_posProj"][(L, Tsub)] = p
+        return p
+
     # optional member: a block's last layernorm and the next block's first one in one pass over the rows
     chain = use_fast and hasattr(ctx, "layernormChain")
 
@@ -263,23 +274,27 @@ def encode_batch(ctx, enc, mels: List[np.ndarray], layer_hook=None, use_fast: bo
             layerArena = ctx.pushArena()
             try:
                 w = enc["layers"][L]
+                if use_fast and "native" in enc:
+                    p = pos_proj(L, w) if W > 1 else peT
+                    nxt = enc["layers"][L + 1]["lnff1"] if L + 1 < LAYERS else None
+                    x, xff = ctx.conformerBlock(enc["native"][L], x, xff, p, W > 1, H, HD, W, dwK, nxt)
+                    ctx.pin(x, True)  # x feeds the next layer: promote to the enclosing arena
+                    if xff is not None:
+                        ctx.pin(xff, True)
+                    if layer_hook is not None:
+                        layer_hook(L, x)
+                    continue
                 x = ff(x, w["lnff1"], w["ff1w1"], w["ff1w2"], w["ff1b1"], w["ff1b2"], xff)
                 xff = None
                 xln = ln_op(x, w["lnatt"])
-                fused_qkv = use_fast and "qkv" in w and W * Tsub >= 256 and 16 <= Tsub <= 192
-                if fused_qkv:
-                    qkv = mm(ctx, xln, w["qkv"], dict(bias=w["qkvb"], operandOnly=True))  # read by attnFusedQKV only
+                fused_qkv = use_fast and "qkv" in w and 16 <= Tsub <= 192
+                if fused_qkv:  # read by attnFusedQKV only; from 256 rows on as the packed operand alone
+                    qkv = mm(ctx, xln, w["qkv"], dict(bias=w["qkvb"], operandOnly=W * Tsub >= 256))
                 else:
                     q = mm(ctx, xln, w["q"], dict(bias=w["qb"]))
                     k = mm(ctx, xln, w["k"], dict(bias=w["kb"]))
                     v = mm(ctx, xln, w["v"], dict(bias=w["vb"]))
-                if W > 1:  # pos projection is constant per (layer, Tsub): cached across groups (:307-317)
-                    p = enc["_posProj"].get((L, Tsub))
-                    if p is None:
-                        p = ctx.pin(mm(ctx, peT, w["pos"]))
-                        enc["_posProj"][(L, Tsub)] = p
-                else:
-                    p = mm(ctx, peT, w["pos"])
+                p = pos_proj(L, w) if W > 1 else mm(ctx, peT, w["pos"])
                 outc = None
                 if fused_qkv:
                     outc = ctx.attnFusedQKV(qkv, p, w["pbuAll"], w["pbvAll"], H, HD, W)

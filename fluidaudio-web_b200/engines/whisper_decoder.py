@@ -55,6 +55,9 @@ class _W:
         else:
             self.t = ctx.uploadF16(np.ascontiguousarray(a, dtype=f32), K, N)
 
+    def native(self):
+        return (self.q, self.s, self.N, self.K) if self.quant == "int8" else self.t
+
 
 def _mm(ctx, x, w: _W, bias=None, act="none"):
     if w.quant == "int8":
@@ -126,8 +129,14 @@ def load_decoder(ctx, weights: Dict[str, np.ndarray], NH: int, quant: Optional[s
     embedTP = np.zeros((D, VOCABP), f32)
     embedTP[:, :VOCAB] = embed.T
     cfg["VOCABP"] = VOCABP
-    return dict(layers=layers, embed=embed, embedT=_W(ctx, embedTP, quant), pos=np.ascontiguousarray(weights["pos"], dtype=f32),
-                lnf=(vec("lnf_w"), vec("lnf_b")), cfg=cfg)
+    dec = dict(layers=layers, embed=embed, embedT=_W(ctx, embedTP, quant), pos=np.ascontiguousarray(weights["pos"], dtype=f32),
+               lnf=(vec("lnf_w"), vec("lnf_b")), cfg=cfg)
+    if hasattr(ctx, "decoderStep"):  # optional member: all layers of a token in one call
+        pair = lambda w, k: (w[k + "w"].native(), w.get(k + "b"))
+        dec["native"] = ctx.decoderWeights([dict(sqkv=pair(w, "sqkv"), so=pair(w, "so"), cq=pair(w, "cq"), co=pair(w, "co"),
+                                                 f1=pair(w, "f1"), f2=pair(w, "f2"), ln1=w["ln1"], ln2=w["ln2"], ln3=w["ln3"])
+                                            for w in layers], dec["lnf"], dec["embedT"].native())
+    return dec
 
 
 def _self_attention(ctx, x, w, cacheK, cacheV, n, S, D, NH, HD):
@@ -168,6 +177,17 @@ def _layer(ctx, x, w, kv, cacheK, cacheV, n, S, D, NH, HD):
     return _linear(ctx, h, w["f2w"], bias=w["f2b"], add=x)
 
 
+def _step(ctx, dec, kv, st, x, n, S):
+    """The device part of one token: x [S, D] (embedding + position n) -> logits [S, VOCABP]."""
+    cfg = dec["cfg"]
+    D, NH, HD = cfg["D"], cfg["NH"], cfg["HD"]
+    if "native" in dec:
+        return ctx.decoderStep(dec["native"], x, [c["k"] for c in kv], [c["v"] for c in kv], st["selfK"], st["selfV"], n, NH, HD)
+    for li, w in enumerate(dec["layers"]):
+        x = _layer(ctx, x, w, kv[li], st["selfK"][li], st["selfV"][li], n, S, D, NH, HD)
+    return _linear(ctx, x, dec["embedT"], norm=dec["lnf"])
+
+
 # ---------------------------------------------------------------------------- one stream (reference form)
 
 def cross_kv(ctx, dec, enc):
@@ -190,19 +210,15 @@ def decode_init(ctx, dec, maxLen: int = 448) -> dict:
 
 def decode_next(ctx, dec, kv, st, token: int) -> np.ndarray:
     """Feed one token through the cached decoder; logits [VOCAB] for it (:103-142)."""
-    cfg = dec["cfg"]
-    D, NH, HD, VOCAB = cfg["D"], cfg["NH"], cfg["HD"], cfg["VOCAB"]
+    D, VOCAB = dec["cfg"]["D"], dec["cfg"]["VOCAB"]
     n = st["n"]
     emb = dec["embed"][token] + dec["pos"][n]
     x = ctx.upload(emb, 1, D)
     arena = ctx.pushArena()
 
     def body():
-        nonlocal x
-        for li, w in enumerate(dec["layers"]):
-            x = _layer(ctx, x, w, kv[li], st["selfK"][li], st["selfV"][li], n, 1, D, NH, HD)
+        logits = _step(ctx, dec, kv, st, x, n, 1)
         st["n"] = n + 1
-        logits = _linear(ctx, x, dec["embedT"], norm=dec["lnf"])  # [1, VOCABP]
         return ctx.stageDownload(logits)
 
     try:
@@ -211,6 +227,7 @@ def decode_next(ctx, dec, kv, st, token: int) -> np.ndarray:
         return full[:VOCAB] if full.size > VOCAB else full
     finally:
         ctx.popArena(arena)
+        ctx.freeTensor(x)
 
 
 def greedy_decode(ctx, dec, enc, prefix: Sequence[int], n_tokens: int, margins: Optional[list] = None) -> List[int]:
@@ -257,12 +274,7 @@ def decode_init_streams(ctx, dec, S: int, maxLen: int = 448) -> dict:
 def step_streams(ctx, dec, kv, st, x, n: int):
     """The device part of one lock-step token for S streams: x [S, D] (embedding + position n) ->
     logits [S, VOCABP].  Same per-row arithmetic as decode_next."""
-    cfg = dec["cfg"]
-    D, NH, HD = cfg["D"], cfg["NH"], cfg["HD"]
-    S = st["S"]
-    for li, w in enumerate(dec["layers"]):
-        x = _layer(ctx, x, w, kv[li], st["selfK"][li], st["selfV"][li], n, S, D, NH, HD)
-    return _linear(ctx, x, dec["embedT"], norm=dec["lnf"])
+    return _step(ctx, dec, kv, st, x, n, st["S"])
 
 
 def decode_next_streams(ctx, dec, kv, st, tokens: Sequence[int], want_logits: bool = False):
@@ -293,6 +305,7 @@ def decode_next_streams(ctx, dec, kv, st, tokens: Sequence[int], want_logits: bo
         return np.argmax(lg, axis=1).astype(np.int64), lg
     finally:
         ctx.popArena(arena)
+        ctx.freeTensor(x)
 
 
 def greedy_decode_streams(ctx, dec, encs: Sequence, prefix: Sequence[int], n_tokens: int,

@@ -76,8 +76,7 @@ const char *fa_last_error(fa_ctx *ctx);
  * attnFused runs as one kernel per call when head width is 128 and T <= 192; 0 = the batched-GEMM form),
  * "nbits_mma_rows" (0..17, default 16: int4 products with more activation rows than the GEMV takes and at most this
  * many - at most 16 - stream the 4-bit weights once as uploaded, widen them to f16 in registers and multiply with
- * mma.sync, when the matrix is narrow enough for that to beat the tensor-core GEMM on the dequantised copy; 17 = for
- * every width; 0 = never), "tc_pair" (0/1, default 1: f16-weight products with more tiles than SMs run on pairs of thread blocks that
+ * mma.sync, for N % 8 == 0 and K <= 8192; 17 = 16; 0 = never), "tc_pair" (0/1, default 1: f16-weight products with more tiles than SMs run on pairs of thread blocks that
  * share one 256-lane tcgen05 MMA, each loading half of the activation rows of the pair's tile; results are
  * bit-identical to the one-block kernel, 0 selects that kernel), "tc_tma_store" (0/1, default 1: results of plain
  * tensor-core products leave through shared-memory slabs and copy-engine stores; 0 = per-lane stores, same values),
@@ -269,6 +268,40 @@ int fa_linear_step(fa_ctx *ctx, const fa_tensor *x, const fa_tensor *gamma, cons
 int fa_attn_step(fa_ctx *ctx, const fa_tensor *q, const fa_tensor *k, const fa_tensor *v, int H, int HD, int W, fa_tensor **out);
 int fa_attn_step_append(fa_ctx *ctx, const fa_tensor *qkv, fa_tensor *cache_k, fa_tensor *cache_v, int n, int NH, int HD,
                         fa_tensor **out);
+/* ---- layer loops of the two transformer engines (optional members) --------------------------------
+ * The members above in the engines' order, issued from native code: one call per decoder token or encoder block.  Results
+ * belong to the caller's newest arena, everything in between is released. */
+typedef struct fa_linear { /* a weight matrix [K][N] and its bias (may be NULL) */
+  void *w;                 /* fa_tensor, or fa_bytes (int8) when scale is given */
+  const fa_tensor *scale, *bias;
+  int N, K;
+} fa_linear;
+typedef struct fa_decoder_layer { /* raw-whisper-decoder.js:38-61; sqkv = self-attention q | k | v, q scaled by 1/sqrt(HD) */
+  fa_linear sqkv, so, cq, co, f1, f2;
+  const fa_tensor *ln1_w, *ln1_b, *ln2_w, *ln2_b, *ln3_w, *ln3_b;
+} fa_decoder_layer;
+/* One token of S streams: x [S, D] (embedding + position) -> logits [S, N].  cross_k / cross_v [S*Tenc, D] and the caches
+ * self_k / self_v [positions, S*D] per layer; row n of the caches becomes the token's (raw-whisper-decoder.js:103-142). */
+int fa_decoder_step(fa_ctx *ctx, const fa_decoder_layer *layers, int n_layers, const fa_tensor *x, fa_tensor *const *cross_k,
+                    fa_tensor *const *cross_v, fa_tensor *const *self_k, fa_tensor *const *self_v, int n, int NH, int HD,
+                    const fa_tensor *lnf_w, const fa_tensor *lnf_b, const fa_linear *logits, fa_tensor **out);
+typedef struct fa_feed_forward {
+  const fa_tensor *ln_w, *ln_b;
+  fa_tensor *w1, *w2;
+  const fa_tensor *b1, *b2;
+} fa_feed_forward;
+typedef struct fa_conformer_layer { /* raw-encoder.js:95-131; biases may be NULL, qkv (q | k | v side by side) too */
+  fa_feed_forward ff1, ff2;
+  const fa_tensor *lnatt_w, *lnatt_b, *lnconv_w, *lnconv_b, *lnout_w, *lnout_b;
+  fa_tensor *q, *k, *v, *qkv, *pos, *out, *pw1, *pw2;
+  const fa_tensor *qb, *kb, *vb, *qkvb, *outb, *pw1b, *pw2b, *pbu, *pbv, *dw, *dwb;
+} fa_conformer_layer;
+/* One conformer block over W windows of x.rows / W frames (raw-encoder.js:270-384).  x_ff: layernorm(x, ff1.ln) when the
+ * block before made it, else NULL.  pos: positional encodings [2T-1, D], or their projection when pos_projected.  With
+ * next_w / next_b (the next block's ff1.ln) *out_ff is layernorm(*out, next), else NULL. */
+int fa_conformer_block(fa_ctx *ctx, const fa_conformer_layer *w, const fa_tensor *x, const fa_tensor *x_ff, const fa_tensor *pos,
+                       int pos_projected, int H, int HD, int W, int dw_k, const fa_tensor *next_w, const fa_tensor *next_b,
+                       fa_tensor **out, fa_tensor **out_ff);
 /* attnFused :247-248 (optional member; may yield no tensor, the caller then uses the separate ops):
  * rel-pos self-attention for W windows of T = q.rows/W frames; pos [2T-1, H*HD] is the projected
  * positional table, pbu/pbv [1, H*HD].  *out == NULL with status 0 means "not this shape". */

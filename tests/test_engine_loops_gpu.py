@@ -1,0 +1,58 @@
+"""The native layer loops issue the members of the host loops: same results, bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+# one short window (few-row products), a group whose q|k|v stays f32, one that keeps it packed, frames past the attention kernel
+@pytest.mark.parametrize("W,samples", [(1, 59200), (3, 64000), (2, 171200), (1, 320000)])
+def test_conformer_blocks(ctx, pkg, W, samples):
+    from fluidaudio_web_b200.engines import fastconformer as fc, synth
+
+    enc = fc.load_encoder(ctx, synth.encoder_weights(dict(synth.PARAKEET_06B, layers=2), seed=4))
+    mel = ctx.logMelWindows(ctx.upload(synth.synth_audio(W, samples=samples, seed=5), W, samples), 128)
+    native = enc.pop("native")
+    host, t0 = fc.encode_batch(ctx, enc, mel)
+    host = ctx.download(host)
+    seen = []
+    enc["native"] = native
+    got, t1 = fc.encode_batch(ctx, enc, mel, layer_hook=lambda L, x: seen.append((L, x.rows)))
+    assert t0 == t1 and [s[0] for s in seen] == [0, 1]
+    assert np.array_equal(ctx.download(got), host)
+
+
+@pytest.mark.parametrize("quant", [None, "int8"])
+@pytest.mark.parametrize("S", [1, 3])
+@pytest.mark.parametrize("NH", [4, 16])  # head widths 64 and 16
+def test_decoder_tokens(ctx, pkg, quant, S, NH):
+    from fluidaudio_web_b200.engines import synth, whisper_decoder as wd
+
+    cfg = dict(D=256, NH=NH, FFN=1024, layers=2, VOCAB=2003, maxPos=40, Tenc=96)
+    dec = wd.load_decoder(ctx, synth.decoder_weights(cfg, seed=11), NH, quant=quant)
+    states = ctx.upload(np.concatenate(synth.encoder_states(cfg, S, seed=13)), S * cfg["Tenc"], cfg["D"])
+    native, runs = dec["native"], []
+    for with_native in (True, False):
+        if not with_native:
+            dec.pop("native")
+        kv = wd.cross_kv_streams(ctx, dec, states)
+        st = wd.decode_init_streams(ctx, dec, S, 8)
+        runs.append([wd.decode_next_streams(ctx, dec, kv, st, [t] * S, want_logits=True)[1] for t in (1, 7, 3)])
+    dec["native"] = native
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b)
+
+
+def test_decode_next_gives_its_row_back(ctx, pkg):
+    from fluidaudio_web_b200.engines import synth, whisper_decoder as wd
+
+    cfg = dict(D=256, NH=4, FFN=1024, layers=2, VOCAB=2003, maxPos=40, Tenc=96)
+    dec = wd.load_decoder(ctx, synth.decoder_weights(cfg, seed=11), 4)
+    kv = wd.cross_kv(ctx, dec, ctx.upload(synth.encoder_states(cfg, 1, seed=13)[0], cfg["Tenc"], cfg["D"]))
+    st = wd.decode_init(ctx, dec, 16)
+    for t in range(3):
+        wd.decode_next(ctx, dec, kv, st, t)
+    before = ctx.memStats()
+    for t in range(5):
+        wd.decode_next(ctx, dec, kv, st, t)
+    assert ctx.memStats() ["created"] == before["created"]
