@@ -306,7 +306,8 @@ __device__ __forceinline__ float block_sum(float v, float *red, int lane, int wa
 //
 // What bounds it: the weight stream of the large matrices (66 MB of int8 for the vocabulary projection), latency for the
 // others: 1.6 MB are 0.3 us of HBM time, so the launch is a chain of load -> row sum -> exchange between K slices.
-// Hence the layout: a block owns 128 columns (one 4-byte int8 or 8-byte f16 load per lane and row) and a K slice, its
+// Hence the layout: a block owns 128 columns (one 4-byte int8 or 8-byte f16 load per lane and row; 64 columns, two rows
+// per warp, where 128 with the widest K split would not give every SM a block) and a K slice, its
 // 8 warps take rows round-robin with two batches of kKnU loads per lane in flight, the first ones requested before the launch waits
 // for its predecessor where the weights can only have been written by an upload (int8 payloads).  K slices are the
 // ranks of a cluster: their sums meet in rank 0's shared memory, in rank order, after one cluster barrier.  (The form
@@ -314,8 +315,9 @@ __device__ __forceinline__ float block_sum(float v, float *red, int lane, int wa
 // Measured, K = N = 1280 int8 in a decoder step: 7.3 us from launch to end, wait for the predecessor included, where the
 // layernorm, product and residual add were three launches; 1280 x 51868 int8 with the layernorm 25 us (2.7 TB/s) against
 // a layernorm, a digit pass and a tensor-core product of 3.8 + 2.6 + 12.5 us that read the row as two int8 digits
-// instead of f32.  A 16-token decoder pass of one stream: 8.24 -> 5.1 ms, what is left is the host's 9 us per launch.
-constexpr int kKnU = 16, kKnCols = 128, kKnSlice = 2048;  // loads in a lane's batch, columns per block, rows of x held at a time
+// instead of f32.  A 16-token decoder pass of one stream: 8.24 -> 5.1 ms.  Blocks of
+// 64 columns (K = 1280 and 5120, N = 1280): 8.2 -> 6.5 us a product on average, the pass 4.85 -> 4.56 ms.
+constexpr int kKnU = 16, kKnCols = 128, kKnSlice = 2048;  // loads in a lane's batch, most columns per block, rows of x held at a time
 constexpr int kKnNormMax = 4096;                           // longest row that the layernorm prologue holds in registers
 
 struct KnParams {
@@ -327,32 +329,33 @@ struct KnParams {
   GemvEp ep;
 };
 
-template <bool I8, bool NORM>
+template <bool I8, bool NORM, int COLS>
 __global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
   __shared__ __align__(16) float xs[kKnSlice];
-  __shared__ __align__(16) float4 red[kThreads / 32][32];
-  __shared__ float cred[8][kKnCols];  // rank 0: the K slices' sums
+  constexpr int RPW = kKnCols / COLS, kStride = 8 * RPW;  // rows a warp reads at once, rows of a block's 8 warps
+  __shared__ __align__(16) float4 red[kThreads / 32][COLS / 4];
+  __shared__ float cred[8][COLS];  // rank 0: the K slices' sums
   __shared__ float stat[kThreads / 32];
   using Raw = typename RawRow<I8>::type;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.y, ks = gridDim.y, N = p.N, K = p.K;
   const int k0 = rank * p.kslice, k1 = min(K, k0 + p.kslice);
-  const int c0 = blockIdx.x * kKnCols + lane * 4;
+  const int c0 = blockIdx.x * COLS + (lane % (COLS / 4)) * 4;
   const bool live = c0 < N;  // N % 4 == 0: a live lane owns four whole columns
   const int cc = live ? c0 : 0;
   Raw ra[kKnU], rb[kKnU];
   auto fetch = [&](Raw(&raw)[kKnU], int kk) {
 #pragma unroll
     for (int u = 0; u < kKnU; u++) {
-      const int k = kk + u * 8;
+      const int k = kk + u * kStride;
       raw[u] = Raw{};
       if (k < k1) raw[u] = load_raw<I8>(p.w, (size_t)k * N + cc);
     }
   };
-  int kk = k0 + warp;  // rows kk, kk + 8, ...
-  if (I8) fetch(ra, kk), fetch(rb, kk + 8 * kKnU);
+  int kk = k0 + warp * RPW + lane / (COLS / 4);  // rows kk, kk + kStride, ...
+  if (I8) fetch(ra, kk), fetch(rb, kk + kStride * kKnU);
   if (ks > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // every rank runs before a remote store
   fa_grid_dep_sync();
-  if (!I8) fetch(ra, kk), fetch(rb, kk + 8 * kKnU);
+  if (!I8) fetch(ra, kk), fetch(rb, kk + kStride * kKnU);
   if (NORM) {
     float4 v[kKnNormMax / 4 / kThreads];
     const int k4 = K >> 2;
@@ -394,7 +397,7 @@ __global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
     auto consume = [&](const Raw(&raw)[kKnU], int kk) {
 #pragma unroll
       for (int u = 0; u < kKnU; u++) {
-        const int k = kk + u * 8;
+        const int k = kk + u * kStride;
         if (k < end) {
           const float a = xs[k - base];
           const float4 f = widen(raw[u]);
@@ -402,25 +405,32 @@ __global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
         }
       }
     };
-    for (; kk < end; kk += 16 * kKnU) {  // no pair of batches straddles `end` on its way: kKnSlice % (16 * kKnU) == 0
+    constexpr int B = kStride * kKnU;  // rows of a batch
+    static_assert(kKnSlice % (2 * B) == 0, "no pair of batches straddles `end` on its way");
+    for (; kk < end; kk += 2 * B) {
       consume(ra, kk);
-      if (kk + 16 * kKnU < k1) fetch(ra, kk + 16 * kKnU);
-      consume(rb, kk + 8 * kKnU);
-      if (kk + 24 * kKnU < k1) fetch(rb, kk + 24 * kKnU);
+      if (kk + 2 * B < k1) fetch(ra, kk + 2 * B);
+      consume(rb, kk + B);
+      if (kk + 3 * B < k1) fetch(rb, kk + 3 * B);
     }
   }
-  red[warp][lane] = acc;
+  if (RPW == 2) {
+    __syncwarp();
+    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 16), acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 16);
+    acc.z += __shfl_xor_sync(0xffffffffu, acc.z, 16), acc.w += __shfl_xor_sync(0xffffffffu, acc.w, 16);
+  }
+  if (lane < COLS / 4) red[warp][lane] = acc;
   __syncthreads();
   float sum = 0.f;
-  if (tid < kKnCols) {
+  if (tid < COLS) {
     const float *r = (const float *)red;
     sum = r[tid];
 #pragma unroll
-    for (int i = 1; i < kThreads / 32; i++) sum += r[i * kKnCols + tid];
+    for (int i = 1; i < kThreads / 32; i++) sum += r[i * COLS + tid];
   }
   if (ks > 1) {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (tid < kKnCols) {
+    if (tid < COLS) {
       uint32_t remote;
       const uint32_t local = (uint32_t)__cvta_generic_to_shared(&cred[rank][tid]);
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(0));
@@ -428,13 +438,13 @@ __global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (rank != 0) return;
-    if (tid < kKnCols) {
+    if (tid < COLS) {
       sum = cred[0][tid];
       for (int i = 1; i < ks; i++) sum += cred[i][tid];
     }
   }
-  const int n = blockIdx.x * kKnCols + tid;
-  if (tid < kKnCols && n < N) p.y[n] = gemv_finish(sum, 0, n, N, p.ep);
+  const int n = blockIdx.x * COLS + tid;
+  if (tid < COLS && n < N) p.y[n] = gemv_finish(sum, 0, n, N, p.ep);
 }
 
 template <int M, int R, int PRE>
@@ -785,7 +795,8 @@ int fa_gemv_kn(fa_ctx *ctx, const float *x, const float *gamma, const float *bet
   KnParams p{x, gamma, beta, w, y, K, N, 0, eps, GemvEp{colscale, bias, add, act}};
   // K slices = ranks of a cluster, as many (1, 2, 4, 8) as give about two blocks per SM and leave 64 rows to each; the
   // layernorm form needs its slice in shared memory whole.
-  const int strips = ceil_div(N, kKnCols);
+  const bool narrow = ceil_div(N, kKnCols) * 8 < ctx->sm_count;
+  const int strips = ceil_div(N, narrow ? kKnCols / 2 : kKnCols);
   int ks = 1;
   while (ks < 8 && strips * ks * 2 <= 2 * ctx->sm_count + ctx->sm_count / 4 && K >= 64 * ks * 2) ks *= 2;
   while (gamma && ks < 8 && ceil_div(K, ks) > kKnSlice) ks *= 2;
@@ -806,10 +817,11 @@ int fa_gemv_kn(fa_ctx *ctx, const float *x, const float *gamma, const float *bet
   cudaError_t e;
   {
     LaunchScope ls(ctx, i8 ? "gemv_i8" : "gemv_f16");
-    if (gamma)
-      e = i8 ? cudaLaunchKernelEx(&cfg, k_gemv_kn<true, true>, p) : cudaLaunchKernelEx(&cfg, k_gemv_kn<false, true>, p);
-    else
-      e = i8 ? cudaLaunchKernelEx(&cfg, k_gemv_kn<true, false>, p) : cudaLaunchKernelEx(&cfg, k_gemv_kn<false, false>, p);
+    auto kern = gamma ? (i8 ? (narrow ? k_gemv_kn<true, true, 64> : k_gemv_kn<true, true, 128>)
+                            : (narrow ? k_gemv_kn<false, true, 64> : k_gemv_kn<false, true, 128>))
+                      : (i8 ? (narrow ? k_gemv_kn<true, false, 64> : k_gemv_kn<true, false, 128>)
+                            : (narrow ? k_gemv_kn<false, false, 64> : k_gemv_kn<false, false, 128>));
+    e = cudaLaunchKernelEx(&cfg, kern, p);
   }
   if (e != cudaSuccess) return fa_fail(ctx, FA_ERR_CUDA, "launch gemv_kn: %s", cudaGetErrorString(e));
   return FA_OK;
