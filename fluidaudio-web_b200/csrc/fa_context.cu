@@ -159,6 +159,10 @@ extern "C" int fa_ctx_set_option(fa_ctx *ctx, const char *key, long long value) 
     ctx->nbits_mma_rows = (int)value;
     return FA_OK;
   }
+  if (!strcmp(key, "tc_wide_stages")) {
+    ctx->tc_wide_stages = value != 0;
+    return FA_OK;
+  }
   if (!strcmp(key, "tc_pair")) {
     ctx->tc_pair = value != 0;
     return FA_OK;

@@ -79,6 +79,7 @@ struct TcParams {
                       // accumulated into the SAME TMEM columns (f32-grade activations for decode-size products)
   int stages;
   int num_kb;         // K chunks of 128 bytes
+  int step;           // K chunks per ring stage, 1 or 2 (see launch_tc)
   int tiles_n, tiles_m;
   int splitk;         // > 1: cluster of `splitk` CTAs along z shares one tile, each taking kb_per_split chunks
   int kb_per_split;
@@ -564,12 +565,15 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
   constexpr uint32_t kWTiles = KIND == 4 ? 2u : 1u;  // weight tiles per stage (KIND 4: value and residue planes)
   constexpr bool kTwoProd = !kDeq;  // a second producer thread (warp 2 + kEpiWarps) loads the activation tiles
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  // carve: [stages] x (P tile 16 KB | Q tile limbs*MT*128 B | raw nibble tile 4 KB for KIND 2), barriers,
+  // carve: [stages] x (P tile 16 KB | Q tile limbs*MT*128 B, both twice with two chunks | raw nibble tile 4 KB for KIND 2), barriers,
   // split-K partial tile
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int q_rows = p.MT * p.limbs;
   const uint32_t q_bytes = (uint32_t)q_rows * kRowBytes;
-  const uint32_t stage_bytes = kWTiles * kPTileBytes + q_bytes + (uint32_t)tc_raw_bytes<KIND>();
+  constexpr bool kStep = KIND <= 1;  // stages of two K chunks: [weights 0 | weights 1 | activations 0 | activations 1]
+  const int step = kStep ? p.step : 1;
+  const uint32_t w_bytes = kWTiles * kPTileBytes * (uint32_t)step;
+  const uint32_t stage_bytes = w_bytes + q_bytes * (uint32_t)step + (uint32_t)tc_raw_bytes<KIND>();
   const uint32_t bars = smem_base + (uint32_t)p.stages * stage_bytes;  // 8-byte aligned (stage_bytes % 1024 == 0)
   auto full_bar = [&](int s) { return bars + (uint32_t)s * 8u; };
   auto empty_bar = [&](int s) { return bars + (uint32_t)(p.stages + s) * 8u; };
@@ -664,13 +668,13 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         int aslab = (p.a_shared ? 0 : batch) * p.limbs * p.num_kb + kb0;
         const int m0 = tm * p.MT;
         const int wh = tile == 0 ? p.withhold_kb : -1;  // test hook: this chunk never arrives
-        for (int kb = kb0; kb < kb1; kb++, wrow += 128, aslab++) {
+        for (int kb = kb0; kb < kb1; kb += step, wrow += 128 * step, aslab += step) {
           if (!__all_sync(0xffffffffu, mbar_wait(fb + eoff, ph ^ 1u, p.wait_limit))) {  // empty barrier of the slot, previous use
             if (lane == 0) set_abort(1, kb);
             stop = true;
             break;
           }
-          if (kb != wh) {
+          if ((unsigned)(wh - kb) >= (unsigned)step) {
             if (KIND == 5) {
               mbar_expect_tx_w(lead, fb, q_bytes + kRaw8TileBytes);
               tma_load_2d_w(lead, dst + kPTileBytes - kRaw8TileBytes, &map_w, 0, (tn * p.num_kb + kb) * 32, fb);  // 8 KB int8 tile, in
@@ -706,7 +710,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     {
       const uint32_t lead = elect_lead();
       const uint32_t fb_end = bars + (uint32_t)p.stages * 8u, eoff = (uint32_t)p.stages * 8u;
-      uint32_t fb = bars, dst = smem_base + kWTiles * kPTileBytes, ph = 0;
+      uint32_t fb = bars, dst = smem_base + w_bytes, ph = 0;
       const uint32_t dst0 = dst;
       bool stop = false;
       for (int tile = blockIdx.x; tile < num_tiles && !stop; tile += gridDim.x) {
@@ -715,16 +719,20 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         int aslab = (p.a_shared ? 0 : batch) * p.limbs * p.num_kb + kb0;
         const int m0 = tm * p.MT;
         const int wh = tile == 0 ? p.withhold_kb : -1;
-        for (int kb = kb0; kb < kb1; kb++, aslab++) {
+        for (int kb = kb0; kb < kb1; kb += step, aslab += step) {
           if (!__all_sync(0xffffffffu, mbar_wait(fb + eoff, ph ^ 1u, p.wait_limit))) {
             if (lane == 0) set_abort(7, kb);
             stop = true;
             break;
           }
-          if (kb != wh) {
-            tma_load_3d_w(lead, dst, &map_a, 0, m0, aslab, fb);
-            for (int l = 1; l < p.limbs; l++)
-              tma_load_3d_w(lead, dst + (uint32_t)(l * p.MT) * kRowBytes, &map_a, 0, m0, aslab + l * p.num_kb, fb);
+          if ((unsigned)(wh - kb) >= (unsigned)step) {
+            if (kStep && step == 2) {
+              tma_load_4d_w(lead, dst, &map_a, 0, m0, 0, kb, fb);  // both chunks, all planes
+            } else {
+              tma_load_3d_w(lead, dst, &map_a, 0, m0, aslab, fb);
+              for (int l = 1; l < p.limbs; l++)
+                tma_load_3d_w(lead, dst + (uint32_t)(l * p.MT) * kRowBytes, &map_a, 0, m0, aslab + l * p.num_kb, fb);
+            }
           }
           fb += 8u;
           dst += stage_bytes;
@@ -746,15 +754,16 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
       const uint32_t idesc = make_idesc(MK, 128, acc_cols);
       const uint64_t desc0 = smem_desc_sw128(smem_base);  // slot 0 weights tile; other tiles are address offsets
       const uint32_t d_hi = (uint32_t)(desc0 >> 32), da0 = (uint32_t)desc0;
-      const uint32_t q_off = (kWTiles * kPTileBytes) >> 4, st_off = stage_bytes >> 4;
+      const uint32_t q_off = w_bytes >> 4, st_off = stage_bytes >> 4;
       const uint32_t wlo_off = kPTileBytes >> 4;                    // KIND 4: residue plane of the weights
       const uint32_t lo_off = (uint32_t)(p.MT * kRowBytes) >> 4;    // residue plane of the activations
       const uint32_t fb_end = bars + (uint32_t)p.stages * 8u, eoff = (uint32_t)p.stages * 8u;
       const uint32_t doff = (2u * (uint32_t)p.stages + 4u) * 8u;    // full barrier -> unpack barrier of the slot
       uint32_t fb = bars, da = da0, ph = 0, lt = 0;
       bool ok = true;
-      auto run = [&](auto ls_tag) {
+      auto run = [&](auto ls_tag, auto step_tag) {
         constexpr bool kLimbSum = decltype(ls_tag)::value;
+        constexpr int kSub = decltype(step_tag)::value;  // K chunks per stage
         for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, lt++) {
           const uint32_t buf = lt & 1, use = lt >> 1;
           if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(acc_empty(buf), (use - 1) & 1, p.wait_limit))) {
@@ -764,7 +773,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + buf * acc_stride;
           uint32_t acc = 0;
-          for (int kb = kb0; kb < kb1; kb++) {
+          for (int kb = kb0; kb < kb1; kb += kSub) {
             if (!__all_sync(0xffffffffu, mbar_wait(fb, ph, p.wait_limit))) {
               if (lane == 0) set_abort(2, kb);
               ok = false;
@@ -778,23 +787,26 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
               }
               tc_fence_after();
             }
-            const uint32_t db = da + q_off;
-            umma_lo_w<MK>(lead, d_tmem, da, db, d_hi, idesc, acc);  // 4 x 32 bytes of K per slot
-            acc = 1u;
-            umma_lo_w<MK>(lead, d_tmem, da + 2, db + 2, d_hi, idesc, 1u);
-            umma_lo_w<MK>(lead, d_tmem, da + 4, db + 4, d_hi, idesc, 1u);
-            umma_lo_w<MK>(lead, d_tmem, da + 6, db + 6, d_hi, idesc, 1u);
-            if (kLimbSum) {
-              umma_lo_w<MK>(lead, d_tmem, da, db + lo_off, d_hi, idesc, 1u);
-              umma_lo_w<MK>(lead, d_tmem, da + 2, db + lo_off + 2, d_hi, idesc, 1u);
-              umma_lo_w<MK>(lead, d_tmem, da + 4, db + lo_off + 4, d_hi, idesc, 1u);
-              umma_lo_w<MK>(lead, d_tmem, da + 6, db + lo_off + 6, d_hi, idesc, 1u);
-            }
-            if (KIND == 4) {  // weights' residue x activations' value
-              umma_lo_w<MK>(lead, d_tmem, da + wlo_off, db, d_hi, idesc, 1u);
-              umma_lo_w<MK>(lead, d_tmem, da + wlo_off + 2, db + 2, d_hi, idesc, 1u);
-              umma_lo_w<MK>(lead, d_tmem, da + wlo_off + 4, db + 4, d_hi, idesc, 1u);
-              umma_lo_w<MK>(lead, d_tmem, da + wlo_off + 6, db + 6, d_hi, idesc, 1u);
+#pragma unroll
+            for (int sub = 0; sub < kSub; sub++) {
+              const uint32_t dw = da + (uint32_t)sub * (kPTileBytes >> 4), db = da + q_off + (uint32_t)sub * (q_bytes >> 4);
+              umma_lo_w<MK>(lead, d_tmem, dw, db, d_hi, idesc, acc);  // 4 x 32 bytes of K per chunk
+              acc = 1u;
+              umma_lo_w<MK>(lead, d_tmem, dw + 2, db + 2, d_hi, idesc, 1u);
+              umma_lo_w<MK>(lead, d_tmem, dw + 4, db + 4, d_hi, idesc, 1u);
+              umma_lo_w<MK>(lead, d_tmem, dw + 6, db + 6, d_hi, idesc, 1u);
+              if (kLimbSum) {
+                umma_lo_w<MK>(lead, d_tmem, dw, db + lo_off, d_hi, idesc, 1u);
+                umma_lo_w<MK>(lead, d_tmem, dw + 2, db + lo_off + 2, d_hi, idesc, 1u);
+                umma_lo_w<MK>(lead, d_tmem, dw + 4, db + lo_off + 4, d_hi, idesc, 1u);
+                umma_lo_w<MK>(lead, d_tmem, dw + 6, db + lo_off + 6, d_hi, idesc, 1u);
+              }
+              if (KIND == 4) {  // weights' residue x activations' value
+                umma_lo_w<MK>(lead, d_tmem, dw + wlo_off, db, d_hi, idesc, 1u);
+                umma_lo_w<MK>(lead, d_tmem, dw + wlo_off + 2, db + 2, d_hi, idesc, 1u);
+                umma_lo_w<MK>(lead, d_tmem, dw + wlo_off + 4, db + 4, d_hi, idesc, 1u);
+                umma_lo_w<MK>(lead, d_tmem, dw + wlo_off + 6, db + 6, d_hi, idesc, 1u);
+              }
             }
             umma_commit_w(lead, fb + eoff);  // frees the slot when these MMAs have read it
             fb += 8u;
@@ -807,7 +819,13 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
           if (ok) umma_commit_w(lead, acc_full(buf));  // this tile's accumulators are complete
         }
       };
-      if (p.limb_sum) run(std::true_type{}); else run(std::false_type{});
+      using One = std::integral_constant<int, 1>;
+      using Two = std::integral_constant<int, 2>;
+      if (kStep && step == 2) {
+        if (p.limb_sum) run(std::true_type{}, Two{}); else run(std::false_type{}, Two{});
+      } else {
+        if (p.limb_sum) run(std::true_type{}, One{}); else run(std::false_type{}, One{});
+      }
     }
     __syncwarp();
   } else if (KIND == 5 && warp >= 2 + kEpiWarps && (warp & 2) == 0) {
@@ -1723,7 +1741,7 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
       while (best_mt > 16 && ceil_div(M, best_mt - 16) == ceil_div(M, best_mt)) best_mt -= 16;  // same tiling, less padding
       for (int sp = 2; sp <= 8 && best_mt <= 64; sp *= 2) {
         if ((long long)p.tiles_n * ceil_div(M, best_mt) * sp > ctx->sm_count || p.num_kb / sp < 4) break;
-        best_s = sp;
+        if ((sp - 1) * ceil_div(p.num_kb, sp) < p.num_kb) best_s = sp;  // (33 chunks by 8: the last CTA would have nothing to sum)
       }
     }
     const int min_s = best_s;
@@ -1807,9 +1825,22 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
   const size_t slab_bytes = slab_bytes_for(p.nslab);
   const size_t tail_bytes = tail_fixed + slab_bytes;
   int stages = (int)((227 * 1024 - tail_bytes) / stage_bytes);
+  // Two K chunks per ring stage: one weight load (a tile's consecutive chunks lie back to back) and one activation load
+  // (both chunks, all digit planes) where there were two and two to six.  A copy-engine thread issues a load every ~150 ns
+  // whatever its size, which is what a small tile's K loop runs at; against that the first chunk arrives later.  So the
+  // int8 form always (its planes are separate loads otherwise) and the f16 form on long K, where the chunks pair up evenly
+  // and three such stages fit.  Measured, us, one chunk -> two: int8 512 x 4096 x 1024 17.1 -> 15.1, 100 x 4096 x 1024 13.3
+  // -> 11.0, 16 x 2048 x 2048 8.4 -> 7.1; f16 804 x 4096 x 1024 13.7 -> 13.0, but 300 x 1024 x 4096 7.15 -> 7.66 and, with
+  // residue planes, 64 x 5120 x 1280 10.3 -> 10.7.
+  p.step = 1;
+  if ((KIND == 1 || (KIND == 0 && limbs == 1 && p.kb_per_split >= 32)) && !pair && p.batches == 1 && ep.n_peers == 0 && !(p.num_kb & 1) &&
+      !(p.kb_per_split & 1) && stages >= 6 && ctx->tc_wide_stages) {
+    p.step = 2;
+    stages /= 2;
+  }
   if (stages > 12) stages = 12;
   const int kb_per_cta = p.kb_per_split * ceil_div(num_tiles, p.splitk > 1 ? num_tiles : (pair ? ctx->sm_count / 2 : ctx->sm_count));
-  if (stages > kb_per_cta) stages = kb_per_cta;
+  if (stages > kb_per_cta / p.step) stages = kb_per_cta / p.step;
   if (stages < 1) stages = 1;
   p.stages = stages;
   p.raw_i32 = raw_i32 ? 1 : 0;
@@ -1824,7 +1855,7 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
   p.wait_limit = ctx->wait_limit;
   p.withhold_kb = ctx->tc_withhold_chunk;
   ctx->tc_withhold_chunk = -1;  // one launch only
-  const size_t smem = stage_bytes * stages + tail_bytes;
+  const size_t smem = stage_bytes * p.step * stages + tail_bytes;
 
   CUtensorMap map_w, map_a;
   // weights: rows of 128 bytes, (tiles_n * num_kb * 128) of them, boxes of 128 rows
@@ -1835,10 +1866,13 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
                   // engine as 16 rows of 256 bytes (as 128 rows of 32 bytes it cost the engine ~0.5 us per tile)
     FA_TRY(tc::make_tmap_bytes2d(ctx, &map_w, w_packed, 256, (uint64_t)p.tiles_n * p.num_kb * 16, 256, 16));
   else
-    FA_TRY(tc::make_tmap_rows128(ctx, &map_w, w_packed, elem, (KIND == 4 ? 2 : 1) * w_batches * p.tiles_n * p.num_kb * 128, 0, 128));
+    FA_TRY(tc::make_tmap_rows128(ctx, &map_w, w_packed, elem, (KIND == 4 ? 2 : 1) * w_batches * p.tiles_n * p.num_kb * 128, 0, 128 * p.step));
   // activations: [limbs * num_kb] slabs of M rows of 128 bytes, boxes of MT rows (rows >= M read as zero)
-  FA_TRY(tc::make_tmap_rows128(ctx, &map_a, a_packed, elem, (uint64_t)M,
-                               (uint64_t)(p.a_shared ? 1 : p.batches) * limbs * p.num_kb, (uint32_t)(pair ? p.MT / 2 : p.MT)));
+  if (p.step == 2)
+    FA_TRY(tc::make_tmap_planes128(ctx, &map_a, a_packed, elem, (uint64_t)M, (uint64_t)limbs, (uint64_t)p.num_kb, (uint32_t)p.MT, 2));
+  else
+    FA_TRY(tc::make_tmap_rows128(ctx, &map_a, a_packed, elem, (uint64_t)M, (uint64_t)(p.a_shared ? 1 : p.batches) * limbs * p.num_kb,
+                                 (uint32_t)(pair ? p.MT / 2 : p.MT)));
   CUtensorMap map_o = map_w, map_o16 = map_w;  // placeholders when unused (never dereferenced then)
   if (p.tma_out) {
     if (!p.skip_f32) FA_TRY(tc::make_tmap_out_f32(ctx, &map_o, (const float *)out, (uint64_t)M, (uint64_t)N, (uint64_t)p.ldc));
@@ -1896,6 +1930,25 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
 
 // Tensor of 128-byte rows: `slabs` == 0 gives a 2-d map [rows][128 B]; otherwise a 3-d map
 // [slabs][rows][128 B] with slabs stored back to back.  Boxes are box_rows x 128 bytes, swizzled.
+// [planes][slabs][rows][128 B] read as boxes of box_slabs x all planes x box_rows rows: in shared memory a slab's planes lie
+// back to back, then the next slab's.
+int tc::make_tmap_planes128(fa_ctx *ctx, CUtensorMap *out, const void *base, int elem_bytes, uint64_t rows, uint64_t planes, uint64_t slabs,
+                            uint32_t box_rows, uint32_t box_slabs) {
+  PFN_encodeTiled enc = get_encode();
+  if (!enc) return fa_fail(ctx, FA_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable in this driver");
+  FA_REQUIRE(ctx, ((uintptr_t)base & 127) == 0, "tensor-core operand %p is not 128-byte aligned", base);
+  const cuuint32_t inner = (cuuint32_t)(kRowBytes / elem_bytes);
+  cuuint64_t dims[4] = {inner, rows, planes, slabs};
+  cuuint64_t strides[3] = {(cuuint64_t)kRowBytes, slabs * rows * (cuuint64_t)kRowBytes, rows * (cuuint64_t)kRowBytes};
+  cuuint32_t box[4] = {inner, box_rows, (cuuint32_t)planes, box_slabs};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = enc(out, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void *>(base), dims,
+                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fa_fail(ctx, FA_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+  return FA_OK;
+}
+
 int tc::make_tmap_rows128(fa_ctx *ctx, CUtensorMap *out, const void *base, int elem_bytes, uint64_t rows, uint64_t slabs,
                           uint32_t box_rows) {
   PFN_encodeTiled enc = get_encode();

@@ -243,6 +243,13 @@ __device__ __forceinline__ void tma_load_3d_w(uint32_t lead, uint32_t dst, const
       "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(lead)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_4d_w(uint32_t lead, uint32_t dst, const CUtensorMap *map, int x, int y, int z, int w, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+      "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}" ::"r"(dst),
+      "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w), "r"(lead)
+      : "memory");
+}
 __device__ __forceinline__ void tma_load_2d_pair_w(uint32_t lead, uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
@@ -353,6 +360,8 @@ __host__ __device__ constexpr uint32_t make_idesc(int kind, int M, int N) {
 // Tensor of 128-byte rows: slabs == 0 gives a 2-d map [rows][128 B], otherwise a 3-d map
 // [slabs][rows][128 B] (slabs back to back).  Boxes are box_rows x 128 bytes with the 128-byte
 // swizzle; rows past the end read as zero, so a ragged M needs no special casing in the kernels.
+int make_tmap_planes128(fa_ctx *ctx, CUtensorMap *out, const void *base, int elem_bytes, uint64_t rows, uint64_t planes, uint64_t slabs,
+                        uint32_t box_rows, uint32_t box_slabs);
 int make_tmap_rows128(fa_ctx *ctx, CUtensorMap *out, const void *base, int elem_bytes, uint64_t rows, uint64_t slabs,
                       uint32_t box_rows);
 int make_tmap_bytes2d(fa_ctx *ctx, CUtensorMap *out, const void *base, uint64_t row_bytes, uint64_t rows,

@@ -1,0 +1,79 @@
+"""Products whose tiles fit one wave of the SMs: the choice of tile height and K split, ring stages of two K chunks, and the
+vector form of the int8 digit pass, at the edges of what each takes."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+# two K chunks per ring stage against one: f16, f16 with residue planes, int8 digits; even and odd chunk counts, K splits,
+# several tiles per CTA, a remainder of rows and columns
+@pytest.mark.parametrize("kind,M,K,N", [("f16", 804, 1024, 1024), ("f16", 300, 4096, 1024), ("f16", 130, 192, 300), ("f16", 70, 128, 64),
+                                        ("f16", 937, 4096, 1024), ("f16", 65, 4096, 6400), ("f16", 47, 1024, 1024), ("f16", 33, 4096, 1000),
+                                        ("i8", 512, 1024, 4096), ("i8", 100, 4096, 1024), ("i8", 17, 256, 260), ("i8", 300, 1280, 520)])
+def test_wide_stages_bit_for_bit(ctx, kind, M, K, N):
+    rng = np.random.default_rng(M + N)
+    a = ctx.upload(rng.standard_normal((M, K)).astype(np.float32), M, K)
+    add = ctx.upload(rng.standard_normal((M, N)).astype(np.float32), M, N)
+    if kind == "f16":
+        w = (ctx.uploadF16((rng.standard_normal((K, N)) / np.sqrt(K)).astype(np.float32), K, N),)
+    else:
+        w = (ctx.uploadBytes(rng.integers(-127, 128, (K, N), dtype=np.int8).view(np.uint8).reshape(-1)),
+             ctx.upload(np.full(N, 0.01, np.float32), 1, N), N, K)
+    outs = []
+    try:
+        for wide in (1, 0):
+            ctx.setOption("tc_wide_stages", wide)
+            outs.append([ctx.download(ctx.linearStep(a, *w, act="silu")), ctx.download(ctx.linearStep(a, *w, add=add))])
+    finally:
+        ctx.setOption("tc_wide_stages", 1)
+    assert np.array_equal(outs[0][0], outs[1][0]) and np.array_equal(outs[0][1], outs[1][1])
+
+
+# f32 weights (residue planes, sums of 2^-20 terms), int8 weights with three digits (2^-22 of the row maximum): heights and
+# splits chosen on both sides of 64 and 128 rows, K chunks that do not divide by the split, one row and a remainder
+@pytest.mark.parametrize("int8", [False, True])
+@pytest.mark.parametrize("M,K,N", [(300, 4096, 1024), (300, 2080, 1024), (100, 4096, 1000), (40, 2112, 2048), (129, 1056, 260), (17, 4100, 512),
+                                   (600, 2048, 1024)])
+def test_tile_and_split_choices(ctx, M, K, N, int8):
+    rng = np.random.default_rng(M + K)
+    a = rng.standard_normal((M, K)).astype(np.float32)
+    add = rng.standard_normal((M, N)).astype(np.float32)
+    ctx.setOption("int8_limbs", 3)
+    try:
+        if int8:
+            q = rng.integers(-127, 128, (K, N), dtype=np.int8)
+            sc = (rng.uniform(0.2, 1.0, N) / (73.3 * np.sqrt(K))).astype(np.float32)
+            got = ctx.linearStep(ctx.upload(a, M, K), ctx.uploadBytes(q.view(np.uint8).reshape(-1)), ctx.upload(sc, 1, N), N, K,
+                                 add=ctx.upload(add, M, N))
+            want = a.astype(np.float64) @ (q * sc.astype(np.float64)) + add
+        else:
+            w = (rng.standard_normal((K, N)) / np.sqrt(K)).astype(np.float32)
+            got = ctx.matmul(ctx.upload(a, M, K), ctx.upload(w, K, N), add=ctx.upload(add, M, N))
+            want = a.astype(np.float64) @ w.astype(np.float64) + add
+        got = ctx.download(got).reshape(M, N)
+    finally:
+        ctx.setOption("int8_limbs", 2)
+    # results of order 1; the tensor core's accumulator drops at most 2^-22 of the sum per step of K / 8 to K / 32 steps
+    assert np.abs(got - want).max() < 2e-4
+
+
+@pytest.mark.parametrize("K", [68, 1024, 1028, 2048, 4092, 8192, 8196, 1027])
+def test_digit_pass_of_whole_quads(ctx, K):
+    """Quads in registers (K % 4 == 0, up to 8192) and the general form beside it.  Three digits carry a row to 2^-22 of its
+    maximum: over the largest |a| ~ 4.5, |w| <= 127 and sqrt(K) growth the sum is off by less than 1e-6 of K."""
+    rng = np.random.default_rng(K)
+    M, N = 9, 128
+    a = rng.standard_normal((M, K)).astype(np.float32)
+    a[3] = 0
+    q = rng.integers(-127, 128, (K, N), dtype=np.int8)
+    ctx.setOption("int8_limbs", 3)
+    ctx.setOption("gemv_rows", 0)
+    try:
+        got = ctx.download(ctx.matmulInt8(ctx.upload(a, M, K), ctx.uploadBytes(q.view(np.uint8).reshape(-1)),
+                                          ctx.upload(np.full(N, 0.01, np.float32), 1, N), N, K)).reshape(M, N)
+    finally:
+        ctx.setOption("int8_limbs", 2)
+        ctx.setOption("gemv_rows", 4)
+    assert np.abs(got - 0.01 * (a.astype(np.float64) @ q)).max() < 1e-6 * K
+    assert not got[3].any()
