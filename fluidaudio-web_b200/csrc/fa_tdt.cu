@@ -63,10 +63,10 @@ __device__ __forceinline__ float t_tanhf(float x) {
   return __fdiv_rn(__fsub_rn(e, 1.0f), __fadd_rn(e, 1.0f));
 }
 
-// State vectors of the prediction network live in "chunk-transposed" form: windows in chunks of 32, element n of
-// window w at ((w / 32) * HID + n) * 32 + w % 32, so that the 32 windows' values of one n are one 128-byte line (what
-// k_tdt_rows streams).  Rows past W in the last chunk stay zero.
-__device__ __forceinline__ size_t t_idx(int w, int n) { return ((size_t)(w >> 5) * HID + n) * 32 + (w & 31); }
+// State vectors of the prediction network live in "chunk-transposed" form: windows in chunks of R = 32 (8 for at most 8
+// windows, lr = log2 R), element n of window w at ((w / R) * HID + n) * R + w % R, so that the windows' values of one n
+// are one contiguous run (what k_tdt_rows streams).  Rows past W in the last chunk stay zero.
+__device__ __forceinline__ size_t t_idx(int w, int n, int lr) { return ((((size_t)(w >> lr) * HID + n) << lr)) + (w & ((1 << lr) - 1)); }
 
 // J[w][n] = relu(proj[w*T + t_w][n] + predproj[w][n]) * scale[n]; finished windows produce zeros.
 __global__ void __launch_bounds__(256) k_tdt_joint_in(const float *__restrict__ proj, const int *__restrict__ t, int T,
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(256) k_tdt_joint_digits(const float *__restric
 // thread's eight logits, the durations, the bookkeeping words, the candidate state), so that the block pays one
 // memory latency for them, not one per loop trip.
 constexpr int kPickThreads = 1024;
-__global__ void __launch_bounds__(kPickThreads) k_tdt_pick(const float *__restrict__ logits, int ld, int T, int cap, int *__restrict__ t,
+__global__ void __launch_bounds__(kPickThreads) k_tdt_pick(const float *__restrict__ logits, int ld, int T, int cap, int lr, int *__restrict__ t,
                                                            int *__restrict__ emitted, int *__restrict__ last_tok, int *__restrict__ counts,
                                                            int *__restrict__ ids, int *__restrict__ frames,
                                                            float *__restrict__ h0t, const float *__restrict__ nh0t,
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kPickThreads) k_tdt_pick(const float *__restri
   }
   float p_h0 = 0.0f, p_h1 = 0.0f, p_c0 = 0.0f, p_c1 = 0.0f;
   if (tid < HID) {
-    p_h0 = nh0t[t_idx(w, tid)], p_h1 = nh1t[t_idx(w, tid)];
+    p_h0 = nh0t[t_idx(w, tid, lr)], p_h1 = nh1t[t_idx(w, tid, lr)];
     p_c0 = nc0[(size_t)w * HID + tid], p_c1 = nc1[(size_t)w * HID + tid];
   }
   float bv = -INFINITY;
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kPickThreads) k_tdt_pick(const float *__restri
   }
   __syncthreads();
   if (s_tok != BLANK && tid < HID) {  // commit_state: H = NH, C = NC (layer 0 finds the new token through last_tok)
-    const size_t i = t_idx(w, tid);
+    const size_t i = t_idx(w, tid, lr);
     h0t[i] = p_h0;
     h1t[i] = p_h1;
     c0[(size_t)w * HID + tid] = p_c0;
@@ -241,12 +241,21 @@ __global__ void __launch_bounds__(kPickThreads) k_tdt_pick(const float *__restri
 // lane, one mbarrier per stage), so that no thread waits on a global load.  A lane holds an 8-row x 10-column
 // accumulator tile for every fourth k of the slice (see the loop); the four k-quarters of a warp meet by shuffles
 // and the 16 warps in shared memory, both in a fixed order.
-constexpr int kRowsWarps = 16, kRowsThreads = kRowsWarps * 32, kRowsCols = 20, kRowsKS = 8, kRowsNS = 3, kRowsAhead = 2;
-constexpr int kRowsStageBytes = kRowsKS * (128 + kRowsCols * 4);                       // 1664
-constexpr int kRowsRingBytes = kRowsWarps * kRowsNS * kRowsStageBytes;                 // 79872
-constexpr int kRowsRedBytes = kRowsWarps * 32 * kRowsCols * 4;                         // 40960
-constexpr int kRowsZBytes = (32 + 1) * kRowsCols * 4;  // the block's sums, then one row for the projection's bias
-constexpr int kRowsSmem = kRowsRingBytes + kRowsRedBytes + kRowsZBytes + kRowsWarps * kRowsNS * 8;
+//
+// Up to 8 windows take chunks of R = 8: the tile of 32 rows spends three quarters of its multiply-adds, which pace it, and
+// of its activation bytes on padding.  A lane then holds 4 rows x 10 columns for every eighth k, and the ring is deep
+// enough to ask for all of layer 0's weights before the launch waits for its predecessor.  Measured, one
+// window, step by step in a decode: layer 1 9.2 -> 6.4 us, projection 5.3 -> 3.0 us, layer 0 7.0 -> 5.8 us.
+constexpr int kRowsWarps = 16, kRowsThreads = kRowsWarps * 32, kRowsCols = 20, kRowsKS = 8;
+template <int R>
+struct RowsCfg {
+  static constexpr int kNS = R == 8 ? 6 : 3, kAhead = kNS - 1;
+  static constexpr int kStageBytes = kRowsKS * (R + kRowsCols) * 4;        // 1664, 896
+  static constexpr int kRingBytes = kRowsWarps * kNS * kStageBytes;        // 79872, 86016
+  static constexpr int kRedBytes = kRowsWarps * R * kRowsCols * 4;         // 40960, 10240
+  static constexpr int kZBytes = (R + 1) * kRowsCols * 4;  // the block's sums, then one row for the projection's bias
+  static constexpr int kSmem = kRingBytes + kRedBytes + kZBytes + kRowsWarps * kNS * 8;
+};
 
 struct RowsParams {
   const float *xa, *xb;  // activations for k < 640 and k >= 640, chunk-transposed
@@ -288,9 +297,13 @@ __device__ __forceinline__ void unpack_f32x2(uint64_t v, float &lo, float &hi) {
 // MODE 0: the projection (K = 640, bias, row-major result).  MODE 1: an LSTM layer over [input | hidden] (K = 1280).
 // MODE 2: an LSTM layer whose input is an embedding row: K = 640 over the hidden state only, the input half of the
 // gates (and the bias) comes from a table indexed by each window's last token.
-template <int MODE>
+template <int MODE, int R>
 __global__ void __launch_bounds__(kRowsThreads, 1) k_tdt_rows(const RowsParams p) {
+  using Cfg = RowsCfg<R>;
   constexpr bool LSTM = MODE != 0;
+  constexpr int kRowsNS = Cfg::kNS, kRowsAhead = Cfg::kAhead, kRowsStageBytes = Cfg::kStageBytes, kRowsRingBytes = Cfg::kRingBytes,
+                kRowsRedBytes = Cfg::kRedBytes, kRowsZBytes = Cfg::kZBytes, kLr = R == 8 ? 3 : 5;
+  static_assert(R == 8 || R == 32, "lane layouts below");
   constexpr int K = MODE == 1 ? 2 * HID : HID, KPER = K / kRowsWarps, NLOAD = KPER / kRowsKS;
   static_assert(KPER % kRowsKS == 0 && HID % KPER == 0, "a warp's K slice is whole stages inside one operand");
   extern __shared__ __align__(128) uint8_t smem[];
@@ -299,9 +312,10 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_tdt_rows(const RowsParams p
   float *z = reinterpret_cast<float *>(smem + kRowsRingBytes + kRowsRedBytes);
   const uint32_t bars = tc::smem_u32(smem + kRowsRingBytes + kRowsRedBytes + kRowsZBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, blk = blockIdx.x, chunk = blockIdx.y;
-  const int ch = lane & 1, rq = (lane >> 1) & 3, kq = lane >> 3;  // gate pair, row octet, k quarter
+  // R = 32: gate pair, row octet, k quarter; R = 8: gate pair, row quad, k eighth
+  const int ch = lane & 1, rq = R == 32 ? (lane >> 1) & 3 : lane >> 4, kq = R == 32 ? lane >> 3 : (lane >> 1) & 7;
   const int k0 = warp * KPER;
-  const float *xsrc = (k0 < HID ? p.xa + ((size_t)chunk * HID + k0) * 32 : p.xb + ((size_t)chunk * HID + (k0 - HID)) * 32);
+  const float *xsrc = (k0 < HID ? p.xa + ((size_t)chunk * HID + k0) * R : p.xb + ((size_t)chunk * HID + (k0 - HID)) * R);
   const float *wsrc = p.wt + ((size_t)blk * K + k0) * kRowsCols;
   uint8_t *my = ring + (size_t)warp * kRowsNS * kRowsStageBytes;
   const uint32_t my_u = tc::smem_u32(my), my_bar = bars + warp * kRowsNS * 8;
@@ -313,8 +327,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_tdt_rows(const RowsParams p
     const uint32_t bar = my_bar + s * 8, dst = my_u + s * kRowsStageBytes;
     if (what & 1) tc::mbar_expect_tx(bar, kRowsStageBytes);
     if (it == wh) return;
-    if (what & 1) bulk_g2s(dst + kRowsKS * 128, wsrc + (size_t)it * kRowsKS * kRowsCols, kRowsKS * kRowsCols * 4, bar);
-    if (what & 2) bulk_g2s(dst, xsrc + (size_t)it * kRowsKS * 32, kRowsKS * 128, bar);
+    if (what & 1) bulk_g2s(dst + kRowsKS * R * 4, wsrc + (size_t)it * kRowsKS * kRowsCols, kRowsKS * kRowsCols * 4, bar);
+    if (what & 2) bulk_g2s(dst, xsrc + (size_t)it * kRowsKS * R, kRowsKS * R * 4, bar);
   };
   constexpr int kFirst = NLOAD < kRowsAhead ? NLOAD : kRowsAhead;
   if (lane == 0) {
@@ -331,8 +345,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_tdt_rows(const RowsParams p
   // what the epilogue needs from global memory, fetched under the K loop
   float e_c = 0.0f, e_b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   if (LSTM) {
-    if (threadIdx.x < 32 * 5) {
-      const int unit = blk * 5 + (threadIdx.x >> 5), w = chunk * 32 + (threadIdx.x & 31);
+    if (threadIdx.x < R * 5) {
+      const int unit = blk * 5 + (threadIdx.x >> kLr), w = chunk * R + (threadIdx.x & (R - 1));
       if (w < p.W) e_c = p.c[(size_t)w * HID + unit];
       if (MODE == 2) {
         if (w < p.W) {
@@ -356,9 +370,10 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_tdt_rows(const RowsParams p
   // halves of the loads as they come, an activation is duplicated into both halves by one move; half the issue
   // slots for the same arithmetic, each lane of a pair rounded exactly like a scalar FFMA.
   // Column pairs: (A0,A1) (A2,A3) (B0,B1) (B2,B3) (A4,B4) for the lane's two gates A, B and units 0..4.
-  uint64_t acc2[8][5];
+  constexpr int RL = R == 32 ? 8 : 4, KL = R == 32 ? 4 : 8;  // rows of a lane, k positions of a warp
+  uint64_t acc2[RL][5];
 #pragma unroll
-  for (int r = 0; r < 8; r++)
+  for (int r = 0; r < RL; r++)
 #pragma unroll
     for (int c = 0; c < 5; c++) acc2[r][c] = 0ull;
   bool ok = true;
@@ -374,19 +389,23 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_tdt_rows(const RowsParams p
       ok = false;
       break;
     }
-    const float4 *xs = reinterpret_cast<const float4 *>(my + s * kRowsStageBytes) + rq * 2;
-    const float *ws = reinterpret_cast<const float *>(my + s * kRowsStageBytes + kRowsKS * 128);
+    const float4 *xs = reinterpret_cast<const float4 *>(my + s * kRowsStageBytes) + rq * (RL / 4);
+    const float *ws = reinterpret_cast<const float *>(my + s * kRowsStageBytes + kRowsKS * R * 4);
 #pragma unroll
-    for (int j = 0; j < kRowsKS / 4; j++) {
-      const int kk = kq + 4 * j;
-      const float4 xa = xs[kk * 8], xb = xs[kk * 8 + 1];
+    for (int j = 0; j < kRowsKS / KL; j++) {
+      const int kk = kq + KL * j;
+      float xr[RL];
+#pragma unroll
+      for (int r = 0; r < RL; r += 4) {
+        const float4 v = xs[kk * (R / 4) + r / 4];
+        xr[r] = v.x, xr[r + 1] = v.y, xr[r + 2] = v.z, xr[r + 3] = v.w;
+      }
       const ulonglong2 wa = *reinterpret_cast<const ulonglong2 *>(ws + kk * kRowsCols + ch * 8);
       const ulonglong2 wb = *reinterpret_cast<const ulonglong2 *>(ws + kk * kRowsCols + ch * 8 + 4);
       const uint64_t wc = *reinterpret_cast<const uint64_t *>(ws + kk * kRowsCols + 16 + ch * 2);
-      const float xr[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
       const uint64_t wp[5] = {wa.x, wa.y, wb.x, wb.y, wc};
 #pragma unroll
-      for (int r = 0; r < 8; r++) {
+      for (int r = 0; r < RL; r++) {
         const uint64_t xx = dup_f32x2(xr[r]);
 #pragma unroll
         for (int c = 0; c < 5; c++) acc2[r][c] = ffma2(xx, wp[c], acc2[r][c]);
@@ -394,9 +413,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_tdt_rows(const RowsParams p
     }
     if (++s == kRowsNS) { s = 0; ph ^= 1u; }
   }
-  float acc[8][10];
+  float acc[RL][10];
 #pragma unroll
-  for (int r = 0; r < 8; r++) {
+  for (int r = 0; r < RL; r++) {
     unpack_f32x2(acc2[r][0], acc[r][0], acc[r][1]);
     unpack_f32x2(acc2[r][1], acc[r][2], acc[r][3]);
     unpack_f32x2(acc2[r][2], acc[r][5], acc[r][6]);
@@ -407,44 +426,46 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_tdt_rows(const RowsParams p
     p.status[1] = (int)blockIdx.x;
     p.status[2] = warp;
   }
-  // The four k-quarters of a warp meet by two exchange steps that halve what a lane holds: lanes 16 apart split the
-  // rows (the lower lane keeps rows 0..3 of its eight), lanes 8 apart split the two gates.  A lane ends with 4 rows x
-  // 5 units of one gate, summed over the warp's whole K slice.
-  const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0;
-  float a1[4][10];
+  // The k parts of a warp meet by exchange steps that halve what a lane holds.  R = 32: lanes 16 apart split the rows (the
+  // lower lane keeps rows 0..3 of its eight), lanes 8 apart split the two gates; a lane ends with 4 rows x 5 units of one
+  // gate.  R = 8: lanes 2 and 4 apart split the rows, lanes 8 apart the two gates; a lane ends with one row x 5 units.
+  // Either way summed over the warp's whole K slice, as partial sums red[warp][row * 5 + unit][lane].
+  auto halve = [](bool upper, float lo, float hi, int mask) {
+    return __fadd_rn(upper ? hi : lo, __shfl_xor_sync(0xffffffffu, upper ? lo : hi, mask));
+  };
+  const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0, b2 = (lane & 4) != 0, b1 = (lane & 2) != 0;
+  constexpr int RR = R == 32 ? 4 : 1;  // rows a lane ends with
+  float a1[RR][10];
+  if constexpr (R == 32) {
 #pragma unroll
-  for (int r = 0; r < 4; r++)
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int c = 0; c < 10; c++) a1[r][c] = halve(b4, acc[r][c], acc[r + 4][c], 16);
+  } else {
 #pragma unroll
     for (int c = 0; c < 10; c++) {
-      const float lo = acc[r][c], hi = acc[r + 4][c];
-      a1[r][c] = __fadd_rn(b4 ? hi : lo, __shfl_xor_sync(0xffffffffu, b4 ? lo : hi, 16));
+      const float u0 = halve(b1, acc[0][c], acc[2][c], 2), u1 = halve(b1, acc[1][c], acc[3][c], 2);
+      a1[0][c] = halve(b2, u0, u1, 4);
     }
-  float a2[4][5];
+  }
 #pragma unroll
-  for (int r = 0; r < 4; r++)
+  for (int r = 0; r < RR; r++)
 #pragma unroll
-    for (int u = 0; u < 5; u++) {
-      const float lo = a1[r][u], hi = a1[r][u + 5];
-      a2[r][u] = __fadd_rn(b3 ? hi : lo, __shfl_xor_sync(0xffffffffu, b3 ? lo : hi, 8));
-    }
-  // partial sums: red[warp][r*5+u][lane]
-#pragma unroll
-  for (int r = 0; r < 4; r++)
-#pragma unroll
-    for (int u = 0; u < 5; u++) red[(warp * 20 + r * 5 + u) * 32 + lane] = a2[r][u];
+    for (int u = 0; u < 5; u++) red[(warp * RR * 5 + r * 5 + u) * 32 + lane] = halve(b3, a1[r][u], a1[r][u + 5], 8);
   __syncthreads();
-  for (int i = threadIdx.x; i < 32 * kRowsCols; i += kRowsThreads) {
+  for (int i = threadIdx.x; i < R * kRowsCols; i += kRowsThreads) {
     float sum = red[i];
 #pragma unroll
-    for (int w = 1; w < kRowsWarps; w++) sum = __fadd_rn(sum, red[w * 32 * kRowsCols + i]);
-    const int j = i >> 5, l = i & 31;  // j = r*5+u; l = lane: bit 0 gate pair, bits 1-2 row octet, bit 3 gate, bit 4 row half
-    const int row = ((l >> 1) & 3) * 8 + (l >> 4) * 4 + j / 5, col = ((l & 1) * 2 + ((l >> 3) & 1)) * 5 + j % 5;
+    for (int w = 1; w < kRowsWarps; w++) sum = __fadd_rn(sum, red[w * R * kRowsCols + i]);
+    const int j = i >> 5, l = i & 31;  // j = row * 5 + unit of the lane; l = lane
+    const int row = R == 32 ? ((l >> 1) & 3) * 8 + (l >> 4) * 4 + j / 5 : (l >> 4) * 4 + ((l >> 1) & 1) * 2 + ((l >> 2) & 1);
+    const int col = ((l & 1) * 2 + ((l >> 3) & 1)) * 5 + j % 5;
     z[row * kRowsCols + col] = sum;
   }
   __syncthreads();
   if (LSTM) {
-    if (threadIdx.x < 32 * 5) {
-      const int row = threadIdx.x & 31, u = threadIdx.x >> 5, unit = blk * 5 + u, w = chunk * 32 + row;
+    if (threadIdx.x < R * 5) {
+      const int row = threadIdx.x & (R - 1), u = threadIdx.x >> kLr, unit = blk * 5 + u, w = chunk * R + row;
       if (w < p.W) {
         const float *zr = z + row * kRowsCols;
         const float zi = __fadd_rn(zr[u], e_b[0]), zo = __fadd_rn(zr[5 + u], e_b[1]);
@@ -452,15 +473,15 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_tdt_rows(const RowsParams p
         const size_t i = (size_t)w * HID + unit;
         const float cc = __fadd_rn(__fmul_rn(t_sigmoid(zf), e_c), __fmul_rn(t_sigmoid(zi), t_tanhf(zc)));
         p.nc[i] = cc;
-        p.nht[t_idx(w, unit)] = __fmul_rn(t_sigmoid(zo), t_tanhf(cc));
+        p.nht[t_idx(w, unit, kLr)] = __fmul_rn(t_sigmoid(zo), t_tanhf(cc));
       }
     }
   } else {
-    if (threadIdx.x < kRowsCols) z[32 * kRowsCols + threadIdx.x] = e_b[0];
+    if (threadIdx.x < kRowsCols) z[R * kRowsCols + threadIdx.x] = e_b[0];
     __syncthreads();
-    for (int i = threadIdx.x; i < 32 * kRowsCols; i += kRowsThreads) {
-      const int row = i / kRowsCols, col = i - row * kRowsCols, w = chunk * 32 + row, n = blk * kRowsCols + col;
-      if (w < p.W) p.out[(size_t)w * HID + n] = __fadd_rn(z[i], z[32 * kRowsCols + col]);
+    for (int i = threadIdx.x; i < R * kRowsCols; i += kRowsThreads) {
+      const int row = i / kRowsCols, col = i - row * kRowsCols, w = chunk * R + row, n = blk * kRowsCols + col;
+      if (w < p.W) p.out[(size_t)w * HID + n] = __fadd_rn(z[i], z[R * kRowsCols + col]);
     }
   }
 }
@@ -583,7 +604,7 @@ namespace {
 
 struct TdtState {
   fa_tensor *state = nullptr;  // every recurrent vector below, one block, cleared by one memset
-  // chunk-transposed [ceil(W/32)][HID][32]: committed and candidate hidden states; [W][HID]: cell states
+  // chunk-transposed (t_idx): committed and candidate hidden states; [W][HID]: cell states
   float *h0t = nullptr, *nh0t = nullptr, *h1t = nullptr, *nh1t = nullptr, *c0 = nullptr, *c1 = nullptr, *nc0 = nullptr, *nc1 = nullptr;
   fa_tensor *predproj = nullptr, *J = nullptr;   // [W][HID]
   fa_tensor *logits = nullptr;                   // [W][LOGITS] when the joint's digit planes are written here
@@ -593,21 +614,29 @@ struct TdtState {
   size_t ints_bytes = 0;
 };
 
+// Windows per chunk of the state vectors (log2): see k_tdt_rows.
+int tdt_lr(int W) { return W <= 8 ? 3 : 5; }
+
+template <int MODE, int R>
+int tdt_rows_r(fa_ctx *ctx, const RowsParams &q, int blocks) {
+  static bool attr_set = false;
+  if (!attr_set) {
+    FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_tdt_rows<MODE, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, RowsCfg<R>::kSmem));
+    attr_set = true;
+  }
+  LaunchScope ls(ctx, MODE ? "tdt_lstm" : "tdt_pred");
+  FA_CHECK_CUDA(ctx, fa_launch_dep(ctx, k_tdt_rows<MODE, R>, dim3(blocks, ceil_div(q.W, R)), dim3(kRowsThreads), RowsCfg<R>::kSmem, q));
+  return FA_OK;
+}
+
 template <int MODE>
 int tdt_rows(fa_ctx *ctx, const RowsParams &p, int blocks, int W, int withhold) {
-  static bool attr_set[3] = {false, false, false};
-  if (!attr_set[MODE]) {
-    FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_tdt_rows<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem));
-    attr_set[MODE] = true;
-  }
   RowsParams q = p;
   q.W = W;
   q.status = ctx->dev_status;
   q.wait_limit = ctx->wait_limit;
   q.withhold = withhold;
-  LaunchScope ls(ctx, MODE ? "tdt_lstm" : "tdt_pred");
-  FA_CHECK_CUDA(ctx, fa_launch_dep(ctx, k_tdt_rows<MODE>, dim3(blocks, ceil_div(W, 32)), dim3(kRowsThreads), kRowsSmem, q));
-  return FA_OK;
+  return tdt_lr(W) == 3 ? tdt_rows_r<MODE, 8>(ctx, q, blocks) : tdt_rows_r<MODE, 32>(ctx, q, blocks);
 }
 
 // predict + compute_predproj for every window, from the committed state and the last token's embedding
@@ -657,7 +686,7 @@ int tdt_round(fa_ctx *ctx, fa_tdt *d, TdtState &s, const fa_tensor *proj, int W,
   const float *lg = (const float *)(logits ? logits->dptr : s.logits->dptr);
   {
     LaunchScope ls(ctx, "tdt_pick");
-    FA_CHECK_CUDA(ctx, fa_launch_dep(ctx, k_tdt_pick, dim3(W), dim3(kPickThreads), 0, lg, LOGITS, T, cap, t, emitted, last_tok, counts,
+    FA_CHECK_CUDA(ctx, fa_launch_dep(ctx, k_tdt_pick, dim3(W), dim3(kPickThreads), 0, lg, LOGITS, T, cap, tdt_lr(W), t, emitted, last_tok, counts,
                                      ids, frames, s.h0t,
                                      s.nh0t, s.h1t, s.nh1t,
                                      s.c0, s.c1, s.nc0,
@@ -687,7 +716,7 @@ extern "C" int fa_tdt_decode_proj(fa_ctx *ctx, fa_tdt *d, const fa_tensor *proj,
   ctx->int8_limbs = 3;  // f32-grade activations for the joint's int8 product: token picks follow the f32 reference
   int rc = FA_OK, rounds = 0;
   auto alloc = [&](int r, int c, fa_tensor **t) { return rc == FA_OK ? (rc = fa_alloc(ctx, r, c, t)) : rc; };
-  const int wpad = ceil_div(W, 32) * 32;
+  const int wpad = ceil_div(W, 1 << tdt_lr(W)) << tdt_lr(W);
   alloc(4 * wpad + 4 * W, HID, &s.state), alloc(W, HID, &s.predproj), alloc(W, HID, &s.J);
   const size_t n_int = (size_t)4 * W + (size_t)2 * W * cap;
   if (rc == FA_OK) rc = fa_block_acquire(ctx, n_int * 4, &s.ints, &s.ints_bytes);
