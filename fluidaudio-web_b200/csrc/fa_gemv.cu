@@ -512,29 +512,37 @@ namespace {
 // the weights stay exact.
 //
 // What bounds it: instruction issue.  A warp owns ONE quad of 32-weight blocks (16 warps x 4 blocks = the 2048 k that the
-// activation planes of 16 rows leave room for in shared memory) and walks up to G groups of 8 output columns with it:
+// activation planes of 16 rows leave room for in shared memory; on shorter slices several warps share a quad's columns) and walks up to G groups of 8 output columns with it:
 //   - a lane loads one whole block per group (16 bytes; the 4 lanes of a column read 64 consecutive bytes), all groups up
 //     front, before the launch waits for its predecessor (the payload is only ever written by an upload);
 //   - a 4 x 4 transpose between the 4 lanes of a column (4 shuffles) gives each lane word j of all four blocks, so that
 //     one mma.sync.m16n8k16 works inside ONE block and the scale can wait for its result;
 //   - a nibble pair (k, k + 4) becomes two f16 `1024 + q` with one mask, minus 1024 + zp: exact.  Which k sits in which of
-//     the instruction's slots does not matter for a sum; the activation rows lie in shared memory in the same order, a
-//     lane's 8 values of a block as one 16-byte load (row pitch = 64 mod 128 bytes: conflict-free), and are read once per
-//     block for all groups;
+//     the instruction's slots does not matter for a sum; rows r and r + 8 lie in shared memory interleaved in the same order,
+//     so that one 16-byte load IS a lane's A operand (four registers in a row: put together from two loads it cost a move per
+//     register, group and block), and are read once per block for all groups (pitch = 64 mod 128 bytes: conflict-free);
 //   - per block and group: 4 mma (value and residue plane of the activations), then 4 multiply-adds with the scale.
 // The 16 warps' sums meet in shared memory in warp order; K beyond 2048 is split over the ranks of a cluster, whose sums
 // meet in rank 0's shared memory in rank order.
-// Measured, 16 rows, recorded blocks: N = 8192, K = 2048 12.4 us and N = 2048, K = 8192 14.7 us, against 14.1 and 20.0 us (digit
-// pass included) for the f16 copy on the tensor cores, which read 33.5 MB where this reads 10.5.
+// Measured, 16 rows, recorded blocks: 13.2 us on average for K = 2048, N = 8192 and K = 8192, N = 2048, against 14.1 and 20.0 us
+// (digit pass included) for the f16 copy on the tensor cores, which read 33.5 MB where this reads 10.5.  What is left is the
+// chain of one launch: its 512 threads of 128 registers cannot start beside the block before them.
 constexpr int kMmaWarps = 16, kMmaThreads = kMmaWarps * 32;
 constexpr int kMmaSliceBlk = kMmaWarps * 4;  // 32-weight blocks per K slice
 constexpr int kMmaMaxSlices = 4;
-__host__ __device__ constexpr int mma_row_pitch(int blks) { return blks * 64 + ((blks & 1) ? 0 : 64); }
+__host__ __device__ constexpr int mma_row_pitch(int blks) { return blks * 128 + 64; }  // rows r and r + 8 together
 
 __device__ __forceinline__ void mma16816_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// The same from a zero accumulator.
+__device__ __forceinline__ void mma16816_f16_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
 }
 
 struct MmaParams {
@@ -545,6 +553,7 @@ struct MmaParams {
   float *y;
   int M, N, K, nblk, zpb;
   int slice;  // blocks per K slice (a multiple of 4, at most kMmaSliceBlk)
+  int lq;     // log2 of the quads per slice that have warps of their own (16, 8 or 4): 16 >> lq warps share a quad's columns
   int gper;   // column groups per thread block
 };
 
@@ -567,10 +576,12 @@ __global__ void __launch_bounds__(kMmaThreads, 1) k_nbits_mma(const MmaParams p)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g4 = lane >> 2, j4 = lane & 3;
   const int rank = blockIdx.y, slices = gridDim.y, b0 = rank * p.slice, nb = min(p.slice, p.nblk - b0);  // blocks of this slice
   const int pitch = mma_row_pitch(p.slice);
-  unsigned char *ap = smem;                                                     // [planes][16 rows][pitch]
-  float4 *red = (float4 *)(smem + (size_t)(HILO ? 2 : 1) * 16 * pitch);         // [16 warps][G][32]
-  float4 *cred = red + kMmaWarps * G * 32;                                      // rank 0: [2][slices][G][32]
-  const int qb = b0 + warp * 4;         // first block of the warp's quad
+  unsigned char *ap = smem;                                                     // [planes][8 row pairs][pitch]
+  float4 *red = (float4 *)(smem + (size_t)(HILO ? 2 : 1) * 8 * pitch);         // [quads][gall][32]
+  const int gw = kMmaWarps >> p.lq, gall = G * gw;                              // warps per quad, groups of a pass
+  float4 *cred = red + kMmaWarps * G * 32;                                      // rank 0: [2][slices][gall][32]
+  const int quad = warp & ((1 << p.lq) - 1), goff = (warp >> p.lq) * G;         // the warp's quad and first group of a pass
+  const int qb = b0 + quad * 4;         // first block of the quad
   const int qn = min(4, b0 + nb - qb);  // its blocks (<= 0: none)
   const int groups = p.N >> 3, gfirst = blockIdx.x * p.gper, gend = min(groups, gfirst + p.gper);
   const uint4 *bq4 = (const uint4 *)p.bq;
@@ -581,50 +592,80 @@ __global__ void __launch_bounds__(kMmaThreads, 1) k_nbits_mma(const MmaParams p)
 #pragma unroll
     for (int g = 0; g < G; g++) {
       w[g] = make_uint4(0u, 0u, 0u, 0u);
-      if (g0 + g < gend && j4 < qn) w[g] = __ldcs(bq4 + (size_t)((g0 + g) * 8 + g4) * p.nblk + qb + j4);
+      if (g0 + goff + g < gend && j4 < qn) w[g] = __ldcs(bq4 + (size_t)((g0 + goff + g) * 8 + g4) * p.nblk + qb + j4);
     }
   };
   fetch(gfirst);
   if (slices > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // every rank runs before a remote store
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  // activation rows of this K slice: 8 consecutive k of one row per step, as halves k0,k4,k1,k5,k2,k6,k3,k7; a thread
-  // requests four steps before it converts the first (every block reads all the rows: 131 KB at 16 x 2048)
+  float sc[G];     // lane: block j4 of column g4
+  unsigned z4[G];  // column g4: zero-points of the quad's blocks, a nibble each
+  auto fetch_scales = [&](int g0) {
+#pragma unroll
+    for (int g = 0; g < G; g++) {
+      sc[g] = 0.f, z4[g] = 0u;
+      if (g0 + goff + g < gend && qn > 0) {
+        const int n = (g0 + goff + g) * 8 + g4;
+        if (j4 < qn) sc[g] = __ldg(p.scales + (size_t)n * p.nblk + qb + j4);
+        const uint8_t *z = p.zp + (size_t)n * p.zpb + (qb >> 1);  // qb is a multiple of 4
+        z4[g] = __ldg(z);
+        if (qn > 2) z4[g] |= (unsigned)__ldg(z + 1) << 8;
+      }
+    }
+  };
+  fetch_scales(gfirst);  // (a kernel may have made them: not before the wait)
+
+  // activation rows of this K slice: 8 consecutive k of rows r and r + 8 per step, as the two A operands {r: k0,k4 | r+8: k0,k4 |
+  // r: k1,k5 | r+8: k1,k5} and the same of k2,k6 and k3,k7, 64 bytes apart; a thread requests two steps before it converts
+  // the first
   const bool quads = (p.K & 3) == 0;
-  for (int i0 = tid; i0 < 16 * p.slice * 4; i0 += 4 * kMmaThreads) {
-    float x[4][8];
+  const int octs = p.slice * 4;
+  for (int i0 = tid; i0 < 8 * octs; i0 += 2 * kMmaThreads) {
+    float x[2][2][8];
+    int r[2], oct[2];
 #pragma unroll
-    for (int s = 0; s < 4; s++) {
-      const int i = i0 + s * kMmaThreads, m = i / (p.slice * 4), k = b0 * 32 + (i - m * p.slice * 4) * 8;
+    for (int s = 0; s < 2; s++) {
+      const int i = i0 + s * kMmaThreads;
+      r[s] = i / octs, oct[s] = i - r[s] * octs;
+      const int k = b0 * 32 + oct[s] * 8;
 #pragma unroll
-      for (int u = 0; u < 8; u++) x[s][u] = 0.f;
-      if (m < p.M) {  // (i past the end: m >= 16)
-        const float *row = p.a + (size_t)m * p.K;
-        if (quads && k + 8 <= p.K) {
-          const float4 x0 = *(const float4 *)(row + k), x1 = *(const float4 *)(row + k + 4);
-          x[s][0] = x0.x, x[s][1] = x0.y, x[s][2] = x0.z, x[s][3] = x0.w, x[s][4] = x1.x, x[s][5] = x1.y, x[s][6] = x1.z, x[s][7] = x1.w;
-        } else {
+      for (int h = 0; h < 2; h++) {
+        const int m = r[s] + 8 * h;
 #pragma unroll
-          for (int u = 0; u < 8; u++)
-            if (k + u < p.K) x[s][u] = row[k + u];
+        for (int u = 0; u < 8; u++) x[s][h][u] = 0.f;
+        if (r[s] < 8 && m < p.M) {
+          const float *row = p.a + (size_t)m * p.K;
+          if (quads && k + 8 <= p.K) {
+            const float4 x0 = *(const float4 *)(row + k), x1 = *(const float4 *)(row + k + 4);
+            x[s][h][0] = x0.x, x[s][h][1] = x0.y, x[s][h][2] = x0.z, x[s][h][3] = x0.w;
+            x[s][h][4] = x1.x, x[s][h][5] = x1.y, x[s][h][6] = x1.z, x[s][h][7] = x1.w;
+          } else {
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+              if (k + u < p.K) x[s][h][u] = row[k + u];
+          }
         }
       }
     }
 #pragma unroll
-    for (int s = 0; s < 4; s++) {
-      const int i = i0 + s * kMmaThreads, m = i / (p.slice * 4), oct = i - m * p.slice * 4;
-      if (m >= 16) break;
-      __half2 h[4];
+    for (int s = 0; s < 2; s++) {
+      if (r[s] >= 8) break;
+      __half2 hi[4][2], lo[4][2];  // [pair (k_u, k_u+4)][row r, row r + 8]
 #pragma unroll
-      for (int u = 0; u < 4; u++) h[u] = __floats2half2_rn(x[s][u], x[s][u + 4]);
-      *(uint4 *)(ap + (size_t)m * pitch + oct * 16) = *(const uint4 *)h;
-      if (HILO) {
+      for (int u = 0; u < 4; u++)
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const float2 f = __half22float2(h[u]);
-          h[u] = __floats2half2_rn(x[s][u] - f.x, x[s][u + 4] - f.y);
+        for (int h = 0; h < 2; h++) {
+          hi[u][h] = __floats2half2_rn(x[s][h][u], x[s][h][u + 4]);
+          const float2 f = __half22float2(hi[u][h]);
+          lo[u][h] = __floats2half2_rn(x[s][h][u] - f.x, x[s][h][u + 4] - f.y);
         }
-        *(uint4 *)(ap + (size_t)(16 + m) * pitch + oct * 16) = *(const uint4 *)h;
+      unsigned char *dst = ap + (size_t)r[s] * pitch + (oct[s] >> 2) * 128 + (oct[s] & 3) * 16;
+      *(uint4 *)dst = *(const uint4 *)hi[0];
+      *(uint4 *)(dst + 64) = *(const uint4 *)hi[2];
+      if (HILO) {
+        *(uint4 *)(dst + (size_t)8 * pitch) = *(const uint4 *)lo[0];
+        *(uint4 *)(dst + (size_t)8 * pitch + 64) = *(const uint4 *)lo[2];
       }
     }
   }
@@ -632,21 +673,8 @@ __global__ void __launch_bounds__(kMmaThreads, 1) k_nbits_mma(const MmaParams p)
   if (slices > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 
   int pass = 0;
-  for (int g0 = gfirst; g0 < gend; g0 += G, pass++) {
-    if (g0 > gfirst) fetch(g0);
-    float sc[G];     // lane: block j4 of column g4
-    unsigned z4[G];  // column g4: zero-points of the quad's blocks, a nibble each
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-      sc[g] = 0.f, z4[g] = 0u;
-      if (g0 + g < gend && qn > 0) {
-        const int n = (g0 + g) * 8 + g4;
-        if (j4 < qn) sc[g] = __ldg(p.scales + (size_t)n * p.nblk + qb + j4);
-        const uint8_t *z = p.zp + (size_t)n * p.zpb + (qb >> 1);  // qb is a multiple of 4
-        z4[g] = __ldg(z);
-        if (qn > 2) z4[g] |= (unsigned)__ldg(z + 1) << 8;
-      }
-    }
+  for (int g0 = gfirst; g0 < gend; g0 += gall, pass++) {
+    if (g0 > gfirst) fetch(g0), fetch_scales(g0);
     float acc[G][4];
 #pragma unroll
     for (int g = 0; g < G; g++) {
@@ -657,13 +685,13 @@ __global__ void __launch_bounds__(kMmaThreads, 1) k_nbits_mma(const MmaParams p)
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       if (i >= qn) break;  // warp-uniform
-      const unsigned char *src = ap + (size_t)g4 * pitch + (warp * 4 + i) * 64 + j4 * 16;
-      const uint4 h0 = *(const uint4 *)src, h1 = *(const uint4 *)(src + (size_t)8 * pitch);
+      const unsigned char *src = ap + (size_t)g4 * pitch + (quad * 4 + i) * 128 + j4 * 16;
+      const uint4 h0 = *(const uint4 *)src, h1 = *(const uint4 *)(src + 64);
       uint4 l0, l1;
-      if (HILO) l0 = *(const uint4 *)(src + (size_t)16 * pitch), l1 = *(const uint4 *)(src + (size_t)24 * pitch);
+      if (HILO) l0 = *(const uint4 *)(src + (size_t)8 * pitch), l1 = *(const uint4 *)(src + (size_t)8 * pitch + 64);
 #pragma unroll
       for (int g = 0; g < G; g++) {
-        if (g0 + g >= gend) break;
+        if (g0 + goff + g >= gend) break;
         const unsigned x = i == 0 ? w[g].x : (i == 1 ? w[g].y : (i == 2 ? w[g].z : w[g].w));
         const unsigned zz = 0x6400u + ((z4[g] >> (4 * i)) & 15u), z2 = zz | (zz << 16);  // 1024 + zp, twice
         uint32_t b[4];
@@ -673,12 +701,12 @@ __global__ void __launch_bounds__(kMmaThreads, 1) k_nbits_mma(const MmaParams p)
           const __half2 d = __hsub2(*(const __half2 *)&q, *(const __half2 *)&z2);
           b[u] = *(const uint32_t *)&d;
         }
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-        mma16816_f16(c, h0.x, h1.x, h0.y, h1.y, b[0], b[1]);
-        mma16816_f16(c, h0.z, h1.z, h0.w, h1.w, b[2], b[3]);
+        float c[4];
+        mma16816_f16_first(c, h0.x, h0.y, h0.z, h0.w, b[0], b[1]);
+        mma16816_f16(c, h1.x, h1.y, h1.z, h1.w, b[2], b[3]);
         if (HILO) {
-          mma16816_f16(c, l0.x, l1.x, l0.y, l1.y, b[0], b[1]);
-          mma16816_f16(c, l0.z, l1.z, l0.w, l1.w, b[2], b[3]);
+          mma16816_f16(c, l0.x, l0.y, l0.z, l0.w, b[0], b[1]);
+          mma16816_f16(c, l1.x, l1.y, l1.z, l1.w, b[2], b[3]);
         }
         const float s0 = __shfl_sync(0xffffffffu, sc[g], j4 * 8 + i), s1 = __shfl_sync(0xffffffffu, sc[g], j4 * 8 + 4 + i);
         acc[g][0] = fmaf(s0, c[0], acc[g][0]), acc[g][1] = fmaf(s1, c[1], acc[g][1]);
@@ -687,56 +715,62 @@ __global__ void __launch_bounds__(kMmaThreads, 1) k_nbits_mma(const MmaParams p)
     }
     if (pass > 0) __syncthreads();  // the sums of the pass before have been read
 #pragma unroll
-    for (int g = 0; g < G; g++) red[(warp * G + g) * 32 + lane] = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+    for (int g = 0; g < G; g++) red[(quad * gall + goff + g) * 32 + lane] = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
     __syncthreads();
-    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (tid < G * 32) {
-      t = red[tid];
-#pragma unroll
-      for (int v = 1; v < kMmaWarps; v++) {
-        const float4 o = red[v * G * 32 + tid];
+    // two buffers: a rank stores pass n + 2 only after the barrier of pass n + 1, which rank 0 reaches when it has read n
+    float4 *buf = cred + (size_t)(pass & 1) * slices * gall * 32;
+    auto store = [&](int e, const float4 &t) {  // e = group of the pass * 32 + lane of the accumulator tile
+      const int g = g0 + (e >> 5), row = (e & 31) >> 2, n = g * 8 + (e & 3) * 2;
+      if (g >= gend) return;
+      if (row < p.M) *(float2 *)(p.y + (size_t)row * p.N + n) = make_float2(t.x, t.y);
+      if (row + 8 < p.M) *(float2 *)(p.y + (size_t)(row + 8) * p.N + n) = make_float2(t.z, t.w);
+    };
+    for (int e = tid; e < gall * 32; e += kMmaThreads) {
+      float4 t = red[e];
+      for (int v = 1; v < (1 << p.lq); v++) {
+        const float4 o = red[v * gall * 32 + e];
         t.x += o.x, t.y += o.y, t.z += o.z, t.w += o.w;
+      }
+      if (slices > 1) {
+        uint32_t remote;
+        const uint32_t local = (uint32_t)__cvta_generic_to_shared(buf + rank * gall * 32 + e);
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(0));
+        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(remote), "f"(t.x), "f"(t.y), "f"(t.z), "f"(t.w) : "memory");
+      } else {
+        store(e, t);
       }
     }
     if (slices > 1) {
-      // two buffers: a rank stores pass n + 2 only after the barrier of pass n + 1, which rank 0 reaches when it has read n
-      float4 *buf = cred + (size_t)(pass & 1) * slices * G * 32;
-      if (tid < G * 32) {
-        uint32_t remote;
-        const uint32_t local = (uint32_t)__cvta_generic_to_shared(buf + rank * G * 32 + tid);
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(0));
-        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(remote), "f"(t.x), "f"(t.y), "f"(t.z), "f"(t.w) : "memory");
-      }
       asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-      if (rank == 0 && tid < G * 32) {
-        t = buf[tid];
-        for (int v = 1; v < slices; v++) {
-          const float4 o = buf[v * G * 32 + tid];
-          t.x += o.x, t.y += o.y, t.z += o.z, t.w += o.w;
+      if (rank == 0)
+        for (int e = tid; e < gall * 32; e += kMmaThreads) {
+          float4 t = buf[e];
+          for (int v = 1; v < slices; v++) {
+            const float4 o = buf[v * gall * 32 + e];
+            t.x += o.x, t.y += o.y, t.z += o.z, t.w += o.w;
+          }
+          store(e, t);
         }
-      }
-    }
-    const int g = g0 + (tid >> 5);
-    if (rank == 0 && tid < G * 32 && g < gend) {
-      const int n = g * 8 + j4 * 2;
-      if (g4 < p.M) *(float2 *)(p.y + (size_t)g4 * p.N + n) = make_float2(t.x, t.y);
-      if (g4 + 8 < p.M) *(float2 *)(p.y + (size_t)(g4 + 8) * p.N + n) = make_float2(t.z, t.w);
     }
   }
 }
 
-size_t mma_smem(bool hilo, int G, int slice, int slices) {
-  return (size_t)(hilo ? 2 : 1) * 16 * mma_row_pitch(slice) + (size_t)G * 32 * 16 * (kMmaWarps + (slices > 1 ? 2 * slices : 0));
+size_t mma_smem(bool hilo, int G, int slice, int slices, int lq) {
+  return (size_t)(hilo ? 2 : 1) * 8 * mma_row_pitch(slice) + (size_t)G * 32 * 16 * (kMmaWarps + (slices > 1 ? 2 * slices * (kMmaWarps >> lq) : 0));
 }
-// K slices (a power of two: clusters of 3 place badly) and blocks per slice, a multiple of 4
-void mma_slices(int nblk, int &slices, int &slice) {
-  for (slices = 1; slices * kMmaSliceBlk < nblk; slices *= 2) {}
+// K slices (a power of two: clusters of 3 place badly) and blocks per slice, a multiple of 4.  Four slices from K = 2048 on:
+// every block of the grid converts all rows of its K slice before it starts, so four times the columns on a quarter of K
+// cost a quarter of that for one cluster hand-over (K = 2048, N = 8192 and back, 16 rows: 129.5 us in one slice per 2048,
+// 127.6 us so, 121.1 us with whole A operands in shared memory).
+void mma_slices(int nblk, int &slices, int &slice, int &lq) {
+  slices = nblk >= kMmaSliceBlk ? kMmaMaxSlices : 1;
   slice = ceil_div(ceil_div(nblk, slices), 4) * 4;
+  lq = slice > 32 ? 4 : (slice > 16 ? 3 : 2);
 }
 
 template <bool HILO, int G>
 cudaError_t launch_mma(fa_ctx *ctx, cudaLaunchConfig_t &cfg, const MmaParams &p) {
-  cfg.dynamicSmemBytes = mma_smem(HILO, G, p.slice, (int)cfg.gridDim.y);
+  cfg.dynamicSmemBytes = mma_smem(HILO, G, p.slice, (int)cfg.gridDim.y, p.lq);
   const cudaError_t e = cudaFuncSetAttribute(k_nbits_mma<HILO, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
   return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, k_nbits_mma<HILO, G>, p);
 }
@@ -750,11 +784,12 @@ bool fa_nbits_mma_ok(int M, int N, int K, int block_size) {
 
 int fa_nbits_mma(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y, int M, int N,
                  int K, int nblk, int zpb, bool hilo) {
-  MmaParams p{a, bq, scales, zp, y, M, N, K, nblk, zpb, 0, 0};
+  MmaParams p{a, bq, scales, zp, y, M, N, K, nblk, zpb, 0, 0, 0};
   int slices;
-  mma_slices(nblk, slices, p.slice);
+  mma_slices(nblk, slices, p.slice, p.lq);
+  const int gw = kMmaWarps >> p.lq;  // warps that share a quad's columns
   // column groups per thread block: as many as leave one wave of blocks (clusters of K slices do not tile every GPC, so
-  // an eighth of the SMs is left out of the count there); walked 8, 4 or 2 at a time
+  // an eighth of the SMs is left out of the count there); walked 8, 4 or 2 at a time by each of the gw warps of a quad
   const int groups = N / 8, room = slices == 1 ? ctx->sm_count : ctx->sm_count * 7 / 8 / slices;
   p.gper = ceil_div(groups, room < 1 ? 1 : room);
   cudaLaunchConfig_t cfg{};
@@ -773,8 +808,8 @@ int fa_nbits_mma(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *sc
   cudaError_t e;
   {
     LaunchScope ls(ctx, "nbits_mma");
-    if (p.gper <= 2) e = hilo ? launch_mma<true, 2>(ctx, cfg, p) : launch_mma<false, 2>(ctx, cfg, p);
-    else if (p.gper <= 4) e = hilo ? launch_mma<true, 4>(ctx, cfg, p) : launch_mma<false, 4>(ctx, cfg, p);
+    if (p.gper <= 2 * gw) e = hilo ? launch_mma<true, 2>(ctx, cfg, p) : launch_mma<false, 2>(ctx, cfg, p);
+    else if (p.gper <= 4 * gw) e = hilo ? launch_mma<true, 4>(ctx, cfg, p) : launch_mma<false, 4>(ctx, cfg, p);
     else e = hilo ? launch_mma<true, 8>(ctx, cfg, p) : launch_mma<false, 8>(ctx, cfg, p);
   }
   if (e != cudaSuccess) return fa_fail(ctx, FA_ERR_CUDA, "launch nbits_mma: %s", cudaGetErrorString(e));

@@ -1,0 +1,34 @@
+"""int4 products of 1 to 16 rows against float64 on the exact weights (q - zp) * scale.
+
+The mma.sync form (5 rows on): rows as f16 value + residue (2^-22 of each value), exact weights, f32 sums of a block's 32 terms
+times its scale: with |a| ~ 1 and weights of norm ~1 per column the result, of order 1, is off by less than 3e-5.  The dp4a
+form (1 to 4 rows): two int8 digits, 2^-15 of the row maximum ~4 on every value: below 2e-3."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+# one block; a K slice not a multiple of four blocks; slices of 16, 20, 32, 36, 64 blocks; a last slice that is short; one
+# column group, several per warp, two passes; rows that do not fill the tile; K that ends inside a block
+@pytest.mark.parametrize("M,K,N", [(16, 32, 8), (5, 96, 16), (16, 2016, 64), (16, 2048, 8192), (7, 2080, 264), (16, 4096, 520), (9, 4128, 128),
+                                   (16, 8192, 2048), (16, 8160, 72), (11, 2560, 5128), (16, 1000, 40), (6, 2050, 48),
+                                   (1, 8192, 2048), (1, 2560, 1288), (1, 512, 2360), (3, 4096, 1100), (4, 2048, 2376)])
+def test_few_rows(ctx, M, K, N):
+    rng = np.random.default_rng(K + N)
+    nblk = (K + 31) // 32
+    a = rng.standard_normal((M, K)).astype(np.float32)
+    q = rng.integers(0, 16, (N, nblk * 32))
+    z = rng.integers(0, 16, (N, (nblk + 1) // 2 * 2))
+    sc = (rng.uniform(0.25, 1.0, (N, nblk)) / (4.6 * np.sqrt(K))).astype(np.float32)
+    w = (q.reshape(N, nblk, 32) - z[:, :nblk, None]) * sc.astype(np.float64)[:, :, None]
+    want = a.astype(np.float64) @ w.reshape(N, -1)[:, :K].T
+    packed = (q[:, 0::2] | (q[:, 1::2] << 4)).astype(np.uint8)
+    zp = (z[:, 0::2] | (z[:, 1::2] << 4)).astype(np.uint8)
+    ctx.startProfile(16)
+    got = ctx.download(ctx.matmulNBits(ctx.upload(a, M, K), ctx.uploadBytes(packed.reshape(-1)), ctx.upload(sc, 1, sc.size),
+                                       ctx.uploadBytes(zp.reshape(-1)), N)).reshape(M, N)
+    labels = [e["label"] for e in ctx.endProfile()]
+    small = N * K < 1 << 18  # little work: the any-shape kernel, exact too
+    assert small or ("nbits_mma" if M > 4 else "gemv_nbits") in labels, labels
+    assert np.abs(got - want).max() < (3e-5 if M > 4 else 2e-3) * max(1.0, np.abs(want).max() / 4)
