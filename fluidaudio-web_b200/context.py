@@ -430,23 +430,22 @@ class CudaContext:
             return _lib.Linear(q.h, scale.h, self._h_of(bias), N, K)
         return _lib.Linear(w.h, None, self._h_of(bias), w.cols, w.rows)
 
-    def decoderWeights(self, layers: Sequence[dict], lnf, logits):
-        """The weights of decoderStep.  A layer maps sqkv, so, cq, co, f1, f2 to (weights, bias) and ln1..ln3 to
-        (gamma, beta); lnf is (gamma, beta), logits the vocabulary matrix."""
-        arr = (_lib.DecoderLayer * len(layers))()
-        for d, w in zip(arr, layers):
-            for n in ("sqkv", "so", "cq", "co", "f1", "f2"):
-                setattr(d, n, self._linear_of(*w[n]))
-            for n in ("ln1", "ln2", "ln3"):
-                setattr(d, n + "_w", w[n][0].h), setattr(d, n + "_b", w[n][1].h)
-        return arr, lnf[0].h, lnf[1].h, self._linear_of(logits, None)
+    def decoderWeights(self, w: dict):
+        """One layer's weights for decoderStep: sqkv, so, cq, co, f1, f2 as (weights, bias), ln1..ln3 as (gamma, beta)."""
+        d = _lib.DecoderLayer()
+        for n in ("sqkv", "so", "cq", "co", "f1", "f2"):
+            setattr(d, n, self._linear_of(*w[n]))
+        for n in ("ln1", "ln2", "ln3"):
+            setattr(d, n + "_w", w[n][0].h), setattr(d, n + "_b", w[n][1].h)
+        return d
 
-    def decoderStep(self, weights, x, crossK, crossV, selfK, selfV, n: int, NH: int, HD: int) -> Tensor:
-        """Optional member: one token of S streams through all layers, x [S, D] -> logits (see fa_decoder_step)."""
-        arr, g, b, logits = weights
-        handles = lambda ts: (C.c_void_p * len(arr))(*[t.h for t in ts])  # noqa: E731
-        return self._op(self._lib.fa_decoder_step, arr, len(arr), x.h, handles(crossK), handles(crossV), handles(selfK), handles(selfV),
-                        n, NH, HD, g, b, C.byref(logits))
+    def decoderStep(self, weights: Sequence, x, crossK, crossV, selfK, selfV, n: int, NH: int, HD: int, lnf, logits) -> Tensor:
+        """Optional member: one token of S streams through all layers (their decoderWeights), x [S, D] -> logits (see
+        fa_decoder_step); lnf is (gamma, beta), logits the vocabulary matrix as a weight of decoderWeights."""
+        L = len(weights)
+        handles = lambda ts: (C.c_void_p * L)(*[t.h for t in ts])  # noqa: E731
+        return self._op(self._lib.fa_decoder_step, (_lib.DecoderLayer * L)(*weights), L, x.h, handles(crossK), handles(crossV),
+                        handles(selfK), handles(selfV), n, NH, HD, lnf[0].h, lnf[1].h, C.byref(self._linear_of(logits, None)))
 
     def conformerWeights(self, w: dict):
         """The weights of conformerBlock from an encoder layer's dict of tensors (absent ones: None)."""

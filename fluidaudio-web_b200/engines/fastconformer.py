@@ -132,10 +132,10 @@ def load_encoder(ctx, weights: Dict[str, np.ndarray], cfg_override: Optional[dic
                 lw["qkvb"] = ctx.upload(b, 1, b.size)
             else:
                 lw["qkvb"] = None
-    enc = dict(sub=sub, layers=layers, cfg=cfg, _pe={}, _posProj={})
-    if hasattr(ctx, "conformerBlock") and not any(isinstance(t, Int8Weight) for lw in layers for t in lw.values()):
-        enc["native"] = [ctx.conformerWeights(lw) for lw in layers]  # optional member: a block in one call
-    return enc
+    for lw in layers:
+        if hasattr(ctx, "conformerBlock") and not any(isinstance(t, Int8Weight) for t in lw.values()):
+            lw["native"] = ctx.conformerWeights(lw)  # optional member: a block in one call
+    return dict(sub=sub, layers=layers, cfg=cfg, _pe={}, _posProj={})
 
 
 def pos_encoding(Tsub: int, D: int) -> np.ndarray:
@@ -274,10 +274,10 @@ def encode_batch(ctx, enc, mels: List[np.ndarray], layer_hook=None, use_fast: bo
             layerArena = ctx.pushArena()
             try:
                 w = enc["layers"][L]
-                if use_fast and "native" in enc:
+                if use_fast and "native" in w:
                     p = pos_proj(L, w) if W > 1 else peT
                     nxt = enc["layers"][L + 1]["lnff1"] if L + 1 < LAYERS else None
-                    x, xff = ctx.conformerBlock(enc["native"][L], x, xff, p, W > 1, H, HD, W, dwK, nxt)
+                    x, xff = ctx.conformerBlock(w["native"], x, xff, p, W > 1, H, HD, W, dwK, nxt)
                     ctx.pin(x, True)  # x feeds the next layer: promote to the enclosing arena
                     if xff is not None:
                         ctx.pin(xff, True)

@@ -129,14 +129,13 @@ def load_decoder(ctx, weights: Dict[str, np.ndarray], NH: int, quant: Optional[s
     embedTP = np.zeros((D, VOCABP), f32)
     embedTP[:, :VOCAB] = embed.T
     cfg["VOCABP"] = VOCABP
-    dec = dict(layers=layers, embed=embed, embedT=_W(ctx, embedTP, quant), pos=np.ascontiguousarray(weights["pos"], dtype=f32),
-               lnf=(vec("lnf_w"), vec("lnf_b")), cfg=cfg)
     if hasattr(ctx, "decoderStep"):  # optional member: all layers of a token in one call
-        pair = lambda w, k: (w[k + "w"].native(), w.get(k + "b"))
-        dec["native"] = ctx.decoderWeights([dict(sqkv=pair(w, "sqkv"), so=pair(w, "so"), cq=pair(w, "cq"), co=pair(w, "co"),
-                                                 f1=pair(w, "f1"), f2=pair(w, "f2"), ln1=w["ln1"], ln2=w["ln2"], ln3=w["ln3"])
-                                            for w in layers], dec["lnf"], dec["embedT"].native())
-    return dec
+        for w in layers:
+            pair = lambda k: (w[k + "w"].native(), w.get(k + "b"))
+            w["native"] = ctx.decoderWeights(dict(sqkv=pair("sqkv"), so=pair("so"), cq=pair("cq"), co=pair("co"), f1=pair("f1"),
+                                                  f2=pair("f2"), ln1=w["ln1"], ln2=w["ln2"], ln3=w["ln3"]))
+    return dict(layers=layers, embed=embed, embedT=_W(ctx, embedTP, quant), pos=np.ascontiguousarray(weights["pos"], dtype=f32),
+                lnf=(vec("lnf_w"), vec("lnf_b")), cfg=cfg)
 
 
 def _self_attention(ctx, x, w, cacheK, cacheV, n, S, D, NH, HD):
@@ -181,8 +180,9 @@ def _step(ctx, dec, kv, st, x, n, S):
     """The device part of one token: x [S, D] (embedding + position n) -> logits [S, VOCABP]."""
     cfg = dec["cfg"]
     D, NH, HD = cfg["D"], cfg["NH"], cfg["HD"]
-    if "native" in dec:
-        return ctx.decoderStep(dec["native"], x, [c["k"] for c in kv], [c["v"] for c in kv], st["selfK"], st["selfV"], n, NH, HD)
+    if all("native" in w for w in dec["layers"]):
+        return ctx.decoderStep([w["native"] for w in dec["layers"]], x, [c["k"] for c in kv], [c["v"] for c in kv], st["selfK"],
+                               st["selfV"], n, NH, HD, dec["lnf"], dec["embedT"].native())
     for li, w in enumerate(dec["layers"]):
         x = _layer(ctx, x, w, kv[li], st["selfK"][li], st["selfV"][li], n, S, D, NH, HD)
     return _linear(ctx, x, dec["embedT"], norm=dec["lnf"])

@@ -12,14 +12,21 @@ def test_conformer_blocks(ctx, pkg, W, samples):
 
     enc = fc.load_encoder(ctx, synth.encoder_weights(dict(synth.PARAKEET_06B, layers=2), seed=4))
     mel = ctx.logMelWindows(ctx.upload(synth.synth_audio(W, samples=samples, seed=5), W, samples), 128)
-    native = enc.pop("native")
+    layers = enc["layers"]
+    enc["layers"] = [{k: v for k, v in w.items() if k != "native"} for w in layers]
     host, t0 = fc.encode_batch(ctx, enc, mel)
     host = ctx.download(host)
     seen = []
-    enc["native"] = native
+    enc["layers"] = layers
     got, t1 = fc.encode_batch(ctx, enc, mel, layer_hook=lambda L, x: seen.append((L, x.rows)))
     assert t0 == t1 and [s[0] for s in seen] == [0, 1]
     assert np.array_equal(ctx.download(got), host)
+    # an encoder put together from another one's layers runs those layers, and half the blocks in each loop are the same blocks
+    last = dict(enc, layers=layers[1:], cfg=dict(enc["cfg"], layers=1), _posProj={})
+    plain = dict(last, layers=[{k: v for k, v in layers[1].items() if k != "native"}], _posProj={})
+    assert np.array_equal(*(ctx.download(fc.encode_batch(ctx, e, mel)[0]) for e in (last, plain)))
+    enc["layers"] = [{k: v for k, v in layers[0].items() if k != "native"}, layers[1]]
+    assert np.array_equal(ctx.download(fc.encode_batch(ctx, enc, mel)[0]), host)
 
 
 @pytest.mark.parametrize("quant", [None, "int8"])
@@ -31,14 +38,13 @@ def test_decoder_tokens(ctx, pkg, quant, S, NH):
     cfg = dict(D=256, NH=NH, FFN=1024, layers=2, VOCAB=2003, maxPos=40, Tenc=96)
     dec = wd.load_decoder(ctx, synth.decoder_weights(cfg, seed=11), NH, quant=quant)
     states = ctx.upload(np.concatenate(synth.encoder_states(cfg, S, seed=13)), S * cfg["Tenc"], cfg["D"])
-    native, runs = dec["native"], []
+    layers, runs = dec["layers"], []
     for with_native in (True, False):
         if not with_native:
-            dec.pop("native")
+            dec["layers"] = [{k: v for k, v in w.items() if k != "native"} for w in layers]
         kv = wd.cross_kv_streams(ctx, dec, states)
         st = wd.decode_init_streams(ctx, dec, S, 8)
         runs.append([wd.decode_next_streams(ctx, dec, kv, st, [t] * S, want_logits=True)[1] for t in (1, 7, 3)])
-    dec["native"] = native
     for a, b in zip(*runs):
         assert np.array_equal(a, b)
 
