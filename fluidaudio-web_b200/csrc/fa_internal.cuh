@@ -157,7 +157,7 @@ struct fa_ctx {
   std::unordered_map<int, int> mel_spans;  // widest filter of each mel count's filterbank, in bins
   // device-side status word written by kernels whose bounded waits ran out
   int *dev_status = nullptr;
-  int *gemv_tickets = nullptr;  // zeroed arrival counters of the split-K GEMV (self-resetting)
+  int *gemv_tickets = nullptr;  // zeroed arrival counters of the decoder attention's key splits (self-resetting)
   int gemv_ticket_count = 0;
   // graph recording: blocks acquired while `capturing` is set belong to that graph
   fa_graph *capturing = nullptr;

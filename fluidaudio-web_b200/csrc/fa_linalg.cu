@@ -2,11 +2,11 @@
 // (the reference's routers: src/gpu/compute.js:401-436, 593-611, 306-316).
 //
 //   tiny or ragged problems            -> any-shape f32 CUDA-core kernels (fa_gemm_simt.cu)
-//   f16-storage B, int8 B, int4 B      -> tcgen05 kernels (fa_gemm_tc.cu) for every other size,
-//                                         decode sizes (M <= 16) included: at 6.5 TB/s of HBM a CUDA
-//                                         core has fewer than 3 lane-operations per int4 weight, so
-//                                         only the tensor pipe keeps a decode product memory-bound.
-//   f32-storage B                      -> f32 CUDA-core kernel (the reference computes those in f32)
+//   one row of f16 / int8 B, one to    -> kernels on the weights as uploaded (fa_gemv.cu): CUDA cores, for 5 to 16 rows
+//   sixteen rows of int4 B                of int4 mma.sync
+//   f16-storage B, int8 B, int4 B      -> tcgen05 kernels (fa_gemm_tc.cu) for every other size
+//   f32-storage B                      -> tcgen05 kernel in f32-grade arithmetic (kind::tf32, value + residue planes) from
+//                                         a few rows and 256 columns on, else the f32 CUDA-core kernel
 #include "fa_internal.cuh"
 
 namespace {
