@@ -83,6 +83,8 @@ struct TcParams {
   int tiles_n, tiles_m;
   int splitk;         // > 1: cluster of `splitk` CTAs along z shares one tile, each taking kb_per_split chunks
   int kb_per_split;
+  int segs, kb_per_seg;  // > 1: a CTA's sum over K is kept as up to `segs` parts of kb_per_seg chunks in TMEM columns of their own,
+                      // added in order by the epilogue (one tile per CTA, plain f16 products; see launch_tc)
   int split_rb;       // split-K: 16-row blocks of a tile each CTA of the cluster owns, ceil(MT / 16 / splitk)
   int raw_i32;        // 1: store the limb-0 int32 accumulators instead of the float epilogue
   // batched mode (attention products): `batches` independent [M][N] problems share one launch.  Batch b
@@ -132,6 +134,8 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ void cluster_arrive_all() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait_all() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
+constexpr int kSiluExact = FA_ACT_SILU + 16;  // TcParams::act: SiLU as fa_actf computes it, not fa_silu_fast
+
 // Activation applied to 16 values at once with the selector outside the loop, so the 16 chains stay
 // independent (one warp per scheduler has no other work to hide a per-element branch behind).
 __device__ __forceinline__ void act16(float (&v)[16], int act) {
@@ -147,6 +151,10 @@ __device__ __forceinline__ void act16(float (&v)[16], int act) {
       // (84 us against 53 us for the same product without activation); ex2.approx + rcp.approx still cost 8 us of
       // special-function time per product.
       for (int j = 0; j < 16; j++) v[j] = fa_silu_fast(v[j]);
+      break;
+    case kSiluExact:
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[j] = fa_actf(v[j], FA_ACT_SILU);
       break;
     default:
 #pragma unroll
@@ -169,7 +177,8 @@ template <int KIND, bool PEERS = false>
 __device__ __forceinline__ void epilogue_tile(const TcParams &p, uint32_t lane_addr, int n0, int m0, int quad, int lane,
                                               int half, float *outb, int r16, int c16, uint32_t partial,
                                               const CUtensorMap *map_o, const CUtensorMap *map_o16, uint32_t slab_f32,
-                                              uint32_t slab_f16, uint32_t &slab_turn, uint32_t cl_rank) {
+                                              uint32_t slab_f16, uint32_t &slab_turn, uint32_t cl_rank, uint32_t nseg,
+                                              uint32_t acc_stride) {
   const int n = n0 + quad * 32 + lane;
   const bool n_ok = n < p.N;
   const float cs = (p.colscale && n_ok) ? p.colscale[n] : 1.0f;
@@ -178,6 +187,13 @@ __device__ __forceinline__ void epilogue_tile(const TcParams &p, uint32_t lane_a
     if (m0 + c >= p.M) break;  // warp-uniform: no rows left in this tile
     uint32_t v0[16], v1[16], v2[16];
     tmem_ld16(lane_addr + (uint32_t)c, v0);
+    for (uint32_t sg = 1; KIND == 0 && sg < nseg; sg++) {  // the parts of K, in order
+      uint32_t w[16];
+      tmem_ld16(lane_addr + sg * acc_stride + (uint32_t)c, w);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; j++) v0[j] = __float_as_uint(__uint_as_float(v0[j]) + __uint_as_float(w[j]));
+    }
     if (KIND == 1 && p.limbs > 1) tmem_ld16(lane_addr + (uint32_t)(p.MT + c), v1);
     if (KIND == 1 && p.limbs > 2) tmem_ld16(lane_addr + (uint32_t)(2 * p.MT + c), v2);
     const bool full_rows = m0 + c + 16 <= p.M;
@@ -593,7 +609,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
   const int acc_cols = p.limb_sum ? p.MT : q_rows;
   uint32_t acc_stride = 32;  // TMEM columns per accumulator buffer
   while ((int)acc_stride < acc_cols) acc_stride <<= 1;
-  const uint32_t tmem_cols = 2 * acc_stride;
+  const uint32_t tmem_cols = (KIND == 0 && p.segs > 2 ? (uint32_t)p.segs : 2u) * acc_stride;
   const int num_tiles = p.tiles_n * p.tiles_m * p.batches;
   const int kb0 = p.splitk > 1 ? (int)blockIdx.z * p.kb_per_split : 0;
   const int kb1 = p.splitk > 1 ? min(p.num_kb, kb0 + p.kb_per_split) : p.num_kb;
@@ -771,50 +787,53 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
             break;
           }
           tc_fence_after();
-          const uint32_t d_tmem = tmem_base + buf * acc_stride;
-          uint32_t acc = 0;
-          for (int kb = kb0; kb < kb1; kb += kSub) {
-            if (!__all_sync(0xffffffffu, mbar_wait(fb, ph, p.wait_limit))) {
-              if (lane == 0) set_abort(2, kb);
-              ok = false;
-              break;
-            }
-            if (kDeq) {
-              if (!__all_sync(0xffffffffu, mbar_wait(fb + doff, ph, p.wait_limit))) {  // weights tile unpacked
-                if (lane == 0) set_abort(6, kb);
+          uint32_t d_tmem = tmem_base + buf * acc_stride;
+          for (int kb = kb0; kb < kb1 && ok; d_tmem += acc_stride) {  // once, or once per part of K
+            const int ke = KIND == 0 ? min(kb1, kb + p.kb_per_seg) : kb1;
+            uint32_t acc = 0;
+            for (; kb < ke; kb += kSub) {
+              if (!__all_sync(0xffffffffu, mbar_wait(fb, ph, p.wait_limit))) {
+                if (lane == 0) set_abort(2, kb);
                 ok = false;
                 break;
               }
-              tc_fence_after();
-            }
+              if (kDeq) {
+                if (!__all_sync(0xffffffffu, mbar_wait(fb + doff, ph, p.wait_limit))) {  // weights tile unpacked
+                  if (lane == 0) set_abort(6, kb);
+                  ok = false;
+                  break;
+                }
+                tc_fence_after();
+              }
 #pragma unroll
-            for (int sub = 0; sub < kSub; sub++) {
-              const uint32_t dw = da + (uint32_t)sub * (kPTileBytes >> 4), db = da + q_off + (uint32_t)sub * (q_bytes >> 4);
-              umma_lo_w<MK>(lead, d_tmem, dw, db, d_hi, idesc, acc);  // 4 x 32 bytes of K per chunk
-              acc = 1u;
-              umma_lo_w<MK>(lead, d_tmem, dw + 2, db + 2, d_hi, idesc, 1u);
-              umma_lo_w<MK>(lead, d_tmem, dw + 4, db + 4, d_hi, idesc, 1u);
-              umma_lo_w<MK>(lead, d_tmem, dw + 6, db + 6, d_hi, idesc, 1u);
-              if (kLimbSum) {
-                umma_lo_w<MK>(lead, d_tmem, dw, db + lo_off, d_hi, idesc, 1u);
-                umma_lo_w<MK>(lead, d_tmem, dw + 2, db + lo_off + 2, d_hi, idesc, 1u);
-                umma_lo_w<MK>(lead, d_tmem, dw + 4, db + lo_off + 4, d_hi, idesc, 1u);
-                umma_lo_w<MK>(lead, d_tmem, dw + 6, db + lo_off + 6, d_hi, idesc, 1u);
+              for (int sub = 0; sub < kSub; sub++) {
+                const uint32_t dw = da + (uint32_t)sub * (kPTileBytes >> 4), db = da + q_off + (uint32_t)sub * (q_bytes >> 4);
+                umma_lo_w<MK>(lead, d_tmem, dw, db, d_hi, idesc, acc);  // 4 x 32 bytes of K per chunk
+                acc = 1u;
+                umma_lo_w<MK>(lead, d_tmem, dw + 2, db + 2, d_hi, idesc, 1u);
+                umma_lo_w<MK>(lead, d_tmem, dw + 4, db + 4, d_hi, idesc, 1u);
+                umma_lo_w<MK>(lead, d_tmem, dw + 6, db + 6, d_hi, idesc, 1u);
+                if (kLimbSum) {
+                  umma_lo_w<MK>(lead, d_tmem, dw, db + lo_off, d_hi, idesc, 1u);
+                  umma_lo_w<MK>(lead, d_tmem, dw + 2, db + lo_off + 2, d_hi, idesc, 1u);
+                  umma_lo_w<MK>(lead, d_tmem, dw + 4, db + lo_off + 4, d_hi, idesc, 1u);
+                  umma_lo_w<MK>(lead, d_tmem, dw + 6, db + lo_off + 6, d_hi, idesc, 1u);
+                }
+                if (KIND == 4) {  // weights' residue x activations' value
+                  umma_lo_w<MK>(lead, d_tmem, dw + wlo_off, db, d_hi, idesc, 1u);
+                  umma_lo_w<MK>(lead, d_tmem, dw + wlo_off + 2, db + 2, d_hi, idesc, 1u);
+                  umma_lo_w<MK>(lead, d_tmem, dw + wlo_off + 4, db + 4, d_hi, idesc, 1u);
+                  umma_lo_w<MK>(lead, d_tmem, dw + wlo_off + 6, db + 6, d_hi, idesc, 1u);
+                }
               }
-              if (KIND == 4) {  // weights' residue x activations' value
-                umma_lo_w<MK>(lead, d_tmem, dw + wlo_off, db, d_hi, idesc, 1u);
-                umma_lo_w<MK>(lead, d_tmem, dw + wlo_off + 2, db + 2, d_hi, idesc, 1u);
-                umma_lo_w<MK>(lead, d_tmem, dw + wlo_off + 4, db + 4, d_hi, idesc, 1u);
-                umma_lo_w<MK>(lead, d_tmem, dw + wlo_off + 6, db + 6, d_hi, idesc, 1u);
-              }
+              umma_commit_w(lead, fb + eoff);  // frees the slot when these MMAs have read it
+              fb += 8u;
+              da += st_off;
+              const bool wrap = fb == fb_end;
+              fb = wrap ? bars : fb;
+              da = wrap ? da0 : da;
+              ph ^= wrap ? 1u : 0u;
             }
-            umma_commit_w(lead, fb + eoff);  // frees the slot when these MMAs have read it
-            fb += 8u;
-            da += st_off;
-            const bool wrap = fb == fb_end;
-            fb = wrap ? bars : fb;
-            da = wrap ? da0 : da;
-            ph ^= wrap ? 1u : 0u;
           }
           if (ok) umma_commit_w(lead, acc_full(buf));  // this tile's accumulators are complete
         }
@@ -1011,7 +1030,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
       if (!ok) break;
       tc_fence_after();
       const uint32_t lane_addr = tmem_base + buf * acc_stride + ((uint32_t)(quad * 32) << 16);
-      if (!kDeq && MK != 1 && p.splitk == 1 && !p.rowscale && !p.rowbias)
+      if (!kDeq && MK != 1 && p.splitk == 1 && (KIND != 0 || p.segs == 1) && !p.rowscale && !p.rowbias)
       {
         if (KIND == 0 && p.tma_add)
           epilogue_tile_resadd(p, lane_addr, n0, m0, quad, lane, half, r16, c16, &map_o, &map_o16, &map_add, slab_f32, slab_f16,
@@ -1026,7 +1045,8 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
       }
       else
         epilogue_tile<MK, KIND == 3>(p, lane_addr, n0, m0, quad, lane, half, outb, r16, c16, partial, &map_o, &map_o16,
-                                     slab_f32, slab_f16, slab_turn, cl_rank);
+                                     slab_f32, slab_f16, slab_turn, cl_rank,
+                                     KIND == 0 ? (uint32_t)((kb1 - kb0 + p.kb_per_seg - 1) / p.kb_per_seg) : 1u, acc_stride);
       // hand the accumulator buffer back to the MMA warp
       tc_fence_before();
       __syncwarp();
@@ -1313,7 +1333,7 @@ k_tc_gemm_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                                          slab_turn);
       else
         epilogue_tile<0, false>(p, lane_addr, n0, m0, quad, lane, half, p.out, 0, 0, 0u, &map_o, &map_o16, slab_f32,
-                                slab_f16, slab_turn, 0u);
+                                slab_f16, slab_turn, 0u, 1u, 0u);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(acc_empty(buf), 0);
@@ -1720,31 +1740,37 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
   // One wave only (a second one costs more than any split saves): clusters do not tile every GPC, so quarters may use
   // 7/8 of the SMs and eighths 2/3; clusters of 3, 5, 6, 7 place badly (2x slower).  Against the rule before it (shortest
   // tile of at least 64 rows, then the widest split), recorded products, us: f32 300 x 4096 x 1024 35.6 -> 28.8, 800 x 4096
-  // x 1024 62.2 -> 51.6; int8 100 x 1024 x 4096 11.7 -> 7.9, 300 x 2048 x 1024 14.0 -> 11.0; f16 300 x 1024 x 1024 8.4 ->
-  // 5.8, 200 x 1024 x 1024 7.2 -> 5.7.
+  // x 1024 62.2 -> 51.6; int8 100 x 1024 x 4096 11.7 -> 7.9, 300 x 2048 x 1024 14.0 -> 11.0; f16 300 x 1024 x 1024 8.6 ->
+  // 6.9, 512 x 512 x 512 7.9 -> 5.8.
   // (the split-K finish stores rows at pitch N: a caller-chosen pitch keeps the one-CTA-per-tile form)
   p.splitk = 1;
   p.kb_per_split = p.num_kb;
+  p.segs = 1;
+  bool exact_silu = false;
   const bool split_ok = !raw_i32 && !ep.out16 && ep.n_peers == 0 && (ep.ldc == 0 || ep.ldc == N) && p.batches == 1;
   if (split_ok && num_tiles <= ctx->sm_count) {
     const int mt_hi = mt < mt_max ? mt : mt_max, w_rows = (KIND == 4 ? 2 : 1) * 128;
     int best_mt = p.MT, best_s = 1;
-    // f32-grade products (residue planes): a sum that stays in one accumulator longer loses more to its truncation, so K is
-    // split at least as wide as by the plain rule: the shortest tile of at least 64 rows that keeps one wave, then the
-    // widest split that does (with the K = 1280 products of a decoder token unsplit, its logits were 5.1e-5 off the CPU
-    // reference, over the 5e-5 that they keep to split four ways)
-    if (KIND == 4 || (KIND == 0 && limbs == 2)) {
-      for (int cand = p.MT; cand >= (p.MT < 64 ? p.MT : 64); cand -= 16) {
-        if ((long long)p.tiles_n * ceil_div(M, cand) > ctx->sm_count) break;
-        best_mt = cand;
-      }
-      while (best_mt > 16 && ceil_div(M, best_mt - 16) == ceil_div(M, best_mt)) best_mt -= 16;  // same tiling, less padding
-      for (int sp = 2; sp <= 8 && best_mt <= 64; sp *= 2) {
-        if ((long long)p.tiles_n * ceil_div(M, best_mt) * sp > ctx->sm_count || p.num_kb / sp < 4) break;
-        if ((sp - 1) * ceil_div(p.num_kb, sp) < p.num_kb) best_s = sp;  // (33 chunks by 8: the last CTA would have nothing to sum)
-      }
+    // The plain rule: the shortest tile of at least 64 rows that keeps one wave, then the widest split that does.  A sum that
+    // stays in one accumulator longer loses more to its truncation (2^-25 of it per step of 32 bytes of K), so every float
+    // form keeps K in at least as many parts as this rule gives: as ranks of the cluster, or, plain f16 products (one operand
+    // plane each), as parts of one CTA's sum in TMEM columns of their own, added in the same order by the epilogue.
+    // Error of products of f16 values against f64, parts kept / one sum: 200 x 1024 x 1024 3.4e-7 / 1.25e-6, 160 x 2048 x 2048
+    // 1.25e-6 / 2.5e-6.  (With the K = 1280 products of a decoder token in one sum, its logits were 5.1e-5 off the CPU
+    // reference, over the 5e-5 that they keep in four parts.)
+    for (int cand = p.MT; cand >= (p.MT < 64 ? p.MT : 64); cand -= 16) {
+      if ((long long)p.tiles_n * ceil_div(M, cand) > ctx->sm_count) break;
+      best_mt = cand;
     }
-    const int min_s = best_s;
+    while (best_mt > 16 && ceil_div(M, best_mt - 16) == ceil_div(M, best_mt)) best_mt -= 16;  // same tiling, less padding
+    for (int sp = 2; sp <= 8 && best_mt <= 64; sp *= 2) {
+      if ((long long)p.tiles_n * ceil_div(M, best_mt) * sp > ctx->sm_count || p.num_kb / sp < 4) break;
+      if ((sp - 1) * ceil_div(p.num_kb, sp) < p.num_kb) best_s = sp;  // (33 chunks by 8: the last CTA would have nothing to sum)
+    }
+    const int parts = best_s;
+    const bool own_parts = KIND == 0 && limbs == 1;
+    const int min_s = KIND == 1 || own_parts ? 1 : parts;  // (integer sums are exact)
+    int best_g = 1;
     long long best = -1;
     for (int cand = mt_hi; cand >= (mt_hi < 32 ? mt_hi : 32); cand -= 16) {
       const int tiles_m = ceil_div(M, cand);
@@ -1755,10 +1781,12 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
         if (ctas > room || (sp > 1 && (cand > kSplitMaxMT || p.num_kb / sp < 4))) continue;
         const long long rows = w_rows + cand * limbs, chunks = ceil_div(p.num_kb, sp);
         if ((sp - 1) * chunks >= p.num_kb) continue;  // the last CTA of the cluster would have nothing
+        const int g = own_parts && sp < parts ? parts / sp : 1;
+        if (g > 1 && g * (cand <= 32 ? 32 : (cand <= 64 ? 64 : (cand <= 128 ? 128 : 256))) > 512) continue;  // TMEM columns
         long long cost = chunks * (rows > 160 ? rows : 160) + 6 * cand + 14 * ctas;
         if (sp > 1)
           cost += (cand > 64 ? 5500 : (KIND == 1 ? 3700 : 1500 + 35 * cand)) + (sp == 2 && cand > 96 ? 2500 : 0) + (sp == 8 ? 600 : 0);
-        if (best < 0 || cost < best) best = cost, best_mt = cand, best_s = sp;
+        if (best < 0 || cost < best) best = cost, best_mt = cand, best_s = sp, best_g = g;
       }
     }
     if (ctx->tc_tile_rows > 0 || ctx->tc_split_k > 0) {  // tuning overrides (options "tc_tile_rows", "tc_split_k")
@@ -1767,6 +1795,7 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
       if (best_mt > kSplitMaxMT) best_s = 1;
       while (best_s > 1 && p.num_kb / best_s < 2) best_s--;
       if (best_s > 1) best_s = ceil_div(p.num_kb, ceil_div(p.num_kb, best_s));
+      best_g = 1;
     }
     p.MT = best_mt;
     p.tiles_m = ceil_div(M, p.MT);
@@ -1774,8 +1803,12 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
       p.kb_per_split = ceil_div(p.num_kb, best_s);
       p.splitk = best_s;
     }
+    p.segs = best_g;
+    // what the plain rule splits had its activation applied by the split's finish, which computes SiLU as fa_actf does
+    exact_silu = parts > 1 && best_s == 1;
     num_tiles = p.tiles_n * p.tiles_m * p.batches;
   }
+  p.kb_per_seg = ceil_div(p.kb_per_split, p.segs);
   // Many tiles: CTA pairs (see k_tc_gemm_pair).  Row tile by the same rule as above over half as many workers,
   // with a per-tile constant for the ramp of a tile's first loads.
   bool pair = false;
@@ -1807,7 +1840,7 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
                   ? 1
                   : 0;
   // the residual through the copy engine (epilogue_tile_resadd): the plain f16 product with an f32 result and TMA stores
-  const bool want_add = KIND == 0 && p.tma_out && ep.add && !p.skip_f32 && !ep.rowscale && !ep.rowbias && (N & 3) == 0 && K <= 2048 &&
+  const bool want_add = KIND == 0 && p.tma_out && p.segs == 1 && ep.add && !p.skip_f32 && !ep.rowscale && !ep.rowbias && (N & 3) == 0 && K <= 2048 &&
                         ((uintptr_t)ep.add & 15) == 0 && ctx->tc_tma_add;
   // two store slabs per warp and result kind, four when that leaves the ring as deep
   auto slab_bytes_for = [&](int nslab) {
@@ -1834,7 +1867,7 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
   // residue planes, 64 x 5120 x 1280 10.3 -> 10.7.
   p.step = 1;
   if ((KIND == 1 || (KIND == 0 && limbs == 1 && p.kb_per_split >= 32)) && !pair && p.batches == 1 && ep.n_peers == 0 && !(p.num_kb & 1) &&
-      !(p.kb_per_split & 1) && stages >= 6 && ctx->tc_wide_stages) {
+      !(p.kb_per_split & 1) && (p.segs == 1 || !(p.kb_per_seg & 1)) && stages >= 6 && ctx->tc_wide_stages) {
     p.step = 2;
     stages /= 2;
   }
@@ -1850,7 +1883,7 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
   p.bias = ep.bias;
   p.add = ep.add;
   p.rowbias = ep.rowbias;
-  p.act = ep.act;
+  p.act = exact_silu && ep.act == FA_ACT_SILU ? kSiluExact : ep.act;
   p.status = ctx->dev_status;
   p.wait_limit = ctx->wait_limit;
   p.withhold_kb = ctx->tc_withhold_chunk;

@@ -77,3 +77,37 @@ def test_digit_pass_of_whole_quads(ctx, K):
         ctx.setOption("gemv_rows", 4)
     assert np.abs(got - 0.01 * (a.astype(np.float64) @ q)).max() < 1e-6 * K
     assert not got[3].any()
+
+
+# parts: how many sums K is kept in at least.  The operands are f16 values, so what is left is the accumulator: a step adds 16
+# products and drops less than 2^-25 of the sum on average, and a part takes K / 16 / parts steps.
+@pytest.mark.parametrize("M,K,N,parts", [(65, 1024, 1024, 4), (200, 1024, 1024, 4), (375, 1024, 1024, 2), (128, 2048, 2048, 4),
+                                         (250, 2048, 2048, 2), (65, 4096, 1024, 8), (100, 1024, 4096, 2), (70, 512, 2048, 2),
+                                         (190, 1000, 1000, 2), (360, 5120, 1280, 2)])
+def test_a_sum_stays_in_parts(ctx, M, K, N, parts):
+    rng = np.random.default_rng(M + K)
+    a, w = (rng.standard_normal(s).astype(np.float16).astype(np.float32) for s in ((M, K), (K, N)))
+    add = rng.standard_normal((M, N)).astype(np.float32)
+    want = a.astype(np.float64) @ w.astype(np.float64)
+    ta, tw = ctx.upload(a, M, K), ctx.uploadF16(w, K, N)
+    for got, ref in ((ctx.matmul(ta, tw), want), (ctx.matmul(ta, tw, add=ctx.upload(add, M, N)), want + add)):
+        err = ctx.download(got).reshape(M, N) - ref
+        assert np.linalg.norm(err) / np.linalg.norm(ref) < K / 16 / parts * 2.0 ** -25
+
+
+@pytest.mark.parametrize("M,K,N", [(100, 1024, 4096), (200, 4096, 1024), (60, 1024, 1024)])
+def test_silu_of_one_wave_int8_products(ctx, M, K, N):
+    """Three digits carry a row to 2^-22 of its maximum and the activation is x / (1 + exp(-x)) in f32, so results of order 1
+    stay within 1e-5, which the epilogue that computes it by an approximate tanh leaves."""
+    rng = np.random.default_rng(M)
+    a = rng.standard_normal((M, K)).astype(np.float32)
+    q = rng.integers(-127, 128, (K, N), dtype=np.int8)
+    sc = np.full(N, 1 / (73.3 * np.sqrt(K)), np.float32)
+    ctx.setOption("int8_limbs", 3)
+    try:
+        got = ctx.download(ctx.matmulInt8(ctx.upload(a, M, K), ctx.uploadBytes(q.view(np.uint8).reshape(-1)), ctx.upload(sc, 1, N), N, K,
+                                          act="silu")).reshape(M, N)
+    finally:
+        ctx.setOption("int8_limbs", 2)
+    z = a.astype(np.float64) @ (q * sc.astype(np.float64))
+    assert np.abs(got - z / (1 + np.exp(-z))).max() < 1e-5
