@@ -409,7 +409,7 @@ extern "C" int fa_linear_step(fa_ctx *ctx, const fa_tensor *x, const fa_tensor *
   auto al = [](const fa_tensor *t) { return ((uintptr_t)t->dptr & 15) == 0; };
   const bool one = x->rows == 1 && x->cols == K && x->storage == FA_F32 && (!w || w->storage == FA_F16) && N > 0 && K > 0 &&
                    gemv_shape_ok(ctx, 1, N, K) && fa_gemv_kn_ok(1, N, K) && act >= 0 && act <= 5 &&
-                   (w || wq->nbytes >= (size_t)N * K) && (!add || (add->rows == 1 && add->cols == N)) &&
+                   (w || wq->nbytes >= (size_t)N * K) && (!add || (fa_valid(ctx, add) && add->rows == 1 && add->cols == N)) &&
                    (!gamma || (fa_gemv_kn_norm_ok(K) && fa_valid(ctx, gamma) && fa_valid(ctx, beta) && al(x) && al(gamma) && al(beta)));
   if (one) {
     FA_TRY(check_vec(ctx, x, K, "linearStep: x"));

@@ -54,3 +54,18 @@ def test_linear_step_checks_its_operands(ctx, pkg):
         ctx.linearStep(x, w, add=ctx.alloc(1, 128))
     with pytest.raises(pkg.CudaError):
         ctx.linearStep(x, w, bias=ctx.alloc(1, 128))
+
+
+def test_stale_handles_are_refused_unread(ctx, pkg):
+    """A handle is looked up before what it points at is read: an address that was never a tensor's (nothing is mapped there)
+    is an error, not a crash."""
+    gone = pkg.Tensor(0x40, 1, 256)
+    for M in (1, 2):
+        x, w, n = ctx.alloc(M, 128), ctx.uploadF16(np.zeros(128 * 256, np.float32), 128, 256), ctx.alloc(1, 128)
+        for kw in (dict(add=gone), dict(bias=gone), dict(norm=(gone, n)), dict(norm=(n, gone))):
+            with pytest.raises(pkg.CudaError):
+                ctx.linearStep(x, w, **kw)
+        with pytest.raises(pkg.CudaError):
+            ctx.linearStep(x, gone)
+        with pytest.raises(pkg.CudaError):
+            ctx.linearStep(gone, w)
