@@ -62,6 +62,7 @@ SIGNATURES = {
     "fa_trim_pool": [P, C.c_size_t],
     "fa_tensor_info": [P, IP, IP, IP, PP],
     "fa_mem_stats": [P, ULLP, ULLP, ULLP, ULLP],
+    "fa_handle_count": [P, C.POINTER(C.c_ulonglong)],
     "fa_host_alloc": [C.c_size_t, PP],
     "fa_host_free": [P],
     "fa_download": [P, P, P],

@@ -591,6 +591,12 @@ class CudaContext:
         self._check(self._lib.fa_mem_stats(self._h, C.byref(a), C.byref(b), C.byref(c), C.byref(d)))
         return {"created": a.value, "createdBytes": b.value, "reused": c.value, "poolBytes": d.value}
 
+    def handleCount(self) -> int:
+        """Live tensor handles, views included."""
+        n = C.c_ulonglong()
+        self._check(self._lib.fa_handle_count(self._h, C.byref(n)))
+        return n.value
+
     def poolInfo(self):
         return {"bytes": self.memStats()["poolBytes"]}
 

@@ -605,6 +605,12 @@ extern "C" int fa_mem_stats(fa_ctx *ctx, unsigned long long *created, unsigned l
   return FA_OK;
 }
 
+extern "C" int fa_handle_count(fa_ctx *ctx, unsigned long long *tensors) {
+  if (!ctx || !tensors) return fa_fail(ctx, FA_ERR_INVALID, "handleCount: NULL argument");
+  *tensors = ctx->tensors.size();
+  return FA_OK;
+}
+
 extern "C" int fa_host_alloc(size_t nbytes, void **out) {
   if (!out) return FA_ERR_INVALID;
   cudaError_t e = cudaMallocHost(out, nbytes ? nbytes : 1);

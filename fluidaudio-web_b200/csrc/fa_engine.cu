@@ -4,7 +4,7 @@
 // 7-9 us of interpreter, foreign-function and handle work around ~4 us of C, more than most of the kernels take.  These
 // entry points issue the same members in the same order (src/engines/asr-whisper/raw-whisper-decoder.js:108-140,
 // src/engines/asr-parakeet/raw-encoder.js:240-386), so that the host calls once per layer stack or block.  Nothing here
-// launches a kernel of its own and no handle is kept.
+// launches a kernel of its own and no handle is kept, views included.
 #include "fa_internal.cuh"
 
 namespace {
@@ -30,31 +30,51 @@ int linear(fa_ctx *ctx, const fa_tensor *x, const fa_tensor *g, const fa_tensor 
                         w.K, w.bias, act, add, out);
 }
 
+// Views of one layer.  No arena owns a view, so they are freed here on every way out, before the arena frees what they look at.
+struct Views {
+  fa_ctx *ctx;
+  fa_tensor *v[6];
+  int n = 0;
+  explicit Views(fa_ctx *c) : ctx(c) {}
+  int add(int rc, fa_tensor **t) {
+    if (rc == FA_OK) v[n++] = *t;
+    return rc;
+  }
+  int reshape(fa_tensor *t, int rows, int cols, fa_tensor **out) { return add(fa_reshape_view(ctx, t, rows, cols, out), out); }
+  int rows(fa_tensor *t, int rows, fa_tensor **out) { return add(fa_rows_view(ctx, t, rows, out), out); }
+  ~Views() {
+    const std::string msg = ctx->err;
+    for (int i = 0; i < n; i++) fa_free_tensor(ctx, v[i]);
+    ctx->err = msg;
+  }
+};
+
 // raw-whisper-decoder.js:112-124 from the separate members, for shapes the one-pass attention declines
-int self_attention_ops(fa_ctx *ctx, const fa_tensor *qkv, fa_tensor *ck, fa_tensor *cv, int n, int NH, int HD, fa_tensor **out) {
+int self_attention_ops(fa_ctx *ctx, Views &views, const fa_tensor *qkv, fa_tensor *ck, fa_tensor *cv, int n, int NH, int HD, fa_tensor **out) {
   const int S = qkv->rows, D = NH * HD;
   fa_tensor *part[3], *flat[3], *K, *V, *sc, *pr, *att;
   for (int i = 0; i < 3; i++) {
     FA_TRY(fa_slice_cols(ctx, qkv, i * D, D, &part[i]));
-    FA_TRY(fa_reshape_view(ctx, part[i], 1, S * D, &flat[i]));
+    FA_TRY(views.reshape(part[i], 1, S * D, &flat[i]));
   }
   FA_TRY(fa_copy_rows(ctx, ck, flat[1], n));
   FA_TRY(fa_copy_rows(ctx, cv, flat[2], n));
-  FA_TRY(fa_rows_view(ctx, ck, n + 1, &K));
-  FA_TRY(fa_rows_view(ctx, cv, n + 1, &V));
+  FA_TRY(views.rows(ck, n + 1, &K));
+  FA_TRY(views.rows(cv, n + 1, &V));
   FA_TRY(fa_bmm_qk(ctx, flat[0], K, nullptr, S * NH, HD, 1, 0, &sc));
   FA_TRY(fa_softmax(ctx, sc, &pr));
   FA_TRY(fa_bmm_pv(ctx, pr, V, S * NH, HD, 1, &att));
-  return fa_reshape_view(ctx, att, S, D, out);
+  return views.reshape(att, S, D, out);
 }
 
 int decoder_layer(fa_ctx *ctx, const fa_decoder_layer &w, const fa_tensor *x, const fa_tensor *kk, const fa_tensor *kv, fa_tensor *ck,
                   fa_tensor *cv, int n, int NH, int HD, fa_tensor **out) {
   const int S = x->rows;
   fa_tensor *qkv, *att = nullptr, *x1, *cq, *x2, *h;
+  Views views(ctx);
   FA_TRY(linear(ctx, x, w.ln1_w, w.ln1_b, w.sqkv, FA_ACT_NONE, nullptr, &qkv));
   FA_TRY(fa_attn_step_append(ctx, qkv, ck, cv, n, NH, HD, &att));
-  if (!att) FA_TRY(self_attention_ops(ctx, qkv, ck, cv, n, NH, HD, &att));
+  if (!att) FA_TRY(self_attention_ops(ctx, views, qkv, ck, cv, n, NH, HD, &att));
   FA_TRY(linear(ctx, att, nullptr, nullptr, w.so, FA_ACT_NONE, x, &x1));
   FA_TRY(linear(ctx, x1, w.ln2_w, w.ln2_b, w.cq, FA_ACT_NONE, nullptr, &cq));
   FA_TRY(fa_attn_step(ctx, cq, kk, kv, NH, HD, S, &att));

@@ -127,6 +127,8 @@ int fa_tensor_ptr(fa_ctx *ctx, const fa_tensor *t, void **device_ptr);
 /* memStats / poolInfo (compute.d.ts:252-254): allocations made, bytes made, pool hits, bytes idle in the pool. */
 int fa_mem_stats(fa_ctx *ctx, unsigned long long *created, unsigned long long *created_bytes,
                  unsigned long long *reused, unsigned long long *pool_bytes);
+/* Live tensor handles, views included. */
+int fa_handle_count(fa_ctx *ctx, unsigned long long *tensors);
 /* Page-locked host memory for callers that want uploads/downloads to be truly asynchronous. */
 int fa_host_alloc(size_t nbytes, void **out);
 int fa_host_free(void *p);

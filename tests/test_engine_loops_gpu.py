@@ -62,3 +62,43 @@ def test_decode_next_gives_its_row_back(ctx, pkg):
     for t in range(5):
         wd.decode_next(ctx, dec, kv, st, t)
     assert ctx.memStats() ["created"] == before["created"]
+
+
+@pytest.mark.parametrize("S", [1, 3])
+def test_decoder_tokens_with_heads_that_the_one_pass_attention_declines(ctx, pkg, S):
+    """Head width 48: the native loop's separate members, same bits as the host loop, and no handle left behind."""
+    from fluidaudio_web_b200.engines import synth, whisper_decoder as wd
+
+    cfg = dict(D=192, NH=4, FFN=768, layers=2, VOCAB=2003, maxPos=40, Tenc=96)
+    dec = wd.load_decoder(ctx, synth.decoder_weights(cfg, seed=17), 4)
+    states = ctx.upload(np.concatenate(synth.encoder_states(cfg, S, seed=13)), S * cfg["Tenc"], cfg["D"])
+    kv, layers, runs = wd.cross_kv_streams(ctx, dec, states), dec["layers"], []
+    for native in (True, False):
+        if not native:
+            dec["layers"] = [{k: v for k, v in w.items() if k != "native"} for w in layers]
+        st = wd.decode_init_streams(ctx, dec, S, 8)
+        before = ctx.handleCount()
+        runs.append([wd.decode_next_streams(ctx, dec, kv, st, [t] * S, want_logits=True)[1] for t in (1, 7, 3)])
+        assert not native or ctx.handleCount() == before
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("W,samples", [(1, 59200), (3, 64000)])
+def test_conformer_blocks_when_the_one_kernel_attention_is_off(ctx, pkg, W, samples):
+    from fluidaudio_web_b200.engines import fastconformer as fc, synth
+
+    enc = fc.load_encoder(ctx, synth.encoder_weights(dict(synth.PARAKEET_06B, layers=2), seed=4))
+    mel = ctx.logMelWindows(ctx.upload(synth.synth_audio(W, samples=samples, seed=5), W, samples), 128)
+    layers = enc["layers"]
+    ctx.setOption("attn_one_kernel", 0)
+    try:
+        native = ctx.download(fc.encode_batch(ctx, enc, mel)[0])
+        before, arena = ctx.handleCount(), ctx.pushArena()
+        fc.encode_batch(ctx, enc, mel)
+        ctx.popArena(arena)
+        assert ctx.handleCount() == before
+        enc["layers"] = [{k: v for k, v in w.items() if k != "native"} for w in layers]
+        assert np.array_equal(ctx.download(fc.encode_batch(ctx, enc, mel)[0]), native)
+    finally:
+        ctx.setOption("attn_one_kernel", 1)
