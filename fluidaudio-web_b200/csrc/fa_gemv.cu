@@ -447,12 +447,15 @@ __global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
   if (tid < COLS && n < N) p.y[n] = gemv_finish(sum, 0, n, N, p.ep);
 }
 
+constexpr size_t kNbitsSmemMax = 97 * 1024;  // fa_gemv_nbits_ok keeps every launch below
+
 template <int M, int R, int PRE>
 int launch_nbits_r(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y, int N,
                    int K, int nblk, int zpb) {
   const size_t smem = (size_t)M * 2 * K + (size_t)M * 2 * nblk * 4 + 8 * M * 4;
   auto kern = k_gemv_nbits<M, R, PRE>;
-  if (smem > 48 * 1024) FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static SmemLimit limit;
+  FA_CHECK_CUDA(ctx, limit.raise(ctx, kern, kNbitsSmemMax));
   // one resident wave: every CTA pays the digit prologue once and a second wave would pay it twice
   int per_sm = 0;
   FA_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem));
@@ -771,7 +774,8 @@ void mma_slices(int nblk, int &slices, int &slice, int &lq) {
 template <bool HILO, int G>
 cudaError_t launch_mma(fa_ctx *ctx, cudaLaunchConfig_t &cfg, const MmaParams &p) {
   cfg.dynamicSmemBytes = mma_smem(HILO, G, p.slice, (int)cfg.gridDim.y, p.lq);
-  const cudaError_t e = cudaFuncSetAttribute(k_nbits_mma<HILO, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+  static SmemLimit limit;
+  const cudaError_t e = limit.raise(ctx, k_nbits_mma<HILO, G>, 227 * 1024);
   return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, k_nbits_mma<HILO, G>, p);
 }
 

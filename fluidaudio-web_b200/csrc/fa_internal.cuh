@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -260,6 +261,20 @@ inline cudaError_t fa_launch_dep(fa_ctx *ctx, void (*kernel)(KArgs...), dim3 gri
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+
+// Raises a kernel's limit of dynamic shared memory, once per device and to the most that any launch of it asks for: the limit
+// belongs to the (kernel, device) pair, and lowering it to one launch's size would fail the launch of another thread's context.
+struct SmemLimit {
+  std::atomic<unsigned long long> devices{0};
+  template <typename... KArgs>
+  cudaError_t raise(const fa_ctx *ctx, void (*kernel)(KArgs...), size_t bytes) {
+    const unsigned long long bit = ctx->device < 64 ? 1ull << ctx->device : 0ull;
+    if (bit && (devices.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) devices.fetch_or(bit, std::memory_order_release);
+    return e;
+  }
+};
 
 // ---- device helpers ----------------------------------------------------------------
 

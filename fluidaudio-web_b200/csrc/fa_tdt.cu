@@ -619,11 +619,8 @@ int tdt_lr(int W) { return W <= 8 ? 3 : 5; }
 
 template <int MODE, int R>
 int tdt_rows_r(fa_ctx *ctx, const RowsParams &q, int blocks) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_tdt_rows<MODE, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, RowsCfg<R>::kSmem));
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  FA_CHECK_CUDA(ctx, limit.raise(ctx, k_tdt_rows<MODE, R>, RowsCfg<R>::kSmem));
   LaunchScope ls(ctx, MODE ? "tdt_lstm" : "tdt_pred");
   FA_CHECK_CUDA(ctx, fa_launch_dep(ctx, k_tdt_rows<MODE, R>, dim3(blocks, ceil_div(q.W, R)), dim3(kRowsThreads), RowsCfg<R>::kSmem, q));
   return FA_OK;
