@@ -423,12 +423,21 @@ class CudaContext:
         return self._wrap(out) if out.value else None
 
     # -- layer loops in native code (optional members) -----------------------------------------------
+    @staticmethod
+    def _live(t) -> Optional[int]:
+        """The handle of a weight, None for an absent one; a freed one would read as absent."""
+        if t is None:
+            return None
+        if not t.h:
+            raise CudaError(-1, "a weight of this layer has been freed")
+        return t.h
+
     def _linear_of(self, w, bias) -> "_lib.Linear":
         """(weights, bias) as the C struct; weights are a tensor [K, N] or (PackedBytes, scale, N, K)."""
         if isinstance(w, tuple):
             q, scale, N, K = w
-            return _lib.Linear(q.h, scale.h, self._h_of(bias), N, K)
-        return _lib.Linear(w.h, None, self._h_of(bias), w.cols, w.rows)
+            return _lib.Linear(self._live(q), self._live(scale), self._live(bias), N, K)
+        return _lib.Linear(self._live(w), None, self._live(bias), w.cols, w.rows)
 
     def decoderWeights(self, w: dict):
         """One layer's weights for decoderStep: sqkv, so, cq, co, f1, f2 as (weights, bias), ln1..ln3 as (gamma, beta)."""
@@ -436,7 +445,7 @@ class CudaContext:
         for n in ("sqkv", "so", "cq", "co", "f1", "f2"):
             setattr(d, n, self._linear_of(*w[n]))
         for n in ("ln1", "ln2", "ln3"):
-            setattr(d, n + "_w", w[n][0].h), setattr(d, n + "_b", w[n][1].h)
+            setattr(d, n + "_w", self._live(w[n][0])), setattr(d, n + "_b", self._live(w[n][1]))
         return d
 
     def decoderStep(self, weights: Sequence, x, crossK, crossV, selfK, selfV, n: int, NH: int, HD: int, lnf, logits) -> Tensor:
@@ -445,17 +454,20 @@ class CudaContext:
         L = len(weights)
         handles = lambda ts: (C.c_void_p * L)(*[t.h for t in ts])  # noqa: E731
         return self._op(self._lib.fa_decoder_step, (_lib.DecoderLayer * L)(*weights), L, x.h, handles(crossK), handles(crossV),
-                        handles(selfK), handles(selfV), n, NH, HD, lnf[0].h, lnf[1].h, C.byref(self._linear_of(logits, None)))
+                        handles(selfK), handles(selfV), n, NH, HD, self._live(lnf[0]), self._live(lnf[1]), C.byref(self._linear_of(logits, None)))
 
     def conformerWeights(self, w: dict):
-        """The weights of conformerBlock from an encoder layer's dict of tensors (absent ones: None)."""
-        h = lambda n, i=None: self._h_of(w.get(n) if i is None else w[n][i])  # noqa: E731
+        """The weights of conformerBlock from an encoder layer's dict of tensors (absent ones: None).  The struct holds raw
+        handles: it is good while the layer's entries are the ones it was made from (engines/layer_weights.py)."""
+        h = lambda n, i=None: self._live(w.get(n) if i is None else w[n][i])  # noqa: E731
         ff = lambda n: _lib.FeedForward(h("ln" + n, 0), h("ln" + n, 1), h(n + "w1"), h(n + "w2"), h(n + "b1"), h(n + "b2"))  # noqa: E731
         d = _lib.ConformerLayer(ff("ff1"), ff("ff2"))
         for n in ("lnatt", "lnconv", "lnout"):
             setattr(d, n + "_w", h(n, 0)), setattr(d, n + "_b", h(n, 1))
-        for n in ("q", "k", "v", "qkv", "pos", "out", "qb", "kb", "vb", "qkvb", "outb", "pw1b", "pw2b", "dw", "dwb"):
+        for n in ("qkv", "pos", "out", "qkvb", "outb", "pw1b", "pw2b", "dw", "dwb"):
             setattr(d, n, h(n))
+        for n in ("q", "k", "v", "qb", "kb", "vb"):  # (a program that only needs the fused form may have freed these)
+            setattr(d, n, self._h_of(w.get(n)) if d.qkv else h(n))
         d.pw1, d.pw2, d.pbu, d.pbv = h("pw1T"), h("pw2T"), h("pbuAll"), h("pbvAll")
         return d
 

@@ -13,6 +13,8 @@ from typing import Dict, List, Optional
 
 import numpy as np
 
+from .layer_weights import LayerWeights, fused_from, native_struct
+
 
 def infer_config(man: Dict[str, np.ndarray]) -> dict:
     """raw-encoder.js:28-35: every size is read off the weight shapes."""
@@ -23,6 +25,12 @@ def infer_config(man: Dict[str, np.ndarray]) -> dict:
     Fsub = man["linw"].shape[0] // Csub
     return dict(D=D, DFF=DFF, H=H, HD=HD, layers=layers, dwK=man["L0_dw"].shape[2], Csub=Csub, Fsub=Fsub,
                 melBins=Fsub * 8)
+
+
+# a layer's entries that conformerBlock reads, and those of them that "qkv" / "qkvb" are made of
+QKV_PARTS = ("q", "k", "v", "qb", "kb", "vb")
+NATIVE_KEYS = QKV_PARTS + ("qkv", "qkvb", "qkv_of", "lnff1", "ff1w1", "ff1w2", "ff1b1", "ff1b2", "lnff2", "ff2w1", "ff2w2", "ff2b1", "ff2b2",
+                           "lnatt", "lnconv", "lnout", "pos", "out", "outb", "pbuAll", "pbvAll", "pw1T", "pw2T", "pw1b", "pw2b", "dw", "dwb")
 
 
 class Int8Weight:
@@ -132,10 +140,20 @@ def load_encoder(ctx, weights: Dict[str, np.ndarray], cfg_override: Optional[dic
                 lw["qkvb"] = ctx.upload(b, 1, b.size)
             else:
                 lw["qkvb"] = None
+            lw["qkv_of"] = tuple(map(lw.get, QKV_PARTS))
     for lw in layers:
         if hasattr(ctx, "conformerBlock") and not any(isinstance(t, Int8Weight) for t in lw.values()):
-            lw["native"] = ctx.conformerWeights(lw)  # optional member: a block in one call
+            lw["native"] = LayerWeights(lw, NATIVE_KEYS, _native_of(ctx))  # optional member: a block in one call
     return dict(sub=sub, layers=layers, cfg=cfg, _pe={}, _posProj={})
+
+
+def _native_of(ctx):
+    """What makes the weights of conformerBlock from a layer; None for a layer with int8 weights, which it does not take."""
+    def make(w):
+        if any(isinstance(w.get(k), Int8Weight) for k in NATIVE_KEYS):
+            return None
+        return ctx.conformerWeights(w if fused_from(w, "qkv", QKV_PARTS) else dict(w, qkv=None, qkvb=None))
+    return make
 
 
 def pos_encoding(Tsub: int, D: int) -> np.ndarray:
@@ -266,6 +284,7 @@ def encode_batch(ctx, enc, mels: List[np.ndarray], layer_hook=None, use_fast: bo
 
     # optional member: a block's last layernorm and the next block's first one in one pass over the rows
     chain = use_fast and hasattr(ctx, "layernormChain")
+    make_native = _native_of(ctx)
 
     def body():
         nonlocal x
@@ -274,10 +293,11 @@ def encode_batch(ctx, enc, mels: List[np.ndarray], layer_hook=None, use_fast: bo
             layerArena = ctx.pushArena()
             try:
                 w = enc["layers"][L]
-                if use_fast and "native" in w:
+                native = native_struct(w, NATIVE_KEYS, make_native) if use_fast and "native" in w else None
+                if native is not None:
                     p = pos_proj(L, w) if W > 1 else peT
                     nxt = enc["layers"][L + 1]["lnff1"] if L + 1 < LAYERS else None
-                    x, xff = ctx.conformerBlock(w["native"], x, xff, p, W > 1, H, HD, W, dwK, nxt)
+                    x, xff = ctx.conformerBlock(native, x, xff, p, W > 1, H, HD, W, dwK, nxt)
                     ctx.pin(x, True)  # x feeds the next layer: promote to the enclosing arena
                     if xff is not None:
                         ctx.pin(xff, True)
@@ -287,7 +307,7 @@ def encode_batch(ctx, enc, mels: List[np.ndarray], layer_hook=None, use_fast: bo
                 x = ff(x, w["lnff1"], w["ff1w1"], w["ff1w2"], w["ff1b1"], w["ff1b2"], xff)
                 xff = None
                 xln = ln_op(x, w["lnatt"])
-                fused_qkv = use_fast and "qkv" in w and 16 <= Tsub <= 192
+                fused_qkv = use_fast and 16 <= Tsub <= 192 and fused_from(w, "qkv", QKV_PARTS)
                 if fused_qkv:  # read by attnFusedQKV only; from 256 rows on as the packed operand alone
                     qkv = mm(ctx, xln, w["qkv"], dict(bias=w["qkvb"], operandOnly=W * Tsub >= 256))
                 else:

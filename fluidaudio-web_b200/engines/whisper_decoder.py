@@ -25,7 +25,13 @@ from typing import Dict, List, Optional, Sequence
 
 import numpy as np
 
+from .layer_weights import LayerWeights, fused_from, native_struct
+
 f32 = np.float32
+
+# a layer's entries that decoderStep reads, and those of them that "sqkvw" / "sqkvb" are made of
+QKV_PARTS = ("sqw", "sqb", "skw", "svw", "svb")
+NATIVE_KEYS = QKV_PARTS + ("sqkvw", "sqkvb", "sqkvw_of", "sow", "sob", "cqw", "cqb", "cow", "cob", "f1w", "f1b", "f2w", "f2b", "ln1", "ln2", "ln3")
 
 
 def infer_config(man: Dict[str, np.ndarray]) -> dict:
@@ -103,15 +109,16 @@ def load_decoder(ctx, weights: Dict[str, np.ndarray], NH: int, quant: Optional[s
         return ctx.upload(a, 1, a.size)
 
     def self_qkv(L):
-        """The self-attention projections: one [D, 3D] matrix q | k | v where the backend has the one-pass attention
-        step that reads it (k has no bias: zeros), three matrices otherwise.  Per-column arithmetic is the same."""
+        """The self-attention projections, and side by side as one [D, 3D] matrix q | k | v (k has no bias: zeros) where the
+        backend has the one-pass attention step that reads it.  Per-column arithmetic is the same."""
         t = lambda s: f"L{L}_{s}"
+        parts = dict(sqw=mat(t("sqw"), SCALE), sqb=vec(t("sqb"), SCALE), skw=mat(t("skw")), svw=mat(t("svw")), svb=vec(t("svb")))
         if not hasattr(ctx, "attnStepAppend"):
-            return dict(sqw=mat(t("sqw"), SCALE), sqb=vec(t("sqb"), SCALE), skw=mat(t("skw")), svw=mat(t("svw")), svb=vec(t("svb")))
+            return parts
         scaled = lambda k: (weights[t(k)].astype(f32) * SCALE).astype(f32)
         wide = np.concatenate([scaled("sqw"), weights[t("skw")].astype(f32), weights[t("svw")].astype(f32)], axis=1)
         bias = np.concatenate([scaled("sqb").reshape(-1), np.zeros(D, f32), weights[t("svb")].astype(f32).reshape(-1)])
-        return dict(sqkvw=_W(ctx, wide, quant), sqkvb=ctx.upload(bias, 1, 3 * D))
+        return dict(parts, sqkvw=_W(ctx, wide, quant), sqkvb=ctx.upload(bias, 1, 3 * D), sqkvw_of=tuple(map(parts.get, QKV_PARTS)))
 
     layers = []
     for L in range(cfg["layers"]):
@@ -131,17 +138,25 @@ def load_decoder(ctx, weights: Dict[str, np.ndarray], NH: int, quant: Optional[s
     cfg["VOCABP"] = VOCABP
     if hasattr(ctx, "decoderStep"):  # optional member: all layers of a token in one call
         for w in layers:
-            pair = lambda k: (w[k + "w"].native(), w.get(k + "b"))
-            w["native"] = ctx.decoderWeights(dict(sqkv=pair("sqkv"), so=pair("so"), cq=pair("cq"), co=pair("co"), f1=pair("f1"),
-                                                  f2=pair("f2"), ln1=w["ln1"], ln2=w["ln2"], ln3=w["ln3"]))
+            w["native"] = LayerWeights(w, NATIVE_KEYS, _native_of(ctx))
     return dict(layers=layers, embed=embed, embedT=_W(ctx, embedTP, quant), pos=np.ascontiguousarray(weights["pos"], dtype=f32),
                 lnf=(vec("lnf_w"), vec("lnf_b")), cfg=cfg)
+
+
+def _native_of(ctx):
+    """What makes a layer's weights for decoderStep; None when q | k | v no longer stand for the layer's three matrices."""
+    def make(w):
+        if not fused_from(w, "sqkvw", QKV_PARTS):
+            return None
+        pair = lambda k: (w[k + "w"].native(), w.get(k + "b"))
+        return ctx.decoderWeights(dict({k: pair(k) for k in ("sqkv", "so", "cq", "co", "f1", "f2")}, ln1=w["ln1"], ln2=w["ln2"], ln3=w["ln3"]))
+    return make
 
 
 def _self_attention(ctx, x, w, cacheK, cacheV, n, S, D, NH, HD):
     """The token rows x [S, D], normed -> attention over the S streams' caches [position, S*D], whose row n becomes the
     token's key and value (raw-whisper-decoder.js:112-124).  Only past+current exist, so there is no mask."""
-    if "sqkvw" in w:
+    if fused_from(w, "sqkvw", QKV_PARTS):
         qkv = _linear(ctx, x, w["sqkvw"], norm=w["ln1"], bias=w["sqkvb"])
         att = ctx.attnStepAppend(qkv, cacheK, cacheV, n, NH, HD)
         if att is not None:
@@ -180,8 +195,10 @@ def _step(ctx, dec, kv, st, x, n, S):
     """The device part of one token: x [S, D] (embedding + position n) -> logits [S, VOCABP]."""
     cfg = dec["cfg"]
     D, NH, HD = cfg["D"], cfg["NH"], cfg["HD"]
-    if all("native" in w for w in dec["layers"]):
-        return ctx.decoderStep([w["native"] for w in dec["layers"]], x, [c["k"] for c in kv], [c["v"] for c in kv], st["selfK"],
+    make = _native_of(ctx)
+    native = [native_struct(w, NATIVE_KEYS, make) if "native" in w else None for w in dec["layers"]]
+    if None not in native:
+        return ctx.decoderStep(native, x, [c["k"] for c in kv], [c["v"] for c in kv], st["selfK"],
                                st["selfV"], n, NH, HD, dec["lnf"], dec["embedT"].native())
     for li, w in enumerate(dec["layers"]):
         x = _layer(ctx, x, w, kv[li], st["selfK"][li], st["selfV"][li], n, S, D, NH, HD)

@@ -102,3 +102,66 @@ def test_conformer_blocks_when_the_one_kernel_attention_is_off(ctx, pkg, W, samp
         assert np.array_equal(ctx.download(fc.encode_batch(ctx, enc, mel)[0]), native)
     finally:
         ctx.setOption("attn_one_kernel", 1)
+
+
+def _no_native(layers):
+    return [{k: v for k, v in w.items() if k != "native"} for w in layers]
+
+
+@pytest.mark.parametrize("W,samples", [(1, 59200), (2, 171200)])  # fewer than 256 rows, more
+def test_a_replaced_matrix_of_an_encoder_layer_is_the_one_that_runs(ctx, pkg, W, samples):
+    from fluidaudio_web_b200.engines import fastconformer as fc, synth
+
+    cfg = dict(synth.PARAKEET_06B, layers=2)
+    enc, other = (fc.load_encoder(ctx, synth.encoder_weights(cfg, seed=s)) for s in (4, 9))
+    mel = ctx.logMelWindows(ctx.upload(synth.synth_audio(W, samples=samples, seed=5), W, samples), 128)
+    run = lambda e: ctx.download(fc.encode_batch(ctx, e, mel)[0])  # noqa: E731
+    seen = [run(enc)]
+    row = lambda v: ctx.upload(np.full(1024, v, np.float32), 1, 1024)  # noqa: E731
+    new = dict({k: other["layers"][0][k] for k in ("ff1w1", "q", "pw2T")}, lnatt=(row(2.0), row(0.1)), vb=row(0.5))
+    for key in new:
+        old = enc["layers"][0][key]
+        enc["layers"][0][key] = new[key]
+        got = run(enc)
+        parts = dict(enc, layers=[{k: v for k, v in w.items() if k not in ("qkv", "qkvb", "qkv_of")} for w in _no_native(enc["layers"])])
+        near = run(parts)  # the host loop over the entries themselves
+        assert np.linalg.norm(got - near) < 2e-3 * np.linalg.norm(near)
+        assert np.linalg.norm(got - seen[0]) > 2e-2 * np.linalg.norm(near)
+        enc["layers"][0][key] = old
+        assert np.array_equal(run(enc), seen[0])
+    derived = dict(enc, layers=[dict(enc["layers"][0], ff1w1=other["layers"][0]["ff1w1"]), enc["layers"][1]])
+    assert not np.array_equal(run(derived), seen[0]) and np.array_equal(run(enc), seen[0])
+    ctx.freeTensor(enc["layers"][0]["lnconv"][0])
+    with pytest.raises(pkg.CudaError):
+        run(enc)
+
+
+@pytest.mark.parametrize("quant", [None, "int8"])
+@pytest.mark.parametrize("S", [1, 2])
+def test_a_replaced_matrix_of_a_decoder_layer_is_the_one_that_runs(ctx, pkg, quant, S):
+    from fluidaudio_web_b200.engines import synth, whisper_decoder as wd
+
+    cfg = dict(D=256, NH=4, FFN=1024, layers=2, VOCAB=2003, maxPos=40, Tenc=96)
+    dec, other = (wd.load_decoder(ctx, synth.decoder_weights(cfg, seed=s), 4, quant=quant) for s in (11, 12))
+    kv = wd.cross_kv_streams(ctx, dec, ctx.upload(np.concatenate(synth.encoder_states(cfg, S, seed=13)), S * cfg["Tenc"], cfg["D"]))
+
+    def run(layers):
+        st = wd.decode_init_streams(ctx, dec, S, 8)
+        return np.stack([wd.decode_next_streams(ctx, dict(dec, layers=layers), kv, st, [t] * S, want_logits=True)[1] for t in (1, 7, 3)])
+
+    first = run(dec["layers"])
+    row = lambda v: ctx.upload(np.full(256, v, np.float32), 1, 256)  # noqa: E731
+    new = dict({k: other["layers"][1][k] for k in ("f1w", "svw", "cow")}, ln2=(row(3.0), row(0.5)), svb=row(0.5), cob=row(0.5))
+    for key in new:
+        old = dec["layers"][1][key]
+        dec["layers"][1][key] = new[key]
+        got = run(dec["layers"])
+        near = run([{k: v for k, v in w.items() if not k.startswith("sqkv")} for w in _no_native(dec["layers"])])
+        assert np.linalg.norm(got - near) < 1e-3 * np.linalg.norm(near)
+        assert np.linalg.norm(got - first) > 5e-3 * np.linalg.norm(near)
+        dec["layers"][1][key] = old
+        assert np.array_equal(run(dec["layers"]), first)
+    ctx.freeTensor(dec["layers"][0]["ln1"][0])
+    ctx.freeTensor(dec["layers"][0]["ln1"][1])
+    with pytest.raises(pkg.CudaError):
+        run(dec["layers"])
