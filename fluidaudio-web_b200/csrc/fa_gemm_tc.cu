@@ -79,7 +79,7 @@ struct TcParams {
                       // accumulated into the SAME TMEM columns (f32-grade activations for decode-size products)
   int stages;
   int num_kb;         // K chunks of 128 bytes
-  int step;           // K chunks per ring stage, 1 or 2 (see launch_tc)
+  int step;           // K chunks per ring stage, 1 or (int8 form) 2 (see launch_tc)
   int tiles_n, tiles_m;
   int splitk;         // > 1: cluster of `splitk` CTAs along z shares one tile, each taking kb_per_split chunks
   int kb_per_split;
@@ -134,11 +134,18 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ void cluster_arrive_all() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait_all() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-constexpr int kSiluExact = FA_ACT_SILU + 16;  // TcParams::act: SiLU as fa_actf computes it, not fa_silu_fast
+constexpr int kSiluFine = FA_ACT_SILU + 16;  // TcParams::act: SiLU to a few units in the last place of f32, not fa_silu_fast
 
 // Activation applied to 16 values at once with the selector outside the loop, so the 16 chains stay
 // independent (one warp per scheduler has no other work to hide a per-element branch behind).
+// FINE: the launch may ask for kSiluFine.
+template <bool FINE = false>
 __device__ __forceinline__ void act16(float (&v)[16], int act) {
+  if (FINE && act == kSiluFine) {  // (as fa_actf has it, sixteen IEEE divisions one after another took 6 us of a 48-row tile)
+#pragma unroll
+    for (int j = 0; j < 16; j++) v[j] = __fdividef(v[j], 1.0f + __expf(-fminf(fmaxf(v[j], -30.0f), 30.0f)));
+    return;
+  }
   switch (act) {
     case FA_ACT_NONE: break;
     case FA_ACT_RELU:
@@ -151,10 +158,6 @@ __device__ __forceinline__ void act16(float (&v)[16], int act) {
       // (84 us against 53 us for the same product without activation); ex2.approx + rcp.approx still cost 8 us of
       // special-function time per product.
       for (int j = 0; j < 16; j++) v[j] = fa_silu_fast(v[j]);
-      break;
-    case kSiluExact:
-#pragma unroll
-      for (int j = 0; j < 16; j++) v[j] = fa_actf(v[j], FA_ACT_SILU);
       break;
     default:
 #pragma unroll
@@ -173,12 +176,13 @@ __device__ __forceinline__ void act16(float (&v)[16], int act) {
 // next to a 6 us main loop.  Two slabs per warp and per result kind alternate; before a slab is refilled the
 // issuing lane waits until the store that last used it has finished reading it.  The other modes (batched
 // attention products, peer stores, raw int32, ragged row pitches) keep the direct stores.
-template <int KIND, bool PEERS = false>
+// PARTS: the sum of the tile lies in `nseg` sets of accumulators, acc_stride columns apart, to be added in order.
+template <int KIND, bool PEERS = false, bool PARTS = false>
 __device__ __forceinline__ void epilogue_tile(const TcParams &p, uint32_t lane_addr, int n0, int m0, int quad, int lane,
                                               int half, float *outb, int r16, int c16, uint32_t partial,
                                               const CUtensorMap *map_o, const CUtensorMap *map_o16, uint32_t slab_f32,
-                                              uint32_t slab_f16, uint32_t &slab_turn, uint32_t cl_rank, uint32_t nseg,
-                                              uint32_t acc_stride) {
+                                              uint32_t slab_f16, uint32_t &slab_turn, uint32_t cl_rank, uint32_t nseg = 1,
+                                              uint32_t acc_stride = 0) {
   const int n = n0 + quad * 32 + lane;
   const bool n_ok = n < p.N;
   const float cs = (p.colscale && n_ok) ? p.colscale[n] : 1.0f;
@@ -187,12 +191,17 @@ __device__ __forceinline__ void epilogue_tile(const TcParams &p, uint32_t lane_a
     if (m0 + c >= p.M) break;  // warp-uniform: no rows left in this tile
     uint32_t v0[16], v1[16], v2[16];
     tmem_ld16(lane_addr + (uint32_t)c, v0);
-    for (uint32_t sg = 1; KIND == 0 && sg < nseg; sg++) {  // the parts of K, in order
-      uint32_t w[16];
-      tmem_ld16(lane_addr + sg * acc_stride + (uint32_t)c, w);
+    for (uint32_t sg = 1; PARTS && sg < nseg; sg += 2) {
+      uint32_t w[2][16];
+      tmem_ld16(lane_addr + sg * acc_stride + (uint32_t)c, w[0]);
+      if (sg + 1 < nseg) tmem_ld16(lane_addr + (sg + 1) * acc_stride + (uint32_t)c, w[1]);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 16; j++) v0[j] = __float_as_uint(__uint_as_float(v0[j]) + __uint_as_float(w[j]));
+      for (int j = 0; j < 16; j++) {
+        float t = __uint_as_float(v0[j]) + __uint_as_float(w[0][j]);
+        if (sg + 1 < nseg) t += __uint_as_float(w[1][j]);
+        v0[j] = __float_as_uint(t);
+      }
     }
     if (KIND == 1 && p.limbs > 1) tmem_ld16(lane_addr + (uint32_t)(p.MT + c), v1);
     if (KIND == 1 && p.limbs > 2) tmem_ld16(lane_addr + (uint32_t)(2 * p.MT + c), v2);
@@ -271,7 +280,7 @@ __device__ __forceinline__ void epilogue_tile(const TcParams &p, uint32_t lane_a
     }
 #pragma unroll
     for (int j = 0; j < 16; j++) v[j] = fmaf(v[j] * rs[j], cs, bs) + rb[j];
-    act16(v, p.act);
+    act16<KIND == 1 || PARTS>(v, p.act);
     if (!PEERS && p.tma_out) {
       const uint32_t b = slab_turn & (uint32_t)(p.nslab - 1);
       slab_turn++;
@@ -571,7 +580,10 @@ __device__ __forceinline__ void epilogue_tile_fast(const TcParams &p, uint32_t l
 // slot to the MMA warp through a third barrier.  HBM sees 0.5 byte per weight instead of a 2-byte f16 copy.
 // Within every group of 8 weights the unpack leaves k in the order 0,4,1,5,2,6,3,7 (the pairs one mask
 // extracts); the activation tile is packed in the same order, and a sum over k does not care.
-template <int KIND>
+// PARTS: a CTA keeps its sum over K in parts (TcParams::segs), one tile per CTA.  A kernel of its own, like the two-chunk stages of
+// the int8 form alone (TcParams::step): code that a product does not run costs it its instruction fetch (with parts and stages of
+// two chunks in the one f16 kernel 8 x 1024 x 1024 took 6.5 us and 804 x 1024 x 1024 7.1, without them 5.9 and 6.6).
+template <int KIND, bool PARTS = false>
 __global__ void __launch_bounds__(tc_threads<KIND>(), 1)
 k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
           const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_o16,
@@ -586,7 +598,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int q_rows = p.MT * p.limbs;
   const uint32_t q_bytes = (uint32_t)q_rows * kRowBytes;
-  constexpr bool kStep = KIND <= 1;  // stages of two K chunks: [weights 0 | weights 1 | activations 0 | activations 1]
+  constexpr bool kStep = KIND == 1;  // stages of two K chunks: [weights 0 | weights 1 | activations 0 | activations 1]
   const int step = kStep ? p.step : 1;
   const uint32_t w_bytes = kWTiles * kPTileBytes * (uint32_t)step;
   const uint32_t stage_bytes = w_bytes + q_bytes * (uint32_t)step + (uint32_t)tc_raw_bytes<KIND>();
@@ -609,7 +621,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
   const int acc_cols = p.limb_sum ? p.MT : q_rows;
   uint32_t acc_stride = 32;  // TMEM columns per accumulator buffer
   while ((int)acc_stride < acc_cols) acc_stride <<= 1;
-  const uint32_t tmem_cols = (KIND == 0 && p.segs > 2 ? (uint32_t)p.segs : 2u) * acc_stride;
+  const uint32_t tmem_cols = (PARTS ? (uint32_t)p.segs : 2u) * acc_stride;
   const int num_tiles = p.tiles_n * p.tiles_m * p.batches;
   const int kb0 = p.splitk > 1 ? (int)blockIdx.z * p.kb_per_split : 0;
   const int kb1 = p.splitk > 1 ? min(p.num_kb, kb0 + p.kb_per_split) : p.num_kb;
@@ -789,7 +801,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
           tc_fence_after();
           uint32_t d_tmem = tmem_base + buf * acc_stride;
           for (int kb = kb0; kb < kb1 && ok; d_tmem += acc_stride) {  // once, or once per part of K
-            const int ke = KIND == 0 ? min(kb1, kb + p.kb_per_seg) : kb1;
+            const int ke = PARTS ? min(kb1, kb + p.kb_per_seg) : kb1;
             uint32_t acc = 0;
             for (; kb < ke; kb += kSub) {
               if (!__all_sync(0xffffffffu, mbar_wait(fb, ph, p.wait_limit))) {
@@ -841,7 +853,9 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
       using One = std::integral_constant<int, 1>;
       using Two = std::integral_constant<int, 2>;
       if (kStep && step == 2) {
-        if (p.limb_sum) run(std::true_type{}, Two{}); else run(std::false_type{}, Two{});
+        run(std::false_type{}, Two{});
+      } else if (KIND == 1) {
+        run(std::false_type{}, One{});
       } else {
         if (p.limb_sum) run(std::true_type{}, One{}); else run(std::false_type{}, One{});
       }
@@ -1030,7 +1044,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
       if (!ok) break;
       tc_fence_after();
       const uint32_t lane_addr = tmem_base + buf * acc_stride + ((uint32_t)(quad * 32) << 16);
-      if (!kDeq && MK != 1 && p.splitk == 1 && (KIND != 0 || p.segs == 1) && !p.rowscale && !p.rowbias)
+      if (!kDeq && !PARTS && MK != 1 && p.splitk == 1 && !p.rowscale && !p.rowbias)
       {
         if (KIND == 0 && p.tma_add)
           epilogue_tile_resadd(p, lane_addr, n0, m0, quad, lane, half, r16, c16, &map_o, &map_o16, &map_add, slab_f32, slab_f16,
@@ -1044,9 +1058,9 @@ k_tc_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
                                                slab_f16, slab_turn);
       }
       else
-        epilogue_tile<MK, KIND == 3>(p, lane_addr, n0, m0, quad, lane, half, outb, r16, c16, partial, &map_o, &map_o16,
+        epilogue_tile<MK, KIND == 3, PARTS>(p, lane_addr, n0, m0, quad, lane, half, outb, r16, c16, partial, &map_o, &map_o16,
                                      slab_f32, slab_f16, slab_turn, cl_rank,
-                                     KIND == 0 ? (uint32_t)((kb1 - kb0 + p.kb_per_seg - 1) / p.kb_per_seg) : 1u, acc_stride);
+                                     PARTS ? (uint32_t)((kb1 - kb0 + p.kb_per_seg - 1) / p.kb_per_seg) : 1u, acc_stride);
       // hand the accumulator buffer back to the MMA warp
       tc_fence_before();
       __syncwarp();
@@ -1333,7 +1347,7 @@ k_tc_gemm_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                                          slab_turn);
       else
         epilogue_tile<0, false>(p, lane_addr, n0, m0, quad, lane, half, p.out, 0, 0, 0u, &map_o, &map_o16, slab_f32,
-                                slab_f16, slab_turn, 0u, 1u, 0u);
+                                slab_f16, slab_turn, 0u);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(acc_empty(buf), 0);
@@ -1746,7 +1760,7 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
   p.splitk = 1;
   p.kb_per_split = p.num_kb;
   p.segs = 1;
-  bool exact_silu = false;
+  bool fine_silu = false;
   const bool split_ok = !raw_i32 && !ep.out16 && ep.n_peers == 0 && (ep.ldc == 0 || ep.ldc == N) && p.batches == 1;
   if (split_ok && num_tiles <= ctx->sm_count) {
     const int mt_hi = mt < mt_max ? mt : mt_max, w_rows = (KIND == 4 ? 2 : 1) * 128;
@@ -1804,8 +1818,8 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
       p.splitk = best_s;
     }
     p.segs = best_g;
-    // what the plain rule splits had its activation applied by the split's finish, which computes SiLU as fa_actf does
-    exact_silu = parts > 1 && best_s == 1;
+    // what the plain rule splits had its activation applied by the split's finish, whose SiLU is good to f32
+    fine_silu = parts > 1 && best_s == 1;
     num_tiles = p.tiles_n * p.tiles_m * p.batches;
   }
   p.kb_per_seg = ceil_div(p.kb_per_split, p.segs);
@@ -1858,16 +1872,16 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
   const size_t slab_bytes = slab_bytes_for(p.nslab);
   const size_t tail_bytes = tail_fixed + slab_bytes;
   int stages = (int)((227 * 1024 - tail_bytes) / stage_bytes);
-  // Two K chunks per ring stage: one weight load (a tile's consecutive chunks lie back to back) and one activation load
-  // (both chunks, all digit planes) where there were two and two to six.  A copy-engine thread issues a load every ~150 ns
-  // whatever its size, which is what a small tile's K loop runs at; against that the first chunk arrives later.  So the
-  // int8 form always (its planes are separate loads otherwise) and the f16 form on long K, where the chunks pair up evenly
-  // and three such stages fit.  Measured, us, one chunk -> two: int8 512 x 4096 x 1024 17.1 -> 15.1, 100 x 4096 x 1024 13.3
-  // -> 11.0, 16 x 2048 x 2048 8.4 -> 7.1; f16 804 x 4096 x 1024 13.7 -> 13.0, but 300 x 1024 x 4096 7.15 -> 7.66 and, with
-  // residue planes, 64 x 5120 x 1280 10.3 -> 10.7.
+  // Two K chunks per ring stage, int8 form: one weight load (a tile's consecutive chunks lie back to back) and one activation
+  // load (both chunks, all digit planes) where there were two and two to six.  A copy-engine thread issues a load every ~150 ns
+  // whatever its size, which is what a small tile's K loop runs at; against that the first chunk arrives later.  Where the
+  // chunks pair up evenly and three such stages fit.  Measured, us, one chunk -> two: 512 x 4096 x 1024 17.1 -> 15.1, 100 x
+  // 4096 x 1024 13.3 -> 11.0, 16 x 2048 x 2048 8.4 -> 7.1.  Not the f16 form: it won 0.7-1.0 us at K = 4096 with tiles of at
+  // most 64 rows (804 rows 13.8 -> 12.9) and lost 1-2 with taller ones (1200 rows 14.4 -> 16.3), and as a second kernel beside
+  // the one of the other products it cost a chain of both more than it won (six blocks of 937 rows 201 -> 211 us).
   p.step = 1;
-  if ((KIND == 1 || (KIND == 0 && limbs == 1 && p.kb_per_split >= 32)) && !pair && p.batches == 1 && ep.n_peers == 0 && !(p.num_kb & 1) &&
-      !(p.kb_per_split & 1) && (p.segs == 1 || !(p.kb_per_seg & 1)) && stages >= 6 && ctx->tc_wide_stages) {
+  if (KIND == 1 && !pair && p.batches == 1 && ep.n_peers == 0 && !(p.num_kb & 1) &&
+      !(p.kb_per_split & 1) && stages >= 6 && ctx->tc_wide_stages) {
     p.step = 2;
     stages /= 2;
   }
@@ -1883,7 +1897,7 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
   p.bias = ep.bias;
   p.add = ep.add;
   p.rowbias = ep.rowbias;
-  p.act = exact_silu && ep.act == FA_ACT_SILU ? kSiluExact : ep.act;
+  p.act = fine_silu && ep.act == FA_ACT_SILU ? kSiluFine : ep.act;
   p.status = ctx->dev_status;
   p.wait_limit = ctx->wait_limit;
   p.withhold_kb = ctx->tc_withhold_chunk;
@@ -1939,7 +1953,11 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
     FA_LAUNCH_CHECK(ctx, "tc_gemm_pair");
     return FA_OK;
   }
-  FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_tc_gemm<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+  auto kern = k_tc_gemm<KIND>;
+  if constexpr (KIND == 0) {
+    if (p.segs > 1) kern = k_tc_gemm<0, true>;
+  }
+  FA_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   if (p.splitk > 1) {
     cfg.gridDim = dim3(num_tiles, 1, p.splitk);
     attr[1].id = cudaLaunchAttributeClusterDimension;
@@ -1952,7 +1970,7 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
   }
   {
     LaunchScope ls(ctx, KIND == 0 ? "tc_gemm_f16" : (KIND == 1 ? "tc_gemm_i8" : (KIND == 2 ? "tc_gemm_nbits" : (KIND == 4 ? "tc_gemm_tf32x3" : (KIND == 5 ? "tc_gemm_i8w_f16a" : "tc_gemm_f16_scatter")))));
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k_tc_gemm<KIND>, map_w, map_a, map_o, map_o16, map_add, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, map_w, map_a, map_o, map_o16, map_add, p);
     if (e != cudaSuccess) return fa_fail(ctx, FA_ERR_CUDA, "launch tc_gemm: %s", cudaGetErrorString(e));
   }
   FA_LAUNCH_CHECK(ctx, "tc_gemm");
