@@ -10,9 +10,9 @@
 //                 y = s_m * sum_blk scale[n,blk] * ((S1 - zp*A1) + (S2 - zp*A2) / 128).
 //                 Arithmetic budget: ~1 lane-op per weight at M = 1 (an f32 unpack-and-FMA needs 4).
 //   k_gemv_kn     matmul with f16-storage B [K][N] (lib.rs:59-94) and matmulInt8 with wq [K][N]
-//                 (lib.rs:143-162) at M = 1: N-contiguous rows.  A block owns 128 consecutive columns, its 8 warps
-//                 take rows k round-robin, K is split over the ranks of a cluster; activations stay f32 (exact), and
-//                 a layernorm of the row can run in front of the product.  Sums meet in a fixed order.
+//                 (lib.rs:143-162) at M = 1: N-contiguous rows.  A block owns 128 or 64 consecutive columns, its 8
+//                 warps take rows k round-robin, K is split over the ranks of a cluster; activations stay f32 (exact),
+//                 and a layernorm of the row can run in front of the product.  Sums meet in a fixed order.
 #include <cuda_fp16.h>
 
 #include <type_traits>
@@ -264,30 +264,44 @@ __device__ __forceinline__ float gemv_finish(float acc, int m, int n, int N, con
   return v;
 }
 
-// Four consecutive weights of a row as loaded (4 bytes of int8, 8 of f16), and as floats.
+// Four consecutive weights of a row as loaded: 4 bytes of int8, 8 of f16.
 template <bool I8>
 struct RawRow {
   using type = typename std::conditional<I8, unsigned, uint2>::type;
 };
-template <bool I8>
-__device__ __forceinline__ typename RawRow<I8>::type load_raw(const void *w, size_t off) {
-  if constexpr (I8)
-    return __ldcs((const unsigned *)((const int8_t *)w + off));
-  else
-    return __ldcs((const uint2 *)((const __half *)w + off));
+// Two f32 values in a register pair, and the packed add and multiply-add on them (each half rounded like the scalar one).
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
 }
-__device__ __forceinline__ float4 widen(unsigned v) {
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// The four weights as f32 pairs of columns (0, 1) and (2, 3).
+__device__ __forceinline__ void widen(unsigned v, uint64_t &w01, uint64_t &w23) {
   // byte b of (q + 128) into the mantissa of 2^23: the float 8388608 + q + 128, then back to q
   const unsigned x = v ^ 0x80808080u;
-  return make_float4(__uint_as_float(__byte_perm(x, 0x4B000000u, 0x7650)) - 8388736.0f,
-                     __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7651)) - 8388736.0f,
-                     __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7652)) - 8388736.0f,
-                     __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7653)) - 8388736.0f);
+  const uint64_t off = pack2(-8388736.0f, -8388736.0f);
+  w01 = add2(pack2(__uint_as_float(__byte_perm(x, 0x4B000000u, 0x7650)), __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7651))), off);
+  w23 = add2(pack2(__uint_as_float(__byte_perm(x, 0x4B000000u, 0x7652)), __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7653))), off);
 }
-__device__ __forceinline__ float4 widen(uint2 v) {
+__device__ __forceinline__ void widen(uint2 v, uint64_t &w01, uint64_t &w23) {
   const __half2 *h = (const __half2 *)&v;
   const float2 a = __half22float2(h[0]), b = __half22float2(h[1]);
-  return make_float4(a.x, a.y, b.x, b.y);
+  w01 = pack2(a.x, a.y), w23 = pack2(b.x, b.y);
 }
 
 __device__ __forceinline__ float block_sum(float v, float *red, int lane, int warp) {
@@ -304,21 +318,25 @@ __device__ __forceinline__ float block_sum(float v, float *red, int lane, int wa
 // y[n] = act(sum_k x[k] * w[k][n] * colscale[n] + bias[n]) + add[n] for ONE row x [K]; with NORM, x is first replaced by
 // its layernorm (gamma, beta: two-pass mean and variance as in k_layernorm_reg).
 //
-// What bounds it: the weight stream of the large matrices (66 MB of int8 for the vocabulary projection), latency for the
-// others: 1.6 MB are 0.3 us of HBM time, so the launch is a chain of load -> row sum -> exchange between K slices.
-// Hence the layout: a block owns 128 columns (one 4-byte int8 or 8-byte f16 load per lane and row; 64 columns, two rows
-// per warp, where 128 with the widest K split would not give every SM a block) and a K slice, its
-// 8 warps take rows round-robin with two batches of kKnU loads per lane in flight, the first ones requested before the launch waits
-// for its predecessor where the weights can only have been written by an upload (int8 payloads).  K slices are the
-// ranks of a cluster: their sums meet in rank 0's shared memory, in rank order, after one cluster barrier.  (The form
-// before this one let the slices meet in global memory behind a ticket, up to 40 partial rows read by the last block.)
-// Measured, K = N = 1280 int8 in a decoder step: 7.3 us from launch to end, wait for the predecessor included, where the
-// layernorm, product and residual add were three launches; 1280 x 51868 int8 with the layernorm 25 us (2.7 TB/s) against
-// a layernorm, a digit pass and a tensor-core product of 3.8 + 2.6 + 12.5 us that read the row as two int8 digits
-// instead of f32.  A 16-token decoder pass of one stream: 8.24 -> 5.1 ms.  Blocks of
-// 64 columns (K = 1280 and 5120, N = 1280): 8.2 -> 6.5 us a product on average, the pass 4.85 -> 4.56 ms.
-constexpr int kKnU = 16, kKnCols = 128, kKnSlice = 2048;  // loads in a lane's batch, most columns per block, rows of x held at a time
-constexpr int kKnNormMax = 4096;                           // longest row that the layernorm prologue holds in registers
+// What bounds it: the instructions of the inner loop and the weight stream for the large matrices, latency for the others:
+// 1.6 MB are 0.3 us of HBM time, so the launch is a chain of load -> row sum -> exchange between K slices.
+// Layout: a block owns 128 columns (one 4-byte int8 or 8-byte f16 load per lane and row; 64 columns, two rows per warp, where
+// 128 with the widest K split would not give every SM a block) and a K slice, its 8 warps take rows round-robin with two
+// batches of U loads per lane in flight, the first ones requested before the launch waits for its predecessor where the
+// weights can only have been written by an upload (int8 payloads).  K slices are the ranks of a cluster: their sums meet in
+// rank 0's shared memory, in rank order, after one cluster barrier.
+// A whole batch is loaded without a bound per row (rows past the end meet a zero activation instead), an activation lies in
+// shared memory twice so that one 8-byte read is the operand of two packed multiply-adds, and U and the resident blocks are
+// chosen together: 16 loads of int8 (8 where two batches of 8 cover the slice) and 8 of f16, at three blocks per SM, or at
+// four in 64 registers where the grid needs them.  With 16 loads of f16 (112 registers, two blocks per SM), a bound per row and
+// scalar arithmetic the wide products took, us at one row -> now: f16 1280 x 5120 10.6 -> 5.8, 1280 x 51868 47.9 -> 23.3 (5.7
+// TB/s), 5120 x 10240 47.0 -> 20.0; int8 1280 x 20484 14.8 -> 10.0, 1280 x 51868 26.7 -> 15.7 (4.2 TB/s), 5120 x 10244 27.3 ->
+// 16.3; small ones 1280 x 1280 3.9 -> 3.3 (int8), 4.6 -> 3.3 (f16).  The same int8 products as a digit pass and a tensor-core
+// product of two int8 digits: 1280 x 51868 16.0, 1280 x 20484 10.3, 5120 x 10244 16.3.
+// In a decoder step the launch stands for a layernorm, a product and a residual add: 1280 x 51868 int8 with its layernorm 16.0 us
+// against 3.8 + 2.6 + 12.5.
+constexpr int kKnCols = 128, kKnSlice = 2048;  // most columns per block, rows of x held at a time
+constexpr int kKnNormMax = 4096;               // longest row that the layernorm prologue holds in registers
 
 struct KnParams {
   const float *x, *gamma, *beta;
@@ -329,33 +347,43 @@ struct KnParams {
   GemvEp ep;
 };
 
-template <bool I8, bool NORM, int COLS>
-__global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
-  __shared__ __align__(16) float xs[kKnSlice];
+template <bool I8, bool NORM, int COLS, int U, int BLOCKS>
+__global__ void __launch_bounds__(kThreads, BLOCKS) k_gemv_kn(const KnParams p) {
   constexpr int RPW = kKnCols / COLS, kStride = 8 * RPW;  // rows a warp reads at once, rows of a block's 8 warps
+  constexpr int B = kStride * U;                          // rows of a batch
+  static_assert(kKnSlice % (2 * B) == 0, "a slice is whole pairs of batches, but for the last");
+  __shared__ __align__(16) float2 xs[kKnSlice];  // each activation twice, zeros up to the end of a pair of batches
   __shared__ __align__(16) float4 red[kThreads / 32][COLS / 4];
   __shared__ float cred[8][COLS];  // rank 0: the K slices' sums
   __shared__ float stat[kThreads / 32];
   using Raw = typename RawRow<I8>::type;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.y, ks = gridDim.y, N = p.N, K = p.K;
-  const int k0 = rank * p.kslice, k1 = min(K, k0 + p.kslice);
+  const int k0 = min(K, rank * p.kslice), k1 = min(K, k0 + p.kslice);
   const int c0 = blockIdx.x * COLS + (lane % (COLS / 4)) * 4;
   const bool live = c0 < N;  // N % 4 == 0: a live lane owns four whole columns
   const int cc = live ? c0 : 0;
-  Raw ra[kKnU], rb[kKnU];
-  auto fetch = [&](Raw(&raw)[kKnU], int kk) {
+  const int below = RPW - 1 - lane / (COLS / 4);  // a warp's last row of a step lies this far below the lane's
+  const size_t elem = I8 ? 1 : 2, step = (size_t)kStride * N * elem;
+  Raw ra[U], rb[U];
+  auto fetch = [&](Raw(&raw)[U], int kk) {
+    const char *q = (const char *)p.w + ((size_t)kk * N + cc) * elem;
+    if (kk + below + (U - 1) * kStride < k1) {
 #pragma unroll
-    for (int u = 0; u < kKnU; u++) {
-      const int k = kk + u * kStride;
-      raw[u] = Raw{};
-      if (k < k1) raw[u] = load_raw<I8>(p.w, (size_t)k * N + cc);
+      for (int u = 0; u < U; u++, q += step) raw[u] = __ldcs((const Raw *)q);
+    } else {
+#pragma unroll
+      for (int u = 0; u < U; u++, q += step) {
+        raw[u] = Raw{};
+        if (kk + u * kStride < k1) raw[u] = __ldcs((const Raw *)q);
+      }
     }
   };
   int kk = k0 + warp * RPW + lane / (COLS / 4);  // rows kk, kk + kStride, ...
-  if (I8) fetch(ra, kk), fetch(rb, kk + kStride * kKnU);
+  if (I8) fetch(ra, kk), fetch(rb, kk + B);
   if (ks > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // every rank runs before a remote store
   fa_grid_dep_sync();
-  if (!I8) fetch(ra, kk), fetch(rb, kk + kStride * kKnU);
+  if (!I8) fetch(ra, kk), fetch(rb, kk + B);
+  auto padded = [](int rows) { return (rows + 2 * B - 1) / (2 * B) * (2 * B); };
   if (NORM) {
     float4 v[kKnNormMax / 4 / kThreads];
     const int k4 = K >> 2;
@@ -380,33 +408,39 @@ __global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
       const int q = tid + u * kThreads, k = q * 4;
       if (q < k4 && k >= k0 && k < k1) {  // kslice % 8 == 0: a quad lies in one slice; the slice fits xs (host check)
         const float4 g = ((const float4 *)p.gamma)[q], b = ((const float4 *)p.beta)[q];
-        *(float4 *)(xs + (k - k0)) = make_float4((v[u].x - mean) * inv * g.x + b.x, (v[u].y - mean) * inv * g.y + b.y,
-                                                 (v[u].z - mean) * inv * g.z + b.z, (v[u].w - mean) * inv * g.w + b.w);
+        const float4 t = make_float4((v[u].x - mean) * inv * g.x + b.x, (v[u].y - mean) * inv * g.y + b.y,
+                                     (v[u].z - mean) * inv * g.z + b.z, (v[u].w - mean) * inv * g.w + b.w);
+        float4 *d = (float4 *)(xs + (k - k0));
+        d[0] = make_float4(t.x, t.x, t.y, t.y), d[1] = make_float4(t.z, t.z, t.w, t.w);
       }
     }
+    for (int i = k1 - k0 + tid; i < padded(k1 - k0); i += kThreads) xs[i] = make_float2(0.f, 0.f);
     __syncthreads();
   }
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto load_x = [&](int base, int end) {
+    for (int i = tid; i < padded(end - base); i += kThreads) {
+      const float x = base + i < end ? p.x[base + i] : 0.0f;
+      xs[i] = make_float2(x, x);
+    }
+    __syncthreads();
+  };
+  if (!NORM) load_x(k0, min(k1, k0 + kKnSlice));
+  uint64_t a01 = 0, a23 = 0;  // sums of columns (0, 1) and (2, 3)
+#pragma unroll 1
   for (int base = k0; base < k1; base += kKnSlice) {
     const int end = min(k1, base + kKnSlice);
-    if (!NORM) {
-      if (base > k0) __syncthreads();
-      for (int i = tid; i < end - base; i += kThreads) xs[i] = p.x[base + i];
-      __syncthreads();
-    }
-    auto consume = [&](const Raw(&raw)[kKnU], int kk) {
+    if (!NORM && base > k0) __syncthreads(), load_x(base, end);
+    auto consume = [&](const Raw(&raw)[U], int kk) {
+      const uint64_t *x = (const uint64_t *)xs + (kk - base);
 #pragma unroll
-      for (int u = 0; u < kKnU; u++) {
-        const int k = kk + u * kStride;
-        if (k < end) {
-          const float a = xs[k - base];
-          const float4 f = widen(raw[u]);
-          acc.x = fmaf(a, f.x, acc.x), acc.y = fmaf(a, f.y, acc.y), acc.z = fmaf(a, f.z, acc.z), acc.w = fmaf(a, f.w, acc.w);
-        }
+      for (int u = 0; u < U; u++) {
+        uint64_t w01, w23;
+        widen(raw[u], w01, w23);
+        const uint64_t a = x[u * kStride];
+        a01 = fma2(a, w01, a01), a23 = fma2(a, w23, a23);
       }
     };
-    constexpr int B = kStride * kKnU;  // rows of a batch
-    static_assert(kKnSlice % (2 * B) == 0, "no pair of batches straddles `end` on its way");
+#pragma unroll 1
     for (; kk < end; kk += 2 * B) {
       consume(ra, kk);
       if (kk + 2 * B < k1) fetch(ra, kk + 2 * B);
@@ -414,6 +448,8 @@ __global__ void __launch_bounds__(kThreads) k_gemv_kn(const KnParams p) {
       if (kk + 3 * B < k1) fetch(rb, kk + 3 * B);
     }
   }
+  const float2 s01 = unpack2(a01), s23 = unpack2(a23);
+  float4 acc = make_float4(s01.x, s01.y, s23.x, s23.y);
   if (RPW == 2) {
     __syncwarp();
     acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 16), acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 16);
@@ -832,12 +868,13 @@ bool fa_gemv_kn_norm_ok(int K) { return K >= 4 && (K & 3) == 0 && K <= kKnNormMa
 int fa_gemv_kn(fa_ctx *ctx, const float *x, const float *gamma, const float *beta, float eps, const void *w, bool i8,
                const float *colscale, const float *bias, int act, const float *add, float *y, int N, int K) {
   KnParams p{x, gamma, beta, w, y, K, N, 0, eps, GemvEp{colscale, bias, add, act}};
-  // K slices = ranks of a cluster, as many (1, 2, 4, 8) as give about two blocks per SM and leave 64 rows to each; the
-  // layernorm form needs its slice in shared memory whole.
+  // K slices = ranks of a cluster, as many (1, 2, 4, 8) as leave at most four blocks per SM and 64 rows to each; the layernorm
+  // form needs its slice in shared memory whole.  More blocks than are resident start in a second wave, clusters last (int8
+  // 1280 x 30724: 482 blocks 12.1 us, 964 15.9, 241 16.2), and blocks that leave an SM with one of them run at half its rate.
   const bool narrow = ceil_div(N, kKnCols) * 8 < ctx->sm_count;
   const int strips = ceil_div(N, narrow ? kKnCols / 2 : kKnCols);
   int ks = 1;
-  while (ks < 8 && strips * ks * 2 <= 2 * ctx->sm_count + ctx->sm_count / 4 && K >= 64 * ks * 2) ks *= 2;
+  while (ks < 8 && (long long)strips * ks * 2 <= 4ll * ctx->sm_count && K >= 64 * ks * 2) ks *= 2;
   while (gamma && ks < 8 && ceil_div(K, ks) > kKnSlice) ks *= 2;
   p.kslice = (ceil_div(K, ks) + 7) / 8 * 8;
   cudaLaunchConfig_t cfg{};
@@ -856,10 +893,24 @@ int fa_gemv_kn(fa_ctx *ctx, const float *x, const float *gamma, const float *bet
   cudaError_t e;
   {
     LaunchScope ls(ctx, i8 ? "gemv_i8" : "gemv_f16");
-    auto kern = gamma ? (i8 ? (narrow ? k_gemv_kn<true, true, 64> : k_gemv_kn<true, true, 128>)
-                            : (narrow ? k_gemv_kn<false, true, 64> : k_gemv_kn<false, true, 128>))
-                      : (i8 ? (narrow ? k_gemv_kn<true, false, 64> : k_gemv_kn<true, false, 128>)
-                            : (narrow ? k_gemv_kn<false, false, 64> : k_gemv_kn<false, false, 128>));
+    // three resident blocks leave the registers for all loads of both batches, four are needed from 3 x the SMs on: int8 1280 x
+    // 51868 (406 blocks) 15.7 us at three, 19.0 at four; 1280 x 30724 (482 blocks) 16.0 and 12.1
+    const bool four = !gamma && !narrow && (long long)strips * ks > 3ll * ctx->sm_count;
+    const bool shallow = p.kslice <= 2 * 8 * (narrow ? 16 : 8);  // two batches of 8 cover the slice
+    auto form = [&](auto i8_tag, auto u_tag, auto blocks_tag) {
+      constexpr bool I8 = decltype(i8_tag)::value;
+      constexpr int U = decltype(u_tag)::value, BL = decltype(blocks_tag)::value;
+      return gamma ? (narrow ? k_gemv_kn<I8, true, 64, U, BL> : k_gemv_kn<I8, true, 128, U, BL>)
+                   : (narrow ? k_gemv_kn<I8, false, 64, U, BL> : k_gemv_kn<I8, false, 128, U, BL>);
+    };
+    using True = std::true_type;
+    using False = std::false_type;
+    using Eight = std::integral_constant<int, 8>;
+    using Sixteen = std::integral_constant<int, 16>;
+    using Three = std::integral_constant<int, 3>;
+    using Four = std::integral_constant<int, 4>;
+    auto kern = i8 ? (shallow ? form(True{}, Eight{}, Four{}) : (four ? k_gemv_kn<true, false, 128, 16, 4> : form(True{}, Sixteen{}, Three{})))
+                   : (four ? k_gemv_kn<false, false, 128, 8, 4> : form(False{}, Eight{}, Three{}));
     e = cudaLaunchKernelEx(&cfg, kern, p);
   }
   if (e != cudaSuccess) return fa_fail(ctx, FA_ERR_CUDA, "launch gemv_kn: %s", cudaGetErrorString(e));
