@@ -561,8 +561,8 @@ namespace {
 //     so that one 16-byte load IS a lane's A operand (four registers in a row: put together from two loads it cost a move per
 //     register, group and block), and are read once per block for all groups (pitch = 64 mod 128 bytes: conflict-free);
 //   - per block and group: 4 mma (value and residue plane of the activations), then 4 multiply-adds with the scale.
-// The 16 warps' sums meet in shared memory in warp order; K beyond 2048 is split over the ranks of a cluster, whose sums
-// meet in rank 0's shared memory in rank order.
+// The 16 warps' sums meet in shared memory in warp order; from K = 2048 on K is split over the four ranks of a cluster, whose
+// sums meet in rank 0's shared memory in rank order.
 // Measured, 16 rows, recorded blocks: 13.2 us on average for K = 2048, N = 8192 and K = 8192, N = 2048, against 14.1 and 20.0 us
 // (digit pass included) for the f16 copy on the tensor cores, which read 33.5 MB where this reads 10.5.  What is left is the
 // chain of one launch: its 512 threads of 128 registers cannot start beside the block before them.
@@ -822,16 +822,37 @@ bool fa_nbits_mma_ok(int M, int N, int K, int block_size) {
   return M >= 1 && M <= 16 && block_size == 32 && K >= 32 && K <= kMmaMaxSlices * kMmaSliceBlk * 32 && N >= 8 && (N & 7) == 0;
 }
 
+// Column groups per thread block: as many as leave one wave of blocks (clusters of K slices do not tile every GPC, so an eighth
+// of the SMs is left out of the count there).
+static int mma_groups(const fa_ctx *ctx, int N, int slices) {
+  const int room = slices == 1 ? ctx->sm_count : ctx->sm_count * 7 / 8 / slices;
+  return ceil_div(N / 8, room < 1 ? 1 : room);
+}
+
+// A block walks its column groups one after another, so the time grows with groups x blocks of its K slice; the product on the
+// f16 copy of the weights reads four times the bytes, but at the tensor cores' and the HBM's rate.  16 rows, us, here / f16 copy:
+//   K = 512   N = 16384 (224) 6.0 / 6.5, 24576 (336) 9.1 / 8.7, 51200 18.2 / 11.9
+//   K = 1024  N = 8192 (224) 6.5 / 8.9, 10240 (288) 9.0 / 7.6, 32768 20.2 / 13.6
+//   K = 1536  N = 5920 (240) 8.4 / 9.5, 8192 (336) 9.7 / 10.2, 10240 (432) 12.9 / 9.5, 51200 49.4 / 28.0
+//   K = 2048  N = 4096 (256) 7.5 / 9.4, 5120 (320) 10.8 / 10.2, 8192 (512) 12.7 / 11.3, 10240 20.1 / 11.0, 51200 79.5 / 36.0
+//   K = 4096  N = 2048 (256) 7.6 / 16.4, 4096 (512) 12.3 / 11.5, 5120 17.5 / 13.5
+//   K = 8192  N = 2048 (512) 13.7 / 19.9, 4096 24.8 / 16.1
+// So up to 256 groups x blocks, and up to 512 with K over a cluster, where the copy is at most a seventh faster and its weights
+// are rounded to f16 ((q - zp) * scale: 4e-4 of a result against 4e-7 here).
+bool fa_nbits_mma_worth(fa_ctx *ctx, int N, int K) {
+  int slices, slice, lq;
+  mma_slices(ceil_div(K, 32), slices, slice, lq);
+  return mma_groups(ctx, N, slices) * slice <= (slices > 1 ? 512 : 256);
+}
+
 int fa_nbits_mma(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y, int M, int N,
                  int K, int nblk, int zpb, bool hilo) {
   MmaParams p{a, bq, scales, zp, y, M, N, K, nblk, zpb, 0, 0, 0};
   int slices;
   mma_slices(nblk, slices, p.slice, p.lq);
   const int gw = kMmaWarps >> p.lq;  // warps that share a quad's columns
-  // column groups per thread block: as many as leave one wave of blocks (clusters of K slices do not tile every GPC, so
-  // an eighth of the SMs is left out of the count there); walked 8, 4 or 2 at a time by each of the gw warps of a quad
-  const int groups = N / 8, room = slices == 1 ? ctx->sm_count : ctx->sm_count * 7 / 8 / slices;
-  p.gper = ceil_div(groups, room < 1 ? 1 : room);
+  const int groups = N / 8;
+  p.gper = mma_groups(ctx, N, slices);  // walked 8, 4 or 2 at a time by each of the gw warps of a quad
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[2];
   cfg.gridDim = dim3(ceil_div(groups, p.gper), slices);

@@ -3,7 +3,7 @@
 //
 //   tiny or ragged problems            -> any-shape f32 CUDA-core kernels (fa_gemm_simt.cu)
 //   one row of f16 / int8 B, one to    -> kernels on the weights as uploaded (fa_gemv.cu): CUDA cores, for 5 to 16 rows
-//   sixteen rows of int4 B                of int4 mma.sync
+//   sixteen rows of int4 B                of int4 mma.sync (while a block's columns are few, fa_nbits_mma_worth)
 //   f16-storage B, int8 B, int4 B      -> tcgen05 kernels (fa_gemm_tc.cu) for every other size
 //   f32-storage B                      -> tcgen05 kernel in f32-grade arithmetic (kind::tf32, value + residue planes) from
 //                                         a few rows and 256 columns on, else the f32 CUDA-core kernel
@@ -504,7 +504,10 @@ extern "C" int fa_matmul_nbits(fa_ctx *ctx, const fa_tensor *a, fa_bytes *bq, co
       rc = fa_tc_gemm_nbits(ctx, (const __half *)sa.p, side, (const float *)(side + tb), side + tb + sb, (float *)c->dptr, M,
                             N, K, nblk);
     }
-  } else if (tc_shape_ok(ctx, M, N, K) && M <= ctx->nbits_mma_rows && fa_nbits_mma_ok(M, N, K, block_size)) {
+  } else if (tc_shape_ok(ctx, M, N, K) && M <= ctx->nbits_mma_rows && fa_nbits_mma_ok(M, N, K, block_size) &&
+             (fa_nbits_mma_worth(ctx, N, K) || ctx->nbits_mma_rows > 16 ||
+              (foreign_to_recording(ctx, bq->dptr) &&  // (the f16 copy is not made inside a recording)
+               !(bq->nk_f16 && bq->f16_N == N && bq->f16_K == K && bq->f16_scales == scales->dptr && bq->f16_zp == zp->dptr)))) {
     rc = fa_nbits_mma(ctx, ap, (const uint8_t *)bq->dptr, (const float *)scales->dptr, (const uint8_t *)zp->dptr, (float *)c->dptr,
                       M, N, K, nblk, zpb, M <= ctx->f16_hilo_rows);
   } else if (tc_shape_ok(ctx, M, N, K)) {

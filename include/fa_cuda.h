@@ -76,7 +76,8 @@ const char *fa_last_error(fa_ctx *ctx);
  * attnFused runs as one kernel per call when head width is 128 and T <= 192; 0 = the batched-GEMM form),
  * "nbits_mma_rows" (0..17, default 16: int4 products with more activation rows than the GEMV takes and at most this
  * many - at most 16 - stream the 4-bit weights once as uploaded, widen them to f16 in registers and multiply with
- * mma.sync, for N % 8 == 0 and K <= 8192; 17 = 16; 0 = never), "tc_pair" (0/1, default 1: f16-weight products with more tiles than SMs run on pairs of thread blocks that
+ * mma.sync, for N % 8 == 0 and K <= 8192, while a thread block walks few column groups; 17 = up to 16 rows whatever N;
+ * 0 = never), "tc_pair" (0/1, default 1: f16-weight products with more tiles than SMs run on pairs of thread blocks that
  * share one 256-lane tcgen05 MMA, each loading half of the activation rows of the pair's tile; results are
  * bit-identical to the one-block kernel, 0 selects that kernel),
  * "tc_wide_stages" (0/1, default 1: two K chunks per stage of a tensor-core product's ring where they pair up; same values), "tc_tma_store" (0/1, default 1: results of plain

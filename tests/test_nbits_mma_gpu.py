@@ -32,3 +32,59 @@ def test_few_rows(ctx, M, K, N):
     small = N * K < 1 << 18  # little work: the any-shape kernel, exact too
     assert small or ("nbits_mma" if M > 4 else "gemv_nbits") in labels, labels
     assert np.abs(got - want).max() < (3e-5 if M > 4 else 2e-3) * max(1.0, np.abs(want).max() / 4)
+
+
+def _int4(ctx, K, N, rng):
+    nblk = K // 32
+    return (ctx.uploadBytes(rng.integers(0, 256, N * nblk * 16, dtype=np.uint8)), ctx.upload(np.full(N * nblk, 0.01, np.float32), 1, N * nblk),
+            ctx.uploadBytes(np.full(N * ((nblk + 1) // 2), 0x88, np.uint8)))
+
+
+# what the default rule takes against the product on the f16 copy: at most a fifth slower (1.8 to 2.2 times as slow when every
+# width streamed the 4-bit weights), and far faster where the columns are few
+@pytest.mark.parametrize("M,K,N,at_most", [(16, 1536, 16384, 1.2), (5, 2048, 20480, 1.2), (16, 8192, 4096, 1.2), (16, 4096, 16384, 1.2),
+                                           (16, 2048, 8192, 1.3), (16, 1024, 2048, 0.8), (16, 4096, 2048, 0.8)])
+def test_the_rule_takes_the_faster_form(ctx, M, K, N, at_most):
+    import time
+
+    rng = np.random.default_rng(K)
+    x, ws = ctx.upload(rng.standard_normal((M, K)).astype(np.float32), M, K), [_int4(ctx, K, N, rng) for _ in range(3)]
+
+    def body():
+        for _ in range(4):
+            for w in ws:
+                ctx.freeTensor(ctx.matmulNBits(x, *w, N))
+
+    times = {}
+    try:
+        for rows in (16, 0):
+            ctx.setOption("nbits_mma_rows", rows)
+            body()
+            batch, _ = ctx.recordBatch(body)
+            best = 1e9
+            for _ in range(6):
+                ctx.sync()
+                t0 = time.perf_counter()
+                for _ in range(5):
+                    batch.launch()
+                ctx.sync()
+                best = min(best, time.perf_counter() - t0)
+            times[rows] = best
+            batch.free()
+    finally:
+        ctx.setOption("nbits_mma_rows", 16)
+    assert times[16] < at_most * times[0], times
+
+
+def test_a_wide_product_first_used_in_a_recording(ctx):
+    """The f16 copy is not started inside a recording: the streaming kernel takes the product there, eager calls the copy."""
+    rng = np.random.default_rng(3)
+    M, K, N = 16, 1024, 16384
+    a, w = rng.standard_normal((M, K)).astype(np.float32), _int4(ctx, K, N, rng)
+    x = ctx.upload(a, M, K)
+    batch, y = ctx.recordBatch(lambda: ctx.matmulNBits(x, *w, N))
+    batch.launch()
+    recorded = ctx.download(y)
+    batch.free()
+    eager = ctx.download(ctx.matmulNBits(x, *w, N))
+    assert np.linalg.norm(recorded - eager) < 1e-3 * np.linalg.norm(eager)  # weights exact, and rounded to f16
