@@ -509,18 +509,21 @@ int launch_nbits_r(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *
 
 // Output columns per warp pass (each digit load is shared between R rows of weights): 4 for one activation row - with two
 // resident CTAs per SM (register cap 128) one wave then covers 148 * 2 * 8 * 4 = 9472 columns - and 2 for more rows,
-// where 4 would not fit the registers next to the early-requested weights; fewer while the CTAs would not cover the SMs.
+// where 4 would not fit the registers next to the early-requested weights; fewer while the CTAs would not cover the SMs, on
+// rows longer than the two blocks per lane that the wide form requests early (K > 2048).
 // Measured at one row, K = 8192, N = 2048 in a recorded chain: 64 CTAs of 4 columns per warp 11.5 us, 256 of 1 column
-// 6.7 us (11 MB: 1.6 us of HBM time); N = 8192, K = 2048 keeps its 4 columns (4.2 us).
+// 6.7 us (11 MB: 1.6 us of HBM time); N = 8192, K = 2048 keeps its 4 columns (4.2 us).  On short rows more CTAs only repeat
+// the digit prologue: N = 2048, K = 2048 2.8 us at 4 columns, 3.2 at 1; four rows, N = 512, K = 2048 4.6 us at 2, 5.1 at 1.
 template <int M>
 int launch_nbits(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y, int N,
                  int K, int nblk, int zpb) {
+  const bool is_short = nblk <= 64;
   if constexpr (M == 1) {
-    if (ceil_div(N, 8 * 4) >= ctx->sm_count) return launch_nbits_r<1, 4, 2>(ctx, a, bq, scales, zp, y, N, K, nblk, zpb);
+    if (is_short || ceil_div(N, 8 * 4) >= ctx->sm_count) return launch_nbits_r<1, 4, 2>(ctx, a, bq, scales, zp, y, N, K, nblk, zpb);
     if (ceil_div(N, 8 * 2) >= ctx->sm_count) return launch_nbits_r<1, 2, 4>(ctx, a, bq, scales, zp, y, N, K, nblk, zpb);
     return launch_nbits_r<1, 1, 8>(ctx, a, bq, scales, zp, y, N, K, nblk, zpb);
   } else {
-    if (ceil_div(N, 8 * 2) >= ctx->sm_count) return launch_nbits_r<M, 2, 2>(ctx, a, bq, scales, zp, y, N, K, nblk, zpb);
+    if (is_short || ceil_div(N, 8 * 2) >= ctx->sm_count) return launch_nbits_r<M, 2, 2>(ctx, a, bq, scales, zp, y, N, K, nblk, zpb);
     return launch_nbits_r<M, 1, 4>(ctx, a, bq, scales, zp, y, N, K, nblk, zpb);
   }
 }

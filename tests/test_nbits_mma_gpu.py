@@ -88,3 +88,10 @@ def test_a_wide_product_first_used_in_a_recording(ctx):
     batch.free()
     eager = ctx.download(ctx.matmulNBits(x, *w, N))
     assert np.linalg.norm(recorded - eager) < 1e-3 * np.linalg.norm(eager)  # weights exact, and rounded to f16
+
+
+# one to four rows on both sides of K = 2048, fewer and more columns than the SMs have warps for
+@pytest.mark.parametrize("M", [1, 2, 4])
+@pytest.mark.parametrize("K,N", [(32, 8192), (2048, 515), (2048, 4730), (2080, 515), (2080, 2370), (2080, 4740)])
+def test_one_to_four_rows(ctx, M, K, N):
+    test_few_rows(ctx, M, K, N)
