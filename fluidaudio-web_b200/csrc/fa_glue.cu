@@ -1159,10 +1159,12 @@ __global__ void __launch_bounds__(256, 4) k_conv2d_c1_3x3(const float *__restric
 }
 
 // Per-row argmax: out[r] = {index, value}; ties resolve to the lowest index like the host loop
-// of src/engines/asr-whisper/index.ts:80-97.  One block of 32 warps per row, eight loads of a thread in flight: a row is
-// too short to split (207 KB at 51866 columns) and what bounds it is the latency of its loads, one batch after another.
-// Measured, 64 rows of 51866 columns: 33 us with 256 threads and one load in flight each, under 10 us so.
-constexpr int kArgThreads = 1024, kArgBatch = 8;
+// of src/engines/asr-whisper/index.ts:80-97.  One block per row, bound by the latency of its loads: a long row takes 32 warps
+// with eight loads of a thread in flight, a short one, or one of so many that the blocks fill the GPU several times, 8 warps
+// with one load each, eight blocks to an SM.  Measured, us, 8 warps / 32 warps: 64 rows of 51866 columns 9.5 / 6.9, of 16384 3.8
+// / 3.3, of 8192 2.6 / 2.6, of 1000 2.0 / 2.5; 512 rows of 8192 4.9 / 4.9, of 4096 3.3 / 4.6; 2048 rows of 16384 27.5 / 26.6,
+// of 8192 11.6 / 14.6, of 1000 4.9 / 14.1.  So 32 warps from 16384 columns on, and from 8192 up to four rows per SM.
+template <int kArgThreads, int kArgBatch>
 __global__ void __launch_bounds__(kArgThreads) k_argmax_rows(const float *__restrict__ x, float *__restrict__ out, int R, int ld,
                                                              int C) {
   fa_grid_dep_sync();
@@ -1198,7 +1200,8 @@ __global__ void __launch_bounds__(kArgThreads) k_argmax_rows(const float *__rest
     if ((threadIdx.x & 31) == 0) { bv[threadIdx.x >> 5] = best; bi[threadIdx.x >> 5] = idx; }
     __syncthreads();
     if (threadIdx.x < 32) {
-      best = bv[threadIdx.x], idx = bi[threadIdx.x];
+      const int w = threadIdx.x < kArgThreads / 32 ? threadIdx.x : 0;  // (a repeated warp changes nothing)
+      best = bv[w], idx = bi[w];
       warp_best();
       if (threadIdx.x == 0) {
         out[(size_t)r * 2] = (float)idx;
@@ -2264,7 +2267,8 @@ extern "C" int fa_argmax_rows(fa_ctx *ctx, const fa_tensor *x, int ncols, fa_ten
     int grid = x->rows < ctx->sm_count * 8 ? x->rows : ctx->sm_count * 8;
     {
       LaunchScope ls(ctx, "argmax_rows");
-      fa_launch_dep(ctx, k_argmax_rows, dim3(grid), dim3(kArgThreads), 0, (const float *)x->dptr, (float *)y->dptr, x->rows, x->cols, ncols);
+      const bool wide = ncols >= 16384 || (ncols >= 8192 && x->rows <= 4 * ctx->sm_count);  // see the kernel
+      fa_launch_dep(ctx, wide ? k_argmax_rows<1024, 8> : k_argmax_rows<256, 1>, dim3(grid), dim3(wide ? 1024 : 256), 0, (const float *)x->dptr, (float *)y->dptr, x->rows, x->cols, ncols);
     }
     FA_LAUNCH_CHECK(ctx, "argmax_rows");
   }
