@@ -1750,6 +1750,7 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
   //   height    6 per row of the tile (its epilogue)
   //   split     3700 for the hand-over of a split tile (f16 and tf32: 1500 + 35 per row) up to 64 rows, 5500 above, 2500
   //             more for halves of tiles above 96 rows, 600 more for eighths
+  //   depth     two fifths of the chunks' time more where a split tile leaves fewer than three ring stages (tf32 above 96 rows)
   //   spread    14 per CTA: of two equal choices the one with fewer, which leaves the next launch room to start
   // One wave only (a second one costs more than any split saves): clusters do not tile every GPC, so quarters may use
   // 7/8 of the SMs and eighths 2/3; clusters of 3, 5, 6, 7 place badly (2x slower).  Against the rule before it (shortest
@@ -1781,28 +1782,38 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
       if ((long long)p.tiles_n * ceil_div(M, best_mt) * sp > ctx->sm_count || p.num_kb / sp < 4) break;
       if ((sp - 1) * ceil_div(p.num_kb, sp) < p.num_kb) best_s = sp;  // (33 chunks by 8: the last CTA would have nothing to sum)
     }
-    const int parts = best_s;
+    const int parts = best_s, plain_mt = best_mt;
     const bool own_parts = KIND == 0 && limbs == 1;
     const int min_s = KIND == 1 || own_parts ? 1 : parts;  // (integer sums are exact)
     int best_g = 1;
+    auto estimate = [&](int cand, int sp) {
+      const long long rows = w_rows + cand * limbs, chunks = ceil_div(p.num_kb, sp);
+      long long t = chunks * (rows > 160 ? rows : 160);
+      if (sp > 1 && rows * kRowBytes * 3 + cand * 512 > 220 * 1024) t += t * 2 / 5;
+      t += 6 * cand + 14ll * p.tiles_n * ceil_div(M, cand) * sp;
+      if (sp > 1)
+        t += (cand > 64 ? 5500 : (KIND == 1 ? 3700 : 1500 + 35 * cand)) + (sp == 2 && cand > 96 ? 2500 : 0) + (sp == 8 ? 600 : 0);
+      return t;
+    };
+    auto room = [&](int sp) { return sp == 8 ? ctx->sm_count * 2 / 3 : (sp == 4 ? ctx->sm_count * 7 / 8 : ctx->sm_count); };
     long long best = -1;
     for (int cand = mt_hi; cand >= (mt_hi < 32 ? mt_hi : 32); cand -= 16) {
       const int tiles_m = ceil_div(M, cand);
       if (cand > 32 && ceil_div(M, cand - 16) == tiles_m) continue;  // same tiling with less padding further down
       for (int sp = min_s; sp <= 8; sp *= 2) {
         const long long ctas = (long long)p.tiles_n * tiles_m * sp;
-        const int room = sp == 8 ? ctx->sm_count * 2 / 3 : (sp == 4 ? ctx->sm_count * 7 / 8 : ctx->sm_count);
-        if (ctas > room || (sp > 1 && (cand > kSplitMaxMT || p.num_kb / sp < 4))) continue;
-        const long long rows = w_rows + cand * limbs, chunks = ceil_div(p.num_kb, sp);
-        if ((sp - 1) * chunks >= p.num_kb) continue;  // the last CTA of the cluster would have nothing
+        if (ctas > room(sp) || (sp > 1 && (cand > kSplitMaxMT || p.num_kb / sp < 4))) continue;
+        if ((sp - 1) * ceil_div(p.num_kb, sp) >= p.num_kb) continue;  // the last CTA of the cluster would have nothing
         const int g = own_parts && sp < parts ? parts / sp : 1;
         if (g > 1 && g * (cand <= 32 ? 32 : (cand <= 64 ? 64 : (cand <= 128 ? 128 : 256))) > 512) continue;  // TMEM columns
-        long long cost = chunks * (rows > 160 ? rows : 160) + 6 * cand + 14 * ctas;
-        if (sp > 1)
-          cost += (cand > 64 ? 5500 : (KIND == 1 ? 3700 : 1500 + 35 * cand)) + (sp == 2 && cand > 96 ? 2500 : 0) + (sp == 8 ? 600 : 0);
+        const long long cost = estimate(cand, sp);
         if (best < 0 || cost < best) best = cost, best_mt = cand, best_s = sp, best_g = g;
       }
     }
+    // (the estimate of the float forms is good to a few percent: within three the plain choice stays; 100 x 1024 x 4096 tf32 16.8
+    // us there and 18.7 in the one estimated 2 % faster, 1200 x 512 x 512 f16 5.0 and 5.3)
+    if (KIND != 1 && best >= 0 && p.tiles_n * ceil_div(M, plain_mt) * parts <= room(parts) && best * 100 >= estimate(plain_mt, parts) * 97)
+      best_mt = plain_mt, best_s = parts, best_g = 1;
     if (ctx->tc_tile_rows > 0 || ctx->tc_split_k > 0) {  // tuning overrides (options "tc_tile_rows", "tc_split_k")
       if (ctx->tc_tile_rows > 0) best_mt = ((ctx->tc_tile_rows + 15) / 16) * 16 < mt_max ? ((ctx->tc_tile_rows + 15) / 16) * 16 : mt_max;
       best_s = ctx->tc_split_k > 0 ? ctx->tc_split_k : 1;

@@ -111,3 +111,43 @@ def test_silu_of_one_wave_int8_products(ctx, M, K, N):
         ctx.setOption("int8_limbs", 2)
     z = a.astype(np.float64) @ (q * sc.astype(np.float64))
     assert np.abs(got - z / (1 + np.exp(-z))).max() < 1e-5
+
+
+# tile height and K split of the plain rule (the shortest tile of at least 64 rows that keeps one wave, then the widest split):
+# what is chosen instead is no slower (it was 8 to 11 % slower where a tall tile left a split fewer than three ring stages)
+@pytest.mark.parametrize("M,K,N,rows,split", [(100, 1024, 4096, 64, 2), (804, 5120, 1280, 64, 1), (200, 2048, 2048, 64, 2), (300, 4096, 1024, 64, 2)])
+def test_choices_against_the_plain_rule(ctx, M, K, N, rows, split):
+    import time
+
+    rng = np.random.default_rng(K)
+    x = ctx.upload(rng.standard_normal((M, K)).astype(np.float32), M, K)
+    ws = [ctx.upload(rng.standard_normal((K, N)).astype(np.float32), K, N) for _ in range(3)]
+
+    def body():
+        for _ in range(4):
+            for w in ws:
+                ctx.freeTensor(ctx.matmul(x, w))
+
+    def best_of():
+        body()
+        batch, _ = ctx.recordBatch(body)
+        best = 1e9
+        for _ in range(8):
+            ctx.sync()
+            t0 = time.perf_counter()
+            for _ in range(3):
+                batch.launch()
+            ctx.sync()
+            best = min(best, time.perf_counter() - t0)
+        batch.free()
+        return best
+
+    chosen = best_of()
+    ctx.setOption("tc_tile_rows", rows)
+    ctx.setOption("tc_split_k", split)
+    try:
+        plain = best_of()
+    finally:
+        ctx.setOption("tc_tile_rows", 0)
+        ctx.setOption("tc_split_k", 0)
+    assert chosen < 1.05 * plain, (chosen, plain)
