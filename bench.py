@@ -297,7 +297,7 @@ class Int8Gemm:
         return self.ops() * self.nsets * steps / seconds / 1e12
 
     def roofline(self, prof, peaks):
-        ent = [e for e in prof if e["label"] == "tc_gemm_i8"]
+        ent = [e for e in prof if e["label"] in ("tc_gemm_i8", "tc_gemm_i8_wide")]
         if not ent:
             return None
         e = ent[0]
@@ -749,7 +749,7 @@ class TdtDecode:
         return self.W * 15.0 * steps / seconds
 
     def roofline(self, prof, peaks):
-        ent = [e for e in prof if e["label"] == "tc_gemm_i8"]
+        ent = [e for e in prof if e["label"] in ("tc_gemm_i8", "tc_gemm_i8_wide")]
         if not ent:
             return None
         e = ent[0]

@@ -1756,7 +1756,7 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
   // 7/8 of the SMs and eighths 2/3; clusters of 3, 5, 6, 7 place badly (2x slower).  Against the rule before it (shortest
   // tile of at least 64 rows, then the widest split), recorded products, us: f32 300 x 4096 x 1024 35.6 -> 28.8, 800 x 4096
   // x 1024 62.2 -> 51.6; int8 100 x 1024 x 4096 11.7 -> 7.9, 300 x 2048 x 1024 14.0 -> 11.0; f16 300 x 1024 x 1024 8.6 ->
-  // 6.9, 512 x 512 x 512 7.9 -> 5.8.
+  // 6.3, 512 x 512 x 512 7.9 -> 5.5.
   // (the split-K finish stores rows at pitch N: a caller-chosen pitch keeps the one-CTA-per-tile form)
   p.splitk = 1;
   p.kb_per_split = p.num_kb;
@@ -1980,7 +1980,7 @@ int launch_tc(fa_ctx *ctx, const void *w_packed, const void *a_packed, int limbs
     cfg.gridDim = dim3(num_tiles < ctx->sm_count ? num_tiles : ctx->sm_count);  // persistent: one CTA per SM
   }
   {
-    LaunchScope ls(ctx, KIND == 0 ? "tc_gemm_f16" : (KIND == 1 ? "tc_gemm_i8" : (KIND == 2 ? "tc_gemm_nbits" : (KIND == 4 ? "tc_gemm_tf32x3" : (KIND == 5 ? "tc_gemm_i8w_f16a" : "tc_gemm_f16_scatter")))));
+    LaunchScope ls(ctx, KIND == 0 ? "tc_gemm_f16" : (KIND == 1 ? (p.step == 2 ? "tc_gemm_i8_wide" : "tc_gemm_i8") : (KIND == 2 ? "tc_gemm_nbits" : (KIND == 4 ? "tc_gemm_tf32x3" : (KIND == 5 ? "tc_gemm_i8w_f16a" : "tc_gemm_f16_scatter")))));
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, map_w, map_a, map_o, map_o16, map_add, p);
     if (e != cudaSuccess) return fa_fail(ctx, FA_ERR_CUDA, "launch tc_gemm: %s", cudaGetErrorString(e));
   }

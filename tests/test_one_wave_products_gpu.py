@@ -1,4 +1,4 @@
-"""Products whose tiles fit one wave of the SMs: the choice of tile height and K split, ring stages of two K chunks, and the
+"""Products whose tiles fit one wave of the SMs: the choice of tile height and K split, ring stages of two K chunks (int8), and the
 vector form of the int8 digit pass, at the edges of what each takes."""
 import numpy as np
 import pytest
@@ -6,27 +6,27 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-# two K chunks per ring stage against one: f16, f16 with residue planes, int8 digits; even and odd chunk counts, K splits,
-# several tiles per CTA, a remainder of rows and columns
-@pytest.mark.parametrize("kind,M,K,N", [("f16", 804, 1024, 1024), ("f16", 300, 4096, 1024), ("f16", 130, 192, 300), ("f16", 70, 128, 64),
-                                        ("f16", 937, 4096, 1024), ("f16", 65, 4096, 6400), ("f16", 47, 1024, 1024), ("f16", 33, 4096, 1000),
-                                        ("i8", 512, 1024, 4096), ("i8", 100, 4096, 1024), ("i8", 17, 256, 260), ("i8", 300, 1280, 520)])
+# two K chunks per ring stage of the int8 form against one: an unsplit sum and a split one, several tiles per CTA, the fewest
+# chunks, a remainder of rows and columns
+@pytest.mark.parametrize("kind,M,K,N", [("i8", 512, 4096, 1024), ("i8", 100, 4096, 1024), ("i8", 17, 256, 260), ("i8", 300, 1280, 520), ("i8", 16, 5120, 1280),
+                                        ("i8", 33, 2048, 1000), ("i8", 48, 1024, 20000)])
 def test_wide_stages_bit_for_bit(ctx, kind, M, K, N):
     rng = np.random.default_rng(M + N)
     a = ctx.upload(rng.standard_normal((M, K)).astype(np.float32), M, K)
     add = ctx.upload(rng.standard_normal((M, N)).astype(np.float32), M, N)
-    if kind == "f16":
-        w = (ctx.uploadF16((rng.standard_normal((K, N)) / np.sqrt(K)).astype(np.float32), K, N),)
-    else:
-        w = (ctx.uploadBytes(rng.integers(-127, 128, (K, N), dtype=np.int8).view(np.uint8).reshape(-1)),
-             ctx.upload(np.full(N, 0.01, np.float32), 1, N), N, K)
-    outs = []
+    w = (ctx.uploadBytes(rng.integers(-127, 128, (K, N), dtype=np.int8).view(np.uint8).reshape(-1)),
+         ctx.upload(np.full(N, 0.01, np.float32), 1, N), N, K)
+    outs, labels = [], []
     try:
         for wide in (1, 0):
             ctx.setOption("tc_wide_stages", wide)
+            ctx.startProfile(16)
+            ctx.linearStep(a, *w)
+            labels.append({e["label"] for e in ctx.endProfile()})
             outs.append([ctx.download(ctx.linearStep(a, *w, act="silu")), ctx.download(ctx.linearStep(a, *w, add=add))])
     finally:
         ctx.setOption("tc_wide_stages", 1)
+    assert "tc_gemm_i8_wide" in labels[0] and "tc_gemm_i8" in labels[1], labels  # each is the form it says it is
     assert np.array_equal(outs[0][0], outs[1][0]) and np.array_equal(outs[0][1], outs[1][1])
 
 
