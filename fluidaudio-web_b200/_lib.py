@@ -20,7 +20,7 @@ class ProfileEntry(C.Structure):
     _fields_ = [("label", C.c_char * 48), ("ms", C.c_float), ("count", C.c_int)]
 
 
-# name -> argtypes (every function returns int except fa_last_error)
+# the weight structs of the native layer loops (include/fa_cuda.h)
 class Linear(C.Structure):
     _fields_ = [("w", P), ("scale", P), ("bias", P), ("N", I), ("K", I)]
 
@@ -40,6 +40,7 @@ class ConformerLayer(C.Structure):
                          "pw1", "pw2", "qb", "kb", "vb", "qkvb", "outb", "pw1b", "pw2b", "pbu", "pbv", "dw", "dwb")]
 
 
+# name -> argtypes (every function returns int except fa_last_error)
 SIGNATURES = {
     "fa_ctx_create": [I, PP],
     "fa_ctx_destroy": [P],

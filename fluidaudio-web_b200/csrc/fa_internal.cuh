@@ -130,7 +130,7 @@ struct fa_ctx {
   int tc_withhold_chunk = -1;      // test hook, one launch: see TcParams::withhold_kb
   int tc_tma_add = 1;              // residual operand of the large f16 products through the copy engine (TcParams::tma_add)
   int tc_pair = 1;       // f16 products with more tiles than SMs run on CTA pairs sharing one 256-lane MMA
-  int tc_wide_stages = 1;  // two K chunks per ring stage where they pair up evenly (0: one)
+  int tc_wide_stages = 1;  // int8 form: two K chunks per ring stage where they pair up evenly (0: one)
   int tc_tma_store = 1;  // results of plain tensor-core products leave through shared-memory slabs and TMA stores (0: per-lane stores)
   int tc_tile_rows = 0, tc_split_k = 0;  // tuning overrides for sub-wave tensor-core products (0 = chosen by the cost model)
   size_t pool_cap = 0;

@@ -1,6 +1,8 @@
-"""Whisper-style KV-cached decoder, op for op the sequence of
+"""Whisper-style KV-cached decoder: the arithmetic of
 src/engines/asr-whisper/raw-whisper-decoder.js (loadWhisperDecoder :14-72, whisperCrossKV :76-84,
-whisperDecodeInit :92-100, whisperDecodeNext :103-142), written only against ComputeContext members.
+whisperDecodeInit :92-100, whisperDecodeNext :103-142).  Where the backend has the optional members a token is one call into
+native code (decoderStep), or a linear layer with its layernorm and residual is (linearStep) and the attention of the new
+token (attnStep, attnStepAppend); on plain ComputeContext members it is the reference's sequence op for op.
 The reference hard-codes whisper-base sizes (:7-11); here every size is read off the weight shapes so
 the same code runs the large-v3-turbo shape (4 layers, D 1280, 20 heads of 64, FFN 5120, vocab 51866).
 
@@ -9,13 +11,13 @@ Each layer: pre-LN causal self-attention against the cache -> pre-LN cross-atten
 from load time.
 
 Two drivers share the weights:
-  * decode_next         one stream, one token: the reference's exact op sequence (M = 1 products);
+  * decode_next         one stream, one token (M = 1 products);
   * decode_next_streams S streams in lock step: every weight is streamed once per step for all
     streams (M = S products).  Cross-attention is the windowed form of bmmQK / bmmPV (W = S, one
     window per stream).  The growing self-attention caches are laid out time-major,
     [position, stream*D], so that rowsView still selects the filled prefix and the per-stream
-    attention is the SAME member with H = S*NH "heads"; the only member outside the reference
-    interface is reshapeView (a JS engine re-labels {rows, cols} for that).
+    attention is the SAME member with H = S*NH "heads"; of the plain sequence only reshapeView is outside
+    the reference interface (a JS engine re-labels {rows, cols} for that).
 Both produce the same logits row for a stream; the tests hold them to the CPU reference's token ids.
 """
 from __future__ import annotations

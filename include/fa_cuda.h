@@ -80,7 +80,7 @@ const char *fa_last_error(fa_ctx *ctx);
  * 0 = never), "tc_pair" (0/1, default 1: f16-weight products with more tiles than SMs run on pairs of thread blocks that
  * share one 256-lane tcgen05 MMA, each loading half of the activation rows of the pair's tile; results are
  * bit-identical to the one-block kernel, 0 selects that kernel),
- * "tc_wide_stages" (0/1, default 1: two K chunks per stage of a tensor-core product's ring where they pair up; same values), "tc_tma_store" (0/1, default 1: results of plain
+ * "tc_wide_stages" (0/1, default 1: two K chunks per stage of an int8 tensor-core product's ring where they pair up; same values), "tc_tma_store" (0/1, default 1: results of plain
  * tensor-core products leave through shared-memory slabs and copy-engine stores; 0 = per-lane stores, same values),
  * "tc_tma_add" (0/1, default 1: the residual operand of an f16-weight product with K <= 2048 and an f32 result reaches
  * the epilogue through copy-engine loads into shared memory, two blocks ahead; 0 = plain loads, same values),
