@@ -832,20 +832,29 @@ static int mma_groups(const fa_ctx *ctx, int N, int slices) {
   return ceil_div(N / 8, room < 1 ? 1 : room);
 }
 
-// A block walks its column groups one after another, so the time grows with groups x blocks of its K slice; the product on the
-// f16 copy of the weights reads four times the bytes, but at the tensor cores' and the HBM's rate.  16 rows, us, here / f16 copy:
-//   K = 512   N = 16384 (224) 6.0 / 6.5, 24576 (336) 9.1 / 8.7, 51200 18.2 / 11.9
-//   K = 1024  N = 8192 (224) 6.5 / 8.9, 10240 (288) 9.0 / 7.6, 32768 20.2 / 13.6
-//   K = 1536  N = 5920 (240) 8.4 / 9.5, 8192 (336) 9.7 / 10.2, 10240 (432) 12.9 / 9.5, 51200 49.4 / 28.0
-//   K = 2048  N = 4096 (256) 7.5 / 9.4, 5120 (320) 10.8 / 10.2, 8192 (512) 12.7 / 11.3, 10240 20.1 / 11.0, 51200 79.5 / 36.0
-//   K = 4096  N = 2048 (256) 7.6 / 16.4, 4096 (512) 12.3 / 11.5, 5120 17.5 / 13.5
-//   K = 8192  N = 2048 (512) 13.7 / 19.9, 4096 24.8 / 16.1
-// So up to 256 groups x blocks, and up to 512 with K over a cluster, where the copy is at most a seventh faster and its weights
-// are rounded to f16 ((q - zp) * scale: 4e-4 of a result against 4e-7 here).
+// A block walks its column groups one after another, `pw` of them a warp (in steps of 2, 4 or 8 at a time), so the time grows
+// with the columns; the product on the f16 copy of the weights reads four times the bytes, but at the tensor cores' and the
+// HBM's rate.  12 rows, us, here / f16 copy:
+//   K = 512   N = 8192 4.1 / 6.8, 16384 (pw 4) 6.0 / 6.5, 24576 (6) 9.1 / 8.7, 51200 18.2 / 11.9
+//   K = 1024  N = 4096 4.9 / 7.2, 8192 (4) 6.4 / 8.9, 10240 (5) 9.0 / 7.6, 32768 20.2 / 13.6
+//   K = 1536  N = 4096 6.7 / 8.7, 8192 (7) 9.6 / 10.3, 10240 (9) 12.9 / 9.5, 51200 49.4 / 28.0
+//   K = 2048  N = 2048 5.2 / 12.5, 4096 (4) 7.5 / 9.5, 5120 (5) 10.9 / 10.2, 8192 (8) 12.8 / 11.4, 10240 20.1 / 11.0, 51200 79.5 / 36.0
+//   K = 2560  N = 2048 (4) 7.2 / 13.2, 2560 (5) 10.1 / 8.9, 4096 (8) 11.3 / 10.1, 6144 (12) 18.7 / 11.4
+//   K = 4096  N = 2048 (4) 7.6 / 16.3, 2560 (5) 10.4 / 10.1, 4096 (8) 12.1 / 11.8, 5120 17.5 / 13.5
+//   K = 5120  N = 2048 (8) 10.7 / 17.2, 2304 (9) 13.9 / 17.5, 2560 (10) 14.6 / 11.0
+//   K = 8192  N = 1536 (6) 11.6 / 11.4, 2048 (8) 13.6 / 19.9, 2304 (9) 17.2 / 20.1, 2560 (10) 18.1 / 13.3, 4096 23.8 / 16.4
+// On one slice of K: four groups a warp where warps share a quad, one pass of eight where none do.  With K over a cluster: the same
+// one pass of eight, and on up to 4096 of K as many groups as stay within a quarter of the copy's time or near it, for the sake
+// of the weights, which the copy rounds to f16 (4e-4 of a result against 4e-7 here).  And up to two passes where the copy's
+// product splits K over clusters of eight that are not all resident at once (13 to 18 column tiles).
 bool fa_nbits_mma_worth(fa_ctx *ctx, int N, int K) {
   int slices, slice, lq;
   mma_slices(ceil_div(K, 32), slices, slice, lq);
-  return mma_groups(ctx, N, slices) * slice <= (slices > 1 ? 512 : 256);
+  const int gper = mma_groups(ctx, N, slices), gw = kMmaWarps >> lq, pw = ceil_div(gper, gw);
+  if (slices == 1) return pw <= (gw == 1 ? 8 : 4);
+  const int eighths = ceil_div(N, 128) * 8, chunks = ceil_div(K, 64);
+  if (eighths > ctx->sm_count * 2 / 3 && eighths <= ctx->sm_count && 7 * ceil_div(chunks, 8) < chunks) return pw <= 16;
+  return gw == 1 ? pw <= 8 : gper * slice <= (gw == 4 ? 512 : 420);
 }
 
 int fa_nbits_mma(fa_ctx *ctx, const float *a, const uint8_t *bq, const float *scales, const uint8_t *zp, float *y, int M, int N,
